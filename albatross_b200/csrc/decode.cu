@@ -93,7 +93,7 @@ __device__ __noinline__ void head_phase(const HeadParams& hp, int bid, int nb, i
             const HeadTags tg = {hp.tag_in != 0, tag_of(epoch, hp.tag_in), tag_of(epoch, hp.tag_out)};
             if (ups) head_ups_compute(hp, tid, dsm, hsh, SyncNamed256(), tg, htl);
             if (htl) htl[2] = global_ns();
-            head_steps(hp, 0, h, tid, st, hsh, ups, SyncNamed256(), tg, (pair && ups) ? head_par_area(hp, dsm) : nullptr);
+            head_step(hp, 0, h, tid, st, hsh, ups, SyncNamed256(), tg, (pair && ups) ? head_par_area(hp, dsm) : nullptr);
             if (htl) htl[3] = global_ns();
             store_state(st, sbase, tid >> 2, tid & 3);
             // token-shift state hand-over. Pair mode: the normalised input of the phase before is still in this

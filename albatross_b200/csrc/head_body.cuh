@@ -291,96 +291,94 @@ __device__ __forceinline__ float wkv_step(StateRow& st, const float* w, const fl
 }
 
 
-// All T steps of one (sequence b, head h) for the 256 threads tid = 0..255.
+// One step (T = 1) of (sequence b, head h) for the 256 threads tid = 0..255.
 // `par`: the head's per-channel parameters staged in shared memory as [8][64] fp16 in the order w0, a0, v0, k_k, k_a, r_k,
 // ln_x weight, ln_x bias (null: read them from global memory).
 __device__ __forceinline__ float head_par(const __half* par, int which, const __half* global_vec, int gc, int c) {
     return __half2float(par ? par[which * 64 + c] : global_vec[gc]);
 }
 template <class Sync>
-__device__ __forceinline__ void head_steps(const HeadParams& p, int b, int h, int tid, StateRow& st, HeadShared& sh,
+__device__ __forceinline__ void head_step(const HeadParams& p, int b, int h, int tid, StateRow& st, HeadShared& sh,
                                            bool ups, Sync sync, const HeadTags tg = HeadTags{false, 0u, 0u},
                                            const __half* par = nullptr) {
     const int i = tid >> 2, q = tid & 3, lane = tid & 31, warp = tid >> 5;
     const int D = p.D;
     float* sr = sh.r; float* sw = sh.w; float* sk = sh.k; float* sa_ = sh.a; float* sb = sh.b; float* sv = sh.v; float* sy = sh.y;
     float (*up)[64] = sh.up;
-    for (int t = 0; t < p.T; ++t) {
-        const size_t off = ((size_t)b * p.T + t) * D + h * 64;
-        if (warp == 0) {
-            // per-channel glue on two channels per lane; head-wide sums are warp shuffles
-            float kk0[2], av[2], rk[2];
-            float ssq = 0.f, rkr = 0.f;
-            // what needs only the adapter outputs and the parameters comes first: in the persistent kernel r, k, v are
-            // the last inputs to arrive, and everything below the wait for them is on the token's critical path
-            float kfac[2], wd2[2], vg2[2], vf2[2];
+    const size_t off = (size_t)b * D + h * 64;
+    if (warp == 0) {
+        // per-channel glue on two channels per lane; head-wide sums are warp shuffles
+        float kk0[2], av[2], rk[2];
+        float ssq = 0.f, rkr = 0.f;
+        // what needs only the adapter outputs and the parameters comes first: in the persistent kernel r, k, v are
+        // the last inputs to arrive, and everything below the wait for them is on the token's critical path
+        float kfac[2], wd2[2], vg2[2], vf2[2];
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = lane + 32 * e, gc = h * 64 + c;
-                const float w_raw = ups ? up[0][c] : lda(p.w_raw + off + c);
-                const float a_raw = ups ? up[1][c] : lda(p.a_raw + off + c);
-                av[e] = rh(sigmoidf_(rh(head_par(par, 1, p.a0, gc, c) + a_raw)));
-                kfac[e] = rh(1.f + rh(rh(av[e] - 1.f) * head_par(par, 4, p.k_a, gc, c)));
-                vg2[e] = vf2[e] = 0.f;
-                if (!p.layer0) {
-                    const float vg_raw = ups ? up[2][c] : lda(p.vg_raw + off + c);
-                    vg2[e] = rh(sigmoidf_(rh(head_par(par, 2, p.v0, gc, c) + vg_raw)));
-                    vf2[e] = lda(p.v_first + off + c);
-                }
-                // decay in fp32 as on the reference's single-token path (reference/rwkv7.py:241)
-                wd2[e] = __expf(-0.606531f * sigmoidf_(rh(head_par(par, 0, p.w0, gc, c) + w_raw)));
+        for (int e = 0; e < 2; ++e) {
+            const int c = lane + 32 * e, gc = h * 64 + c;
+            const float w_raw = ups ? up[0][c] : lda(p.w_raw + off + c);
+            const float a_raw = ups ? up[1][c] : lda(p.a_raw + off + c);
+            av[e] = rh(sigmoidf_(rh(head_par(par, 1, p.a0, gc, c) + a_raw)));
+            kfac[e] = rh(1.f + rh(rh(av[e] - 1.f) * head_par(par, 4, p.k_a, gc, c)));
+            vg2[e] = vf2[e] = 0.f;
+            if (!p.layer0) {
+                const float vg_raw = ups ? up[2][c] : lda(p.vg_raw + off + c);
+                vg2[e] = rh(sigmoidf_(rh(head_par(par, 2, p.v0, gc, c) + vg_raw)));
+                vf2[e] = lda(p.v_first + off + c);
             }
-            float rr2[2], kr2[2], vv2[2];
-            head_ld_rkv(p, off, lane, tg, rr2, kr2, vv2);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = lane + 32 * e, gc = h * 64 + c;
-                const float rr = rr2[e];
-                const float kr = kr2[e];
-                float vv = vv2[e];
-                kk0[e] = rh(kr * head_par(par, 3, p.k_k, gc, c));
-                ssq = fmaf(kk0[e], kk0[e], ssq);
-                const float k2 = rh(kr * kfac[e]);
-                if (p.layer0) p.v_first[off + c] = __float2half_rn(vv);
-                else vv = rh(vv + rh(rh(vf2[e] - vv) * vg2[e]));
-                sr[c] = rr; sw[c] = wd2[e]; sk[c] = k2; sv[c] = vv;
-                rk[e] = rh(rh(rr * k2) * head_par(par, 5, p.r_k, gc, c));
-                rkr += rk[e];
-            }
-            ssq = warp_sum(ssq);
-            rkr = rh(warp_sum(rkr));
-            const float nrm = fmaxf(rh(sqrtf(ssq)), 1e-12f);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = lane + 32 * e;
-                const float kk = rh(kk0[e] / nrm);
-                sa_[c] = -kk;
-                sb[c] = rh(kk * av[e]);
-            }
-            sync();
-            const float y = wkv_step(st, sw, sk, sa_, sb, sr, sv[i], q);
-            if (q == 0) sy[i] = rh(y);
-            sync();
-            // group norm over the head's 64 channels (eps 64e-5), bonus, gate
-            const float y0 = sy[lane], y1 = sy[lane + 32];
-            const float mean = warp_sum(y0 + y1) * (1.f / 64.f);
-            const float d0 = y0 - mean, d1 = y1 - mean;
-            const float var = warp_sum(d0 * d0 + d1 * d1) * (1.f / 64.f);
-            const float rstd = rsqrtf(var + 64e-5f);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = lane + 32 * e, gc = h * 64 + c;
-                float o = rh((e ? d1 : d0) * rstd * head_par(par, 6, p.lnx_w, gc, c) + head_par(par, 7, p.lnx_b, gc, c));
-                o = rh(o + rh(rkr * sv[c]));
-                const float g = ups ? up[3][c] : lda(p.g + off + c);
-                head_st(p.out, off + c, o * g, tg);
-            }
-        } else {
-            sync();
-            const float y = wkv_step(st, sw, sk, sa_, sb, sr, sv[i], q);
-            if (q == 0) sy[i] = rh(y);
-            sync();
+            // decay in fp32 as on the reference's single-token path (reference/rwkv7.py:241)
+            wd2[e] = __expf(-0.606531f * sigmoidf_(rh(head_par(par, 0, p.w0, gc, c) + w_raw)));
         }
+        float rr2[2], kr2[2], vv2[2];
+        head_ld_rkv(p, off, lane, tg, rr2, kr2, vv2);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = lane + 32 * e, gc = h * 64 + c;
+            const float rr = rr2[e];
+            const float kr = kr2[e];
+            float vv = vv2[e];
+            kk0[e] = rh(kr * head_par(par, 3, p.k_k, gc, c));
+            ssq = fmaf(kk0[e], kk0[e], ssq);
+            const float k2 = rh(kr * kfac[e]);
+            if (p.layer0) p.v_first[off + c] = __float2half_rn(vv);
+            else vv = rh(vv + rh(rh(vf2[e] - vv) * vg2[e]));
+            sr[c] = rr; sw[c] = wd2[e]; sk[c] = k2; sv[c] = vv;
+            rk[e] = rh(rh(rr * k2) * head_par(par, 5, p.r_k, gc, c));
+            rkr += rk[e];
+        }
+        ssq = warp_sum(ssq);
+        rkr = rh(warp_sum(rkr));
+        const float nrm = fmaxf(rh(sqrtf(ssq)), 1e-12f);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = lane + 32 * e;
+            const float kk = rh(kk0[e] / nrm);
+            sa_[c] = -kk;
+            sb[c] = rh(kk * av[e]);
+        }
+        sync();
+        const float y = wkv_step(st, sw, sk, sa_, sb, sr, sv[i], q);
+        if (q == 0) sy[i] = rh(y);
+        sync();
+        // group norm over the head's 64 channels (eps 64e-5), bonus, gate
+        const float y0 = sy[lane], y1 = sy[lane + 32];
+        const float mean = warp_sum(y0 + y1) * (1.f / 64.f);
+        const float d0 = y0 - mean, d1 = y1 - mean;
+        const float var = warp_sum(d0 * d0 + d1 * d1) * (1.f / 64.f);
+        const float rstd = rsqrtf(var + 64e-5f);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = lane + 32 * e, gc = h * 64 + c;
+            float o = rh((e ? d1 : d0) * rstd * head_par(par, 6, p.lnx_w, gc, c) + head_par(par, 7, p.lnx_b, gc, c));
+            o = rh(o + rh(rkr * sv[c]));
+            const float g = ups ? up[3][c] : lda(p.g + off + c);
+            head_st(p.out, off + c, o * g, tg);
+        }
+    } else {
+        sync();
+        const float y = wkv_step(st, sw, sk, sa_, sb, sr, sv[i], q);
+        if (q == 0) sy[i] = rh(y);
+        sync();
     }
 }
 

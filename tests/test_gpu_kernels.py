@@ -123,6 +123,35 @@ def test_wkv7_operator_against_oracle(B, T, H):
         assert torch.equal(y1, y[0]) and torch.equal(S1, S[0])
 
 
+@pytest.mark.parametrize("T", [2, 7, 8, 9, 16, 31, 33, 41, 130])
+@pytest.mark.parametrize("B,H,shift", [(1, 2, 0), (3, 1, 0), (1, 1, 1)])
+def test_wkv7_sequences_around_the_chunk_size(B, H, T, shift):
+    """The sequence kernel works in chunks of 8 steps through a ring of four: lengths around both, several sequences, and
+    inputs on odd 2-byte boundaries (shift = 1), which take the plain kernel. Bound: y is rounded to fp16 once (2**-11 of
+    the value); the state differs by the order of fp32 sums only."""
+    from albatross_b200 import RWKV7_BATCH_OP
+    torch.manual_seed(T * 10 + B)
+    Cn = H * 64
+    kk = torch.nn.functional.normalize(torch.randn(B, T, H, 64), dim=-1).view(B, T, Cn)
+    vec = [torch.randn(B, T, Cn), -torch.nn.functional.softplus(-torch.randn(B, T, Cn)) - 0.5, torch.randn(B, T, Cn),
+           torch.randn(B, T, Cn), -kk, kk * torch.sigmoid(torch.randn(B, T, Cn))]
+    vec = [v.half() for v in vec]
+    S0 = torch.randn(B, H, 64, 64) * 0.3
+    S_ref = S0.clone()
+    y_ref = Oracle.wkv7_kernel(S_ref, *vec)
+    S, dev = S0.cuda(), []
+    for v in vec:
+        buf = torch.empty(v.numel() + shift, dtype=torch.float16, device="cuda")
+        buf[shift:] = v.flatten().cuda()
+        dev.append(buf[shift:].view(B, T, Cn))
+    y = RWKV7_BATCH_OP(S, *dev)
+    torch.cuda.synchronize()
+    from albatross_b200 import _lib
+    assert _lib.device_status() == 0
+    assert rel_err(y.float().cpu(), y_ref.float()) < 2e-3
+    assert rel_err(S.cpu(), S_ref) < 1e-5
+
+
 def test_wkv7_operator_rejects_bad_shapes():
     from albatross_b200 import _lib
     assert _lib.lib.ab_wkv7_fwd(1, 1, 96, 2, 16, 16, 16, 16, 16, 16, 16, 16, None) == -1
