@@ -8,24 +8,30 @@
 //
 // The weights are the M side of the MMA so that every weight byte is read from HBM exactly once per
 // N tile; the batch (up to 320 rows per block: an MMA of N = 192 and one for the rest) is the N side.
+//   weight warp: brings raw quantised rows in with TMA, 128 bytes of each of the 128 rows at a time (2 k-steps of int8, 4 of
+//               NVFP4 with their block scales beside them, 1 of fp16), into as many shared-memory slots as the activation
+//               stages leave room for; no producer computes an address or waits for a copy of its own.
 //   producer groups (G_NG groups of 4 warps; thread = one of the block's 128 weight rows): group g owns
-//               k-steps g, g + G_NG, ... It brings the row's 64 inputs of a k-step in (cp.async ring of raw
-//               quantised bytes; fp16 rows go straight to registers), de-quantises in registers (int8 ->
-//               fp16 exactly; e2m1 x e4m3 block scale -> fp16 exactly) and writes them to tensor memory
-//               (tcgen05.st: its 32 registers = 32 columns of its own TMEM lane), from where the MMA reads its
-//               weight operand; shared memory carries only the activation tiles. (Compiled with G_A_TMEM_=0
-//               the weights go to shared memory instead, K-major with the 128-byte swizzle.)
+//               k-steps g, g + G_NG, ... It reads the row's 64 inputs of a k-step from the slot, de-quantises in
+//               registers (int8 -> fp16 exactly; e2m1 x e4m3 block scale -> fp16 exactly) and writes them to tensor
+//               memory (tcgen05.st: its 32 registers = 32 columns of its own TMEM lane), from where the MMA reads its
+//               weight operand; shared memory carries the raw rows and the activation tiles.
 //               One warp per scheduler cannot hide the latencies of this
 //               serial instruction stream; several groups on different k-steps can. Afterwards all groups
 //               run the epilogue: tcgen05.ld of 32 columns of their 32 TMEM lanes, row / tensor scale,
 //               activation or residual; the fp16 tile is laid out in shared memory and leaves through TMA stores
 //               (a residual tile comes in through TMA loads); products with a ragged row pitch store directly;
-//   next warp : one thread issues the TMA loads of the activation tile (tensor map over X, 128B swizzle);
-//   last warp : allocates TMEM; one thread issues tcgen05.mma (kind::f16) and commits to mbarriers.
+//   activation warp: TMA loads of the activation tile (tensor map over X, 128B swizzle);
+//   MMA warp  : allocates TMEM; issues tcgen05.mma (kind::f16) and commits to mbarriers.
 // Four-stage operand ring, all waits bounded (status word on expiry), TMEM freed on every path. Short grids with
 // long K loops are split along K: every block of a tile finishes a share of its 32-row chunks, fetching the other
 // blocks' fp32 partial sums of them from a scratch area with bulk copies and adding them in a fixed order. Launched with
 // programmatic stream serialisation the kernel starts its weight stream before it waits for its predecessor.
+//
+// What bounds it: from 256 batch rows on the tensor core (a k-step of 320 rows takes 717 cycles of 640 at its rate,
+// 256 rows 559 of 512); below that the hand-over between the warps, about 450 cycles a k-step whatever the batch.
+// 16384 x 4096, back to back: 320 rows nvfp4 39.2 -> 34.4 us, 64 rows nvfp4 32.0 -> 19.7, 8 rows int8 32.6 -> 22.0, against
+// the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below).
 #include <cuda.h>
 
 #include <type_traits>
@@ -44,20 +50,15 @@ constexpr int G_NG = G_NG_;      // producer groups
 constexpr int G_PROD = 128 * G_NG;
 constexpr int GT = G_PROD + 128; // threads per block: producers + a warpgroup holding the TMA warp, the MMA warp and two idle warps
                                  // (register re-allocation works on whole, aligned warpgroups)
-#ifndef G_A_TMEM_
-#define G_A_TMEM_ 1
-#endif
 #ifndef G_STAGES_
 #define G_STAGES_ 4
 #endif
 constexpr int G_STAGES = G_STAGES_;
-constexpr bool G_A_TMEM = G_A_TMEM_ != 0;   // de-quantised weights go to tensor memory instead of shared memory
 constexpr int G_A_COLS = 32;             // TMEM columns of one weight stage: 64 inputs as fp16 pairs
 constexpr int G_BM = 128;        // weight rows per block
 constexpr int G_BK = 64;         // inputs per k-step (128 bytes of fp16 = one swizzle row)
-constexpr int G_A_BYTES = G_BM * G_BK * 2;
-constexpr int G_RAW_BYTES = 56 * 1024;   // rings of raw (still quantised) weight k-steps filled by cp.async
-constexpr int G_RAW_GROUP = (G_RAW_BYTES / G_NG) & ~1023;   // one ring per producer group
+constexpr int G_RAW_ROW = 128;            // bytes of each weight row per raw slot: 1 / 2 / 4 k-steps of fp16 / int8 / NVFP4
+constexpr int G_RAW_SLOTS = 12;           // at most this many raw slots
 constexpr int G_REGS_PROD = 136, G_REGS_REST = 96;   // (136 - 128) * 384 producer threads <= (128 - 96) * 128 others
 constexpr int G_MAX_OPS = 8;
 constexpr int G_COUNTERS = 4096;         // split-K arrival counters at the start of the scratch area
@@ -73,6 +74,7 @@ struct GemmProb {
     int tile_base;    // first split-K tile id (counter / partial index)
     long long part_base;   // float offset of its split-K partial sums in the scratch area
     int tma_out;      // output (and residual) tiles go through shared memory and the TMA unit
+    int scale_map;    // NVFP4: the block scales come by TMA with the weights (else each thread loads its own)
     int recv_slots;   // split K: own chunks whose slices fit the receive area at a time
 };
 struct GemmGroup {
@@ -86,17 +88,40 @@ struct GemmGroup {
     int a_col0;     // first TMEM column of the weight stages (behind the accumulators)
     unsigned* counters;
     float* partials;
+    int raw_bytes;  // shared memory for the raw slots
     int recv_off;   // split K: byte offset of the area the partial sums are fetched to, in the block's shared memory
 };
 struct GemmMaps {
     CUtensorMap m[G_MAX_OPS];   // activations X
     CUtensorMap y[G_MAX_OPS];   // outputs Y, boxes of 32 batch rows x 128 features
     CUtensorMap r[G_MAX_OPS];   // residuals, same boxes
+    CUtensorMap w[G_MAX_OPS];   // weights as bytes, boxes of 128 rows x 128 bytes
+    CUtensorMap s[G_MAX_OPS];   // NVFP4 block scales, boxes of 128 rows x 16 bytes (k a multiple of 256)
 };
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers (tcgen05 / TMA)
 // ---------------------------------------------------------------------------------------------
+// The wrappers named *_one are called by a whole, converged warp; one elected lane performs the operation. The election
+// sits inside the assembly on purpose: tcgen05 and TMA instructions take their operands from registers shared by the
+// warp, and in code that only one lane runs (`if (lane == 0)`) the compiler wraps every one of them in a loop that
+// moves the operands over lane by lane. An MMA issued that way took 95 - 120 cycles, which bounded every product here
+// whatever its batch (a k-step of four: 480 cycles at 16 batch rows as at 192); elected it takes 34 (N <= 64) and runs
+// at the tensor core's rate above (4 x N = 128: 257 cycles).
+__device__ __forceinline__ void tma_load_2d_one(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+        " @q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_one(uint64_t* bar, uint32_t bytes) {
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(
+                     smem_u32(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -121,22 +146,18 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_commit_one(uint64_t* bar) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar))
         : "memory");
 }
-// The same product with the weight operand read from tensor memory (128 lanes = weight rows, 8 columns = 16 inputs
-// as fp16 pairs) instead of shared memory.
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D (tensor memory) += A * B with the weight operand A read from tensor memory (128 lanes = weight rows, 8 columns = 16
+// inputs as fp16 pairs) and the activations B from shared memory.
+__device__ __forceinline__ void tc_mma_f16_one(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        "{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -163,21 +184,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* v) {
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ uint4 ldg_nc16(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src, bool ok) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 4 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -207,14 +213,28 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// De-quantise the 64 inputs of this thread's row from a landed ring slot into eight 16-byte chunks of fp16
-// (chunk c = inputs 8c..8c+7). Invalid rows / inputs were zero-filled by the copy.
-__device__ __forceinline__ void raw_dequant(int fmt, int r_local, const unsigned char* slot, uint4* out) {
-    if (fmt == FMT_I8) {
+__host__ __device__ constexpr int raw_ksteps(int fmt) { return fmt == FMT_I8 ? 2 : (fmt == FMT_FP4 ? 4 : 1); }   // k-steps per raw slot
+__host__ __device__ constexpr int raw_slot_bytes(int fmt) { return G_BM * (G_RAW_ROW + (fmt == FMT_FP4 ? 16 : 0)); }
+
+// 16-byte chunk c of row r of a raw slot (128-byte rows, 128-byte swizzle: eight consecutive rows, eight bank groups)
+__device__ __forceinline__ uint4 raw_chunk(const unsigned char* slot, int r, int c) {
+    return *reinterpret_cast<const uint4*>(slot + r * G_RAW_ROW + ((c ^ (r & 7)) << 4));
+}
+// De-quantise the 64 inputs of k-step `sub` of a raw slot for row r into eight 16-byte chunks of fp16 (chunk c =
+// inputs 8c..8c+7): the raw bytes first (`raw`, so that the slot can be given back), then the arithmetic. Rows and
+// inputs outside the matrix were zero-filled by the copy. sc4: NVFP4, the four block scales of these inputs.
+template <int F>
+__device__ __forceinline__ void raw_fetch(const unsigned char* slot, int r, int sub, uint4* raw) {
+    constexpr int nq = 8 / raw_ksteps(F);
+#pragma unroll
+    for (int q = 0; q < nq; ++q) raw[q] = raw_chunk(slot, r, sub * nq + q);
+}
+template <int F>
+__device__ __forceinline__ void raw_dequant(const uint4* raw, uint32_t sc4, uint4* out) {
+    if (F == FMT_I8) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint4 raw = *reinterpret_cast<const uint4*>(slot + q * 2048 + r_local * 16);
-            const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
+            const uint32_t words[4] = {raw[q].x, raw[q].y, raw[q].z, raw[q].w};
             uint32_t h[8];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -230,14 +250,11 @@ __device__ __forceinline__ void raw_dequant(int fmt, int r_local, const unsigned
             out[2 * q] = make_uint4(h[0], h[1], h[2], h[3]);
             out[2 * q + 1] = make_uint4(h[4], h[5], h[6], h[7]);
         }
-    } else if (fmt == FMT_F16) {
+    } else if (F == FMT_F16) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) out[c] = *reinterpret_cast<const uint4*>(slot + c * 2048 + r_local * 16);
+        for (int c = 0; c < 8; ++c) out[c] = raw[c];
     } else {
-        const uint4 r0 = *reinterpret_cast<const uint4*>(slot + r_local * 16);
-        const uint4 r1 = *reinterpret_cast<const uint4*>(slot + 2048 + r_local * 16);
-        const uint32_t sc4 = *reinterpret_cast<const uint32_t*>(slot + 4096 + r_local * 4);
-        const uint32_t words[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+        const uint32_t words[8] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w, raw[1].x, raw[1].y, raw[1].z, raw[1].w};
         // the four block scales of these 64 inputs, each duplicated into both halves of a half2
         const __half2 s01 = e4m3x2_to_half2(sc4 & 0xffffu), s23 = e4m3x2_to_half2(sc4 >> 16);
         const __half2 scs[4] = {__low2half2(s01), __high2half2(s01), __low2half2(s23), __high2half2(s23)};
@@ -276,7 +293,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ GemmMaps maps,
                                                         const __grid_constant__ GemmGroup g) {
     extern __shared__ __align__(1024) unsigned char gsm[];
-    __shared__ uint64_t full[G_STAGES], empty[G_STAGES], accum_bar, resid_bar, recv_bar;
+    __shared__ uint64_t full[G_STAGES], empty[G_STAGES], raw_full[G_RAW_SLOTS], raw_empty[G_RAW_SLOTS], accum_bar, resid_bar, recv_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -288,25 +305,33 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
     const int m_tile = local / pb.ksplit, z = local - m_tile * pb.ksplit;
     const int m0 = m_tile * G_BM;
     const int n0 = blockIdx.y * g.n_tile;
-    const int total_ksteps = (pb.w.k + G_BK - 1) / G_BK;
-    const int ks_begin = (int)((long long)total_ksteps * z / pb.ksplit);
-    const int ks_end = (int)((long long)total_ksteps * (z + 1) / pb.ksplit);
-    const int n_ksteps = ks_end - ks_begin;
+    // K is dealt out in raw slots of `per` k-steps
+    const int fmt = pb.w.fmt, per = raw_ksteps(fmt);
+    const int total_ksteps = (pb.w.k + G_BK - 1) / G_BK, total_raw = (total_ksteps + per - 1) / per;
+    const int raw_begin = (int)((long long)total_raw * z / pb.ksplit), raw_end = (int)((long long)total_raw * (z + 1) / pb.ksplit);
+    const int n_raw = raw_end - raw_begin;
+    const int n_ksteps = min(raw_end * per, total_ksteps) - raw_begin * per;
     // Blocks walk K in rotated order: at any moment they read different columns of the (shared) activation
-    // matrix, instead of all hitting the same few L2 lines.
-    const int rot = (int)((blockIdx.x * 7u + blockIdx.y * 3u) % (unsigned)n_ksteps);
-    auto kstep_of = [&](int i) { int k = i + rot; if (k >= n_ksteps) k -= n_ksteps; return ks_begin + k; };
+    // matrix, instead of all hitting the same few L2 lines. (Not where the last slot is only partly used: it comes last.)
+    const int rot = total_ksteps % per ? 0 : (int)((blockIdx.x * 7u + blockIdx.y * 3u) % (unsigned)n_raw);
+    auto raw_of = [&](int i) { int k = i + rot; if (k >= n_raw) k -= n_raw; return raw_begin + k; };   // i-th slot worked on
+    auto kstep_of = [&](int i) { return raw_of(i / per) * per + i % per; };
+    const int slot_bytes = raw_slot_bytes(fmt);
+    const int n_slots = min(G_RAW_SLOTS, g.raw_bytes / slot_bytes);
 
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)gsm + 1023) & ~(uintptr_t)1023);
     const int b_bytes = g.n_tile * 128;
-    unsigned char* smA = base;                                  // G_STAGES x 16 KB (unused when the weights go to TMEM)
-    unsigned char* smB = base + (G_A_TMEM ? 0 : G_STAGES * G_A_BYTES);   // G_STAGES x n_tile x 128 B
-    unsigned char* smRaw = smB + G_STAGES * b_bytes;            // raw weight ring
+    unsigned char* smB = base;                                  // G_STAGES x n_tile x 128 B
+    unsigned char* smRaw = smB + G_STAGES * b_bytes;            // raw weight slots
 
     if (tid == 0) {
         for (int s = 0; s < G_STAGES; ++s) {
             mbar_init(&full[s], 5);   // the four warps of the group that owns the k-step + the TMA thread's expect_tx
             mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < n_slots; ++s) {
+            mbar_init(&raw_full[s], 1);
+            mbar_init(&raw_empty[s], 4 * per);   // the four warps of the group that owns each of its k-steps
         }
         mbar_init(&accum_bar, 1);
         mbar_init(&resid_bar, 1);
@@ -341,9 +366,10 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         // ===== weight producers: thread = weight row of the tile, group = every G_NG-th k-step =====
         const int grp = warp >> 2, r_local = tid & 127;
         const int row = m0 + r_local;
-        const int fmt = pb.w.fmt;
         const int n_out = pb.w.n_out;
         const bool row_ok = row < n_out;
+        float scale = 1.f;   // of the output row; requested here, used in the epilogue
+        if (row_ok) scale = fmt == FMT_I8 ? __ldg(reinterpret_cast<const float*>(pb.w.scale) + row) : pb.w.tscale;
 
         // de-quantised k-step -> operand stage (swizzled), then tell the MMA warp
         // (j = how many k-steps this group has done before; with as many groups as stages a group always fills the
@@ -351,93 +377,64 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         auto put_stage = [&](int ks, int j, const uint4* cur) {
             const int s = G_NG == G_STAGES ? grp : ks % G_STAGES, f = G_NG == G_STAGES ? j : ks / G_STAGES;
             if (f > 0) wait_ok(&empty[s], (f - 1) & 1);
-            if (G_A_TMEM) {
-                tc_fence_after();   // the MMAs that read this stage are complete (their commit released it)
-                // this thread's 64 inputs = 32 registers -> 32 columns of its own TMEM lane
-                tc_st32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g.a_col0 + s * G_A_COLS),
-                        reinterpret_cast<const uint32_t*>(cur));
-                tc_fence_before();
-            } else {
-                unsigned char* dst = smA + s * G_A_BYTES + r_local * 128;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(dst + ((c ^ (r_local & 7)) << 4)) = cur[c];
-                fence_proxy_async();   // generic-proxy stores -> visible to the tensor core's async proxy
-            }
+            tc_fence_after();   // the MMAs that read this stage are complete (their commit released it)
+            // this thread's 64 inputs = 32 registers -> 32 columns of its own TMEM lane
+            tc_st32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g.a_col0 + s * G_A_COLS),
+                    reinterpret_cast<const uint32_t*>(cur));
+            tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);   // one arrival per warp of the owning group
         };
 
-        if (fmt == FMT_F16) {
-            // fp16 rows need no conversion: global -> registers one own k-step ahead -> operand stage
-            const unsigned char* rowp = reinterpret_cast<const unsigned char*>(pb.w.w) + (row_ok ? (size_t)row * pb.w.k * 2 : 0);
-            auto fetch = [&](int ks, uint4* dst) {
-                const int k0 = kstep_of(ks) * G_BK;
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    dst[c] = (row_ok && k0 + c * 8 < pb.w.k) ? ldg_nc16(rowp + (size_t)(k0 + c * 8) * 2) : make_uint4(0, 0, 0, 0);
+        // One instance of the loop per weight format: chunk counts are constants in it, slots are walked with wrapping counters.
+        auto produce = [&](auto fmt_c) {
+            constexpr int F = decltype(fmt_c)::value;
+            constexpr int P = raw_ksteps(F), SB = raw_slot_bytes(F);
+            // block scales without a tensor map (k not a multiple of 256): this thread's own words, one own k-step ahead
+            const bool own_sc = F == FMT_FP4 && !pb.scale_map;
+            const unsigned char* srow = reinterpret_cast<const unsigned char*>(pb.w.scale) + (F == FMT_FP4 && row_ok ? (size_t)row * (pb.w.k / 16) : 0);
+            auto scale_word = [&](int ks) -> uint32_t {
+                const int a = kstep_of(ks);
+                return row_ok && AB_BC(a >= 0 && a * 4 + 4 <= pb.w.k / 16) ? __ldg(reinterpret_cast<const unsigned*>(srow) + a) : 0u;
             };
-            uint4 nxt[8];
-            if (grp < n_ksteps) fetch(grp, nxt);
-            pdl_wait();
+            uint32_t sc_next = own_sc && grp < n_ksteps ? scale_word(grp) : 0u;
+            int slot = grp / P, sub = grp % P;
+            uint32_t parity = 0;
+            bool reused = false;   // the slot has held an earlier part of K
+            while (slot >= n_slots) { slot -= n_slots; parity ^= 1u; reused = true; }
             int j = 0;
             for (int ks = grp; ks < n_ksteps; ks += G_NG, ++j) {
-                uint4 cur[8];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) cur[c] = nxt[c];
-                if (ks + G_NG < n_ksteps) fetch(ks + G_NG, nxt);
+                const unsigned char* raw_slot = smRaw + slot * SB;
+                uint32_t sc4 = sc_next;
+                if (own_sc && ks + G_NG < n_ksteps) sc_next = scale_word(ks + G_NG);
+                // A slot's earlier content may have been another group's, and copies finish in any order: that copy may still
+                // be under way although this group's last one, issued after it, has landed. The phase bit alone cannot
+                // tell "two phases back" from "done", so first see that the earlier content has been used up. (Its
+                // copy had been issued by then, copies being issued in order, so this wait is at most one phase back.)
+                if (reused) wait_ok(&raw_empty[slot], parity ^ 1u);
+                wait_ok(&raw_full[slot], parity);
+                uint4 raw[8 / P], cur[8];
+                raw_fetch<F>(raw_slot, r_local, sub, raw);
+                if (F == FMT_FP4 && !own_sc) sc4 = *reinterpret_cast<const uint32_t*>(raw_slot + G_BM * G_RAW_ROW + r_local * 16 + sub * 4);
+                raw_dequant<F>(raw, sc4, cur);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&raw_empty[slot]);
+                sub += G_NG;
+                while (sub >= P) {
+                    sub -= P;
+                    if (++slot == n_slots) { slot = 0; parity ^= 1u; reused = true; }
+                }
                 put_stage(ks, j, cur);
             }
-        } else {
-            // One instance of the loop per weight format: ring depth, slot size and chunk counts are constants in it,
-            // the ring slots are walked with wrapping counters and the row's base addresses are computed once.
-            auto quant_loop = [&](auto fmt_c) {
-                constexpr int F = decltype(fmt_c)::value;
-                constexpr int rb = F == FMT_I8 ? 64 : 32, nq = rb / 16, epc = 16 * 64 / rb;
-                constexpr int slot_bytes = rb * G_BM + (F == FMT_FP4 ? G_BM * 4 : 0);
-                constexpr int depth = G_RAW_GROUP / slot_bytes > 6 ? 6 : G_RAW_GROUP / slot_bytes;   // own k-steps in flight
-                static_assert(depth >= 1, "raw ring too small");
-                unsigned char* ring = smRaw + grp * G_RAW_GROUP;
-                const int K = pb.w.k;
-                const unsigned char* wrow = reinterpret_cast<const unsigned char*>(pb.w.w) + (row_ok ? (size_t)row * K * rb / 64 : 0);
-                const unsigned char* srow = reinterpret_cast<const unsigned char*>(pb.w.scale) + (row_ok && F == FMT_FP4 ? (size_t)row * K / 16 : 0);
-                // chunk-major slot: chunk q of row r at q * 2048 + r * 16 (conflict-free read-back); NVFP4 block scales follow
-                auto issue = [&](int ks_abs, unsigned char* slot) {
-                    const int k0 = ks_abs * G_BK;
-#pragma unroll
-                    for (int q = 0; q < nq; ++q)
-                        cp_async_16(slot + q * 2048 + r_local * 16, wrow + (size_t)ks_abs * rb + q * 16,
-                                    row_ok && k0 + q * epc < K && AB_BC(ks_abs >= 0 && (size_t)ks_abs * rb + q * 16 + 16 <= (size_t)K * rb / 64));
-                    if (F == FMT_FP4) cp_async_4(slot + nq * 2048 + r_local * 4, srow + (size_t)ks_abs * 4, row_ok && k0 < K);
-                };
-#pragma unroll
-                for (int j = 0; j < depth - 1; ++j) {
-                    const int ks = grp + j * G_NG;
-                    if (ks < n_ksteps) issue(kstep_of(ks), ring + j * slot_bytes);
-                    cp_async_commit();
-                }
-                pdl_wait();
-                int j = 0, wslot = depth - 1, rslot = 0;
-                for (int ks = grp; ks < n_ksteps; ks += G_NG, ++j) {
-                    const int ks_a = ks + (depth - 1) * G_NG;
-                    if (ks_a < n_ksteps) issue(kstep_of(ks_a), ring + wslot * slot_bytes);
-                    if (++wslot == depth) wslot = 0;
-                    cp_async_commit();
-                    cp_async_wait<depth - 1>();   // all but the newest depth-1 groups have landed: k-step ks is there
-                    uint4 cur[8];
-                    raw_dequant(F, r_local, ring + rslot * slot_bytes, cur);
-                    if (++rslot == depth) rslot = 0;
-                    put_stage(ks, j, cur);
-                }
-            };
-            if (fmt == FMT_I8) quant_loop(std::integral_constant<int, FMT_I8>());
-            else quant_loop(std::integral_constant<int, FMT_FP4>());
-        }
+        };
+        if (fmt == FMT_I8) produce(std::integral_constant<int, FMT_I8>());
+        else if (fmt == FMT_FP4) produce(std::integral_constant<int, FMT_FP4>());
+        else produce(std::integral_constant<int, FMT_F16>());
+        pdl_wait();   // residuals and outputs belong to the preceding grids until here
 
         // ===== epilogue: thread = output feature (TMEM lane); groups take turns on chunks of 32 batch rows =====
         wait_ok(&accum_bar, 0);
         tc_fence_after();
-        float scale = 1.f;
-        if (row_ok) scale = fmt == FMT_I8 ? reinterpret_cast<const float*>(pb.w.scale)[row] : pb.w.tscale;
         const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         const int n_valid = min(g.n_tile, g.rows - n0);
         const int n_chunks = (n_valid + 31) / 32;
@@ -472,7 +469,7 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         // Preferred way out: the finished tile is laid out in shared memory as [batch row][128 features] fp16 (the
         // operand stages are idle by now) and leaves through the TMA unit in full lines; the unit clips rows and
         // features beyond the matrix. A residual tile comes in the same way and is updated in place.
-        __half* stg = reinterpret_cast<__half*>(smA);
+        __half* stg = reinterpret_cast<__half*>(base);
         const bool staged = pb.tma_out != 0;
         auto stage32 = [&](int ci, const float* v) {
             __half* t = stg + (size_t)ci * 32 * G_BM + r_local;
@@ -525,11 +522,8 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         if (!SPLIT || pb.ksplit == 1) {
             fetch_resid();
             for (int ci = grp; ci < n_chunks; ci += G_NG) {
-                uint32_t raw[32];
-                tc_ld32(lane_addr + (uint32_t)(ci * 32), raw);
                 float v[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(raw[i]);
+                tc_ld32(lane_addr + (uint32_t)(ci * 32), reinterpret_cast<uint32_t*>(v));
                 emit(ci, v);
             }
             flush();
@@ -548,11 +542,11 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             fetch_resid(false);
             for (int ci = grp; ci < n_chunks; ci += G_NG) {
                 if (ci % nz == z) continue;
-                uint32_t raw[32];
-                tc_ld32(lane_addr + (uint32_t)(ci * 32), raw);
+                float v[32];
+                tc_ld32(lane_addr + (uint32_t)(ci * 32), reinterpret_cast<uint32_t*>(v));
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                    if (ci * 32 + i < g.n_tile) __stcg(mine + (size_t)(ci * 32 + i) * G_BM + r_local, __uint_as_float(raw[i]));
+                    if (ci * 32 + i < g.n_tile) __stcg(mine + (size_t)(ci * 32 + i) * G_BM + r_local, v[i]);
             }
             __threadfence();
             epi_sync();
@@ -596,15 +590,14 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
                 for (int kk = k0; kk < k1; ++kk) {
                     if (kk % G_NG != grp) continue;
                     const int ci = z + kk * nz;
-                    uint32_t raw[32];
-                    tc_ld32(lane_addr + (uint32_t)(ci * 32), raw);
-                    float v[32];
+                    float own[32], v[32];
+                    tc_ld32(lane_addr + (uint32_t)(ci * 32), reinterpret_cast<uint32_t*>(own));
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = 0.f;
                     for (int zz = 0; zz < nz; ++zz) {
                         if (zz == z) {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(raw[i]);
+                            for (int i = 0; i < 32; ++i) v[i] += own[i];
                         } else {
                             const float* src = reinterpret_cast<const float*>(recv + (size_t)((kk - k0) * (nz - 1) + (zz < z ? zz : zz - 1)) * G_CHUNK_F32) + r_local;
 #pragma unroll
@@ -624,64 +617,77 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         tc_fence_before();
     } else if (warp == 4 * G_NG) {
         // ===== activation tiles by TMA =====
-        if (lane == 0) {
-            const CUtensorMap* map = &maps.m[pi];
-            pdl_wait();
-            for (int ks = 0; ks < n_ksteps; ++ks) {
-                const int s = ks % G_STAGES, f = ks / G_STAGES;
-                if (f > 0) wait_ok(&empty[s], (f - 1) & 1);
-                mbar_expect_tx(&full[s], (uint32_t)b_bytes);
-                for (int r = 0; r < g.n_tile; r += g.tma_rows)
-                    tma_load_2d(smB + s * b_bytes + r * 128, map, kstep_of(ks) * G_BK, n0 + r, &full[s]);
+        const CUtensorMap* map = &maps.m[pi];
+        const bool two_boxes = g.tma_rows < g.n_tile;
+        const int x_begin = raw_begin * per * G_BK, x_end = raw_end * per * G_BK;
+        int x = kstep_of(0) * G_BK;   // the k-steps in rotated order, walked without divisions
+        uint32_t parity = 1;          // the first round finds every stage free
+        pdl_wait();
+        for (int ks0 = 0; ks0 < n_ksteps; ks0 += G_STAGES, parity ^= 1u) {
+#pragma unroll
+            for (int s = 0; s < G_STAGES; ++s) {
+                if (ks0 + s >= n_ksteps) break;
+                if (ks0 > 0) wait_ok(&empty[s], parity);
+                __syncwarp();
+                mbar_expect_tx_one(&full[s], (uint32_t)b_bytes);
+                tma_load_2d_one(smB + s * b_bytes, map, x, n0, &full[s]);
+                if (two_boxes) tma_load_2d_one(smB + s * b_bytes + g.tma_rows * 128, map, x, n0 + g.tma_rows, &full[s]);
+                x += G_BK;
+                if (x == x_end) x = x_begin;
             }
         }
+    } else if (warp == 4 * G_NG + 2) {
+        // ===== raw weights by TMA: never written by anybody, so they start before the preceding grid is done =====
+        const uint32_t bytes = (uint32_t)(G_BM * G_RAW_ROW + (pb.scale_map ? G_BM * 16 : 0));
+        int slot = 0;
+        uint32_t parity = 1;   // the first round finds every slot free
+        for (int i = 0; i < n_raw; ++i) {
+            if (i >= n_slots) wait_ok(&raw_empty[slot], parity);
+            __syncwarp();
+            unsigned char* dst = smRaw + slot * slot_bytes;
+            const int ra = raw_of(i);
+            mbar_expect_tx_one(&raw_full[slot], bytes);
+            tma_load_2d_one(dst, &maps.w[pi], ra * G_RAW_ROW, m0, &raw_full[slot]);
+            if (pb.scale_map) tma_load_2d_one(dst + G_BM * G_RAW_ROW, &maps.s[pi], ra * 16, m0, &raw_full[slot]);
+            if (++slot == n_slots) { slot = 0; parity ^= 1u; }
+        }
     } else if (warp == 4 * G_NG + 1) {
-        // ===== MMA issue =====
-        if (lane == 0) {
-            // One thread feeds the tensor core, so its instruction stream is kept short: descriptors are built
-            // once, a stage or a 16-input step further is an add to the (address >> 4) field.
-            // An MMA is at most 256 batch rows wide and runs in steps of 64 of them: a 320-row tile is issued as
-            // 192 + 128 on separate TMEM columns (160 + 160 would cost as much as 192 + 192).
-            const bool two = g.n_first < g.n_tile;
-            const uint32_t idesc = umma_idesc_f16(g.n_first), idesc1 = umma_idesc_f16(two ? g.n_tile - g.n_first : 16);
-            const uint64_t da0 = umma_desc_sw128(smA), db0 = umma_desc_sw128(smB);
-            const uint64_t a_stage = (uint64_t)(G_A_BYTES >> 4), b_stage = (uint64_t)(b_bytes >> 4);
+        // ===== MMA issue: the whole warp walks the loop, one elected lane issues =====
+        // One lane feeds the tensor core, so its instruction stream is kept short: descriptors are built
+        // once, a stage or a 16-input step further is an add to the (address >> 4) field.
+        // An MMA is at most 256 batch rows wide and runs in steps of 64 of them: a 320-row tile is issued as
+        // 192 + 128 on separate TMEM columns (160 + 160 would cost as much as 192 + 192).
+        const uint32_t idesc = umma_idesc_f16(g.n_first);
+        const uint64_t db0 = umma_desc_sw128(smB), b_stage = (uint64_t)(b_bytes >> 4);
+        // unrolled over the stages: stage index, descriptors and barrier addresses are compile-time offsets
+        auto issue = [&](auto two_c) {
+            constexpr bool TWO = decltype(two_c)::value;
+            const uint32_t idesc1 = TWO ? umma_idesc_f16(g.n_tile - g.n_first) : 0u, d1 = tmem_base + (uint32_t)g.n_first;
             const uint64_t b_half = (uint64_t)((g.n_first * 128) >> 4);
-            const uint32_t d1 = tmem_base + (uint32_t)g.n_first;
-            // unrolled over the stages: stage index, descriptors and barrier addresses are compile-time offsets
             uint32_t parity = 0;
             for (int ks0 = 0; ks0 < n_ksteps; ks0 += G_STAGES, parity ^= 1u) {
 #pragma unroll
                 for (int s = 0; s < G_STAGES; ++s) {
-                    const int ks = ks0 + s;
-                    if (ks >= n_ksteps) break;
-                    const uint64_t da = da0 + (uint64_t)s * a_stage, db = db0 + (uint64_t)s * b_stage;
+                    if (ks0 + s >= n_ksteps) break;
+                    const uint64_t db = db0 + (uint64_t)s * b_stage;
+                    const uint32_t ta = tmem_base + (uint32_t)(g.a_col0 + s * G_A_COLS);
                     wait_ok(&full[s], parity);
+                    __syncwarp();
                     tc_fence_after();
-                    const uint32_t acc0 = ks > 0 ? 1u : 0u;
-                    // advancing 16 inputs = 32 bytes inside the swizzle row: +2 in the (address >> 4) field
-                    if (G_A_TMEM) {
-                        const uint32_t ta = tmem_base + (uint32_t)(g.a_col0 + s * G_A_COLS);
+                    const uint32_t acc0 = s > 0 || ks0 > 0 ? 1u : 0u;
 #pragma unroll
-                        for (int k4 = 0; k4 < G_BK / 16; ++k4) {   // 16 inputs = 8 columns of the weight stage
-                            const uint32_t acc = k4 ? 1u : acc0;
-                            tc_mma_f16_ts(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, acc);
-                            if (two) tc_mma_f16_ts(d1, ta + (uint32_t)(8 * k4), db + b_half + (uint64_t)(2 * k4), idesc1, acc);
-                        }
-                    } else {
-                        tc_mma_f16(tmem_base, da, db, idesc, acc0);
-                        if (two) tc_mma_f16(d1, da, db + b_half, idesc1, acc0);
-#pragma unroll
-                        for (int k4 = 1; k4 < G_BK / 16; ++k4) {
-                            tc_mma_f16(tmem_base, da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, 1u);
-                            if (two) tc_mma_f16(d1, da + (uint64_t)(2 * k4), db + b_half + (uint64_t)(2 * k4), idesc1, 1u);
-                        }
+                    for (int k4 = 0; k4 < G_BK / 16; ++k4) {   // 16 inputs = 8 columns of the weight stage, 32 bytes of the swizzle row
+                        const uint32_t acc = k4 ? 1u : acc0;
+                        tc_mma_f16_one(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, acc);
+                        if (TWO) tc_mma_f16_one(d1, ta + (uint32_t)(8 * k4), db + b_half + (uint64_t)(2 * k4), idesc1, acc);
                     }
-                    tc_commit(&empty[s]);   // the stage may be refilled once these MMAs have read it
+                    tc_commit_one(&empty[s]);   // the stage may be refilled once these MMAs have read it
                 }
             }
-            tc_commit(&accum_bar);
-        }
+        };
+        if (g.n_first < g.n_tile) issue(std::true_type());
+        else issue(std::false_type());
+        tc_commit_one(&accum_bar);
         tc_fence_before();
     }
     __syncthreads();
@@ -750,13 +756,11 @@ struct GroupShape {
     int n_split_tiles;
 };
 
-// Shared memory of a block (beyond the 1 KB alignment slack): operand stages + raw weight rings.
-size_t block_smem(int n_tile) {
-    if (!G_A_TMEM) return (size_t)G_STAGES * (G_A_BYTES + (size_t)n_tile * 128) + G_RAW_BYTES;
-    // activation stages + raw rings, and some more for the epilogue (output staging, split-K slices), up to 224 KB
-    const size_t need = (size_t)G_STAGES * n_tile * 128 + G_RAW_BYTES, want = need + 48 * 1024;
-    return want < 224 * 1024 ? want : (need > 224 * 1024 ? need : 224 * 1024);
-}
+// Shared memory of a block (beyond the 1 KB alignment slack): a block owns its SM (registers), so it takes all of it.
+constexpr size_t G_SMEM = 225 * 1024;
+size_t block_smem(int n_tile) { (void)n_tile; return G_SMEM; }
+// ... of which the raw weight slots get what the operand stages leave.
+size_t raw_smem(int n_tile) { return G_SMEM - (size_t)G_STAGES * n_tile * 128; }
 // Split K: how many of its own chunks a block can fetch the other blocks' partial sums for at a time. They land
 // in the operand stages behind the output staging area.
 int split_recv_slots(int n_tile, int ks) {
@@ -771,10 +775,10 @@ int split_recv_slots(int n_tile, int ks) {
 GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm) {
     GroupShape gs = {};
     if (rows <= 256) { gs.n_tile = (rows + 15) & ~15; gs.n_first = gs.tma_rows = gs.n_tile; }
-    else if (rows <= 320) { gs.n_tile = (rows + 31) & ~31; gs.n_first = 192; gs.tma_rows = gs.n_tile % 64 ? 32 : 64; }
+    else if (rows <= 320) { gs.n_tile = (rows + 31) & ~31; gs.n_first = 192; gs.tma_rows = gs.n_tile / 2; }
     else { gs.n_tile = gs.n_first = gs.tma_rows = 256; }
     gs.tmem_cols = 32;
-    const int a_cols = G_A_TMEM ? G_STAGES * G_A_COLS : 0;   // weight stages behind the accumulators
+    constexpr int a_cols = G_STAGES * G_A_COLS;   // weight stages behind the accumulators
     while (gs.tmem_cols < ((gs.n_tile + 31) & ~31) + a_cols) gs.tmem_cols *= 2;
     gs.n_tiles_y = (rows + gs.n_tile - 1) / gs.n_tile;
     int base_ctas = 0, slow_ctas = 0;
@@ -859,6 +863,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
     GemmMaps maps;
     g.n_prob = n; g.rows = rows; g.n_tile = gs.n_tile; g.n_first = gs.n_first; g.tma_rows = gs.tma_rows; g.tmem_cols = gs.tmem_cols;
     g.a_col0 = (gs.n_tile + 31) & ~31;
+    g.raw_bytes = (int)raw_smem(gs.n_tile);
     g.recv_off = (gs.n_tile + 31) / 32 * 32 * G_BM * 2;
     g.counters = reinterpret_cast<unsigned*>(scratch);
     g.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + (size_t)G_COUNTERS * 4) : nullptr;
@@ -895,6 +900,22 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
             set_error("gemm: cuTensorMapEncodeTiled failed with %d (rows=%d k=%d)", (int)cr, rows, m.k);
             return ERR_CUDA;
         }
+        // weights: rows as they are stored; the block scales need a row pitch of a multiple of 16 bytes
+        pb.scale_map = m.fmt == FMT_FP4 && m.k % 256 == 0 && ((uintptr_t)m.scale & 15) == 0 ? 1 : 0;
+        for (int which = 0; which < 1 + pb.scale_map; ++which) {
+            const cuuint64_t pitch = which ? m.k / 16 : (m.fmt == FMT_F16 ? 2ull * m.k : m.fmt == FMT_I8 ? (cuuint64_t)m.k : m.k / 2);
+            const cuuint64_t wdim[2] = {pitch, (cuuint64_t)m.n_out};
+            const cuuint32_t wbox[2] = {which ? 16u : (cuuint32_t)G_RAW_ROW, (cuuint32_t)G_BM};
+            const CUresult cw = encode(which ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                                       const_cast<void*>(which ? m.scale : m.w), wdim, &pitch, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                       which ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (cw != CUDA_SUCCESS) {
+                set_error("gemm: cuTensorMapEncodeTiled (weights) failed with %d (n_out=%d k=%d fmt=%d)", (int)cw, m.n_out, m.k, m.fmt);
+                return ERR_CUDA;
+            }
+        }
+        if (!pb.scale_map) maps.s[i] = maps.w[i];
         // output / residual tiles through the TMA unit when the row pitch and the pointers allow it
         pb.tma_out = (m.n_out % 8 == 0 && m.n_out >= G_BM && ((uintptr_t)op.y & 15) == 0 &&
                       (op.epi != EPI_RESID || ((uintptr_t)op.resid & 15) == 0)) ? 1 : 0;
@@ -917,7 +938,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
             }
         }
     }
-    for (int i = n; i < G_MAX_OPS; ++i) { maps.m[i] = maps.m[0]; maps.y[i] = maps.m[0]; maps.r[i] = maps.m[0]; }
+    for (int i = n; i < G_MAX_OPS; ++i) maps.m[i] = maps.y[i] = maps.r[i] = maps.w[i] = maps.s[i] = maps.m[0];
 
     const size_t smem = 1024 + block_smem(gs.n_tile);
     {

@@ -209,6 +209,24 @@ def test_batched_product_split_k_batch_sizes(rows):
         assert torch.equal(_gemm(pm, x.cuda(), epi, r), got)
 
 
+@pytest.mark.parametrize("fmt,rows,n,k", [("none", 320, 4096, 4096), ("int8", 320, 2048, 4096), ("nvfp4", 320, 2048, 8192),
+                                          ("none", 256, 2048, 4160), ("int8", 40, 300, 8256), ("nvfp4", 40, 300, 8512)])
+def test_batched_product_recycles_its_weight_slots(fmt, rows, n, k):
+    """The weight slots in shared memory are reused many times while copies complete in any order (tall batches leave the
+    fewest slots; one, two or four k-steps of 64 inputs per slot, the last slot partly used): every launch gives the same
+    bits, and the right ones."""
+    from albatross_b200 import quant
+    torch.manual_seed(rows + k)
+    w = torch.randn(n, k, device="cuda") * 0.02
+    x = torch.randn(rows, k, device="cuda").half()
+    pm = quant.quantize(w, None if fmt == "none" else fmt)
+    want = (x.double() @ pm.dequantize().double().t()).cpu().numpy()
+    got = _gemm(pm, x)
+    assert rel_err(got.float().cpu().numpy(), want) < 3e-3          # fp16 output rounding, as in the tests above
+    for _ in range(20):
+        assert torch.equal(_gemm(pm, x), got)
+
+
 def test_batched_product_small_k_and_epilogues():
     """Adapter-sized products (K = 16 ... 480, not multiples of the 64-input k-step) and the fused epilogues."""
     from albatross_b200 import _lib, quant
