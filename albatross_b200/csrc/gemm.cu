@@ -28,12 +28,15 @@
 // blocks' fp32 partial sums of them from a scratch area with bulk copies and adding them in a fixed order. Launched with
 // programmatic stream serialisation the kernel starts its weight stream before it waits for its predecessor.
 //
-// What bounds it: from 256 batch rows on the tensor core (a k-step of 320 rows takes 717 cycles of 640 at its rate,
-// 256 rows 559 of 512); below that the hand-over between the warps, about 450 cycles a k-step whatever the batch.
-// 16384 x 4096, back to back: 320 rows nvfp4 39.2 -> 34.4 us, 64 rows nvfp4 32.0 -> 19.7, 8 rows int8 32.6 -> 22.0, against
+// What bounds it: from 256 batch rows on the tensor core (a k-step of 320 rows takes 670 cycles of 640 at its rate); below
+// that the memory and the hand-over between the warps, about 390 cycles a k-step whatever the batch (int8 rows at the
+// copy bandwidth: 350). Around the main loop a block spends 1 us before it (tensor memory, barriers, first rows on their
+// way) and 1 - 3 us behind it; the exchange of a split K costs 5 us.
+// 16384 x 4096, back to back: 320 rows nvfp4 39.2 -> 33.3 us, 64 rows nvfp4 32.0 -> 17.9, 8 rows int8 32.6 -> 19.7, against
 // the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below).
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "gemm.cuh"
@@ -69,7 +72,6 @@ struct GemmProb {
     const __half* resid;
     __half* y;
     int epi;
-    int cta_base;     // first blockIdx.x of this product
     int ksplit;       // blocks that share one output tile along K
     int tile_base;    // first split-K tile id (counter / partial index)
     long long part_base;   // float offset of its split-K partial sums in the scratch area
@@ -78,6 +80,7 @@ struct GemmProb {
     int recv_slots;   // split K: own chunks whose slices fit the receive area at a time
 };
 struct GemmGroup {
+    int cta_base[G_MAX_OPS];   // first blockIdx.x of each product (unused ones: INT_MAX)
     GemmProb pr[G_MAX_OPS];
     int n_prob;
     int rows;       // batch rows (B*T)
@@ -276,7 +279,6 @@ template <int EPI>
 __device__ __forceinline__ float apply_epi_t(float o) {
     if (EPI == EPI_TANH) return tanhf(o);
     if (EPI == EPI_SIGMOID) return sigmoidf_(o);
-    if (EPI == EPI_RELU2) { o = fmaxf(o, 0.f); return o * o; }
     return o;
 }
 __device__ __forceinline__ float apply_epi(int epi, float o) {
@@ -289,57 +291,58 @@ __device__ __forceinline__ float apply_epi(int epi, float o) {
 }
 
 // SPLIT: some product of the launch is split along K (the lean instance is compiled without that ending).
-template <bool SPLIT>
-__global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ GemmMaps maps,
-                                                        const __grid_constant__ GemmGroup g) {
+// KS: k-steps per operand stage. The hand-over of a stage between the warps (waits, elections, commits) costs about 300
+// cycles, an MMA of up to 64 batch rows 34: with up to 128 batch rows two k-steps share a hand-over (16384 x 4096, 8 rows
+// int8: 22.0 -> 19.7 us, 128 rows: 23.9 -> 21.0). Taller tiles are bound by the tensor core and need the shared memory for
+// the depth of the ring.
+template <bool SPLIT, int KS>
+__device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup& g) {
     extern __shared__ __align__(1024) unsigned char gsm[];
-    __shared__ uint64_t full[G_STAGES], empty[G_STAGES], raw_full[G_RAW_SLOTS], raw_empty[G_RAW_SLOTS], accum_bar, resid_bar, recv_bar;
+    constexpr int N_BARS = 2 * G_STAGES + 2 * G_RAW_SLOTS + 3;
+    __shared__ uint64_t bars[N_BARS];
+    uint64_t *full = bars, *empty = full + G_STAGES, *raw_full = empty + G_STAGES, *raw_empty = raw_full + G_RAW_SLOTS;
+    uint64_t &accum_bar = bars[N_BARS - 3], &resid_bar = bars[N_BARS - 2], &recv_bar = bars[N_BARS - 1];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 4 * G_NG + 1) tmem_alloc(&tmem_base_s, (uint32_t)g.tmem_cols);
     // ---- which product, which tile, which K split
     int pi = 0;
-    while (pi + 1 < g.n_prob && (int)blockIdx.x >= g.pr[pi + 1].cta_base) ++pi;
+#pragma unroll
+    for (int i = 1; i < G_MAX_OPS; ++i) pi += (int)blockIdx.x >= g.cta_base[i] ? 1 : 0;
     const GemmProb& pb = g.pr[pi];
-    const int local = blockIdx.x - pb.cta_base;
-    const int m_tile = local / pb.ksplit, z = local - m_tile * pb.ksplit;
+    const int local = blockIdx.x - g.cta_base[pi];
+    const bool split = SPLIT && pb.ksplit > 1;
+    const int m_tile = split ? (int)((unsigned)local / (unsigned)pb.ksplit) : local, z = split ? local - m_tile * pb.ksplit : 0;
     const int m0 = m_tile * G_BM;
     const int n0 = blockIdx.y * g.n_tile;
     // K is dealt out in raw slots of `per` k-steps
     const int fmt = pb.w.fmt, per = raw_ksteps(fmt);
     const int total_ksteps = (pb.w.k + G_BK - 1) / G_BK, total_raw = (total_ksteps + per - 1) / per;
-    const int raw_begin = (int)((long long)total_raw * z / pb.ksplit), raw_end = (int)((long long)total_raw * (z + 1) / pb.ksplit);
+    const int raw_begin = split ? (int)((unsigned)total_raw * (unsigned)z / (unsigned)pb.ksplit) : 0;
+    const int raw_end = split ? (int)((unsigned)total_raw * (unsigned)(z + 1) / (unsigned)pb.ksplit) : total_raw;
     const int n_raw = raw_end - raw_begin;
-    const int n_ksteps = min(raw_end * per, total_ksteps) - raw_begin * per;
+    const int n_ksteps = min(raw_end * per, total_ksteps) - raw_begin * per, n_stages = (n_ksteps + KS - 1) / KS;
     // Blocks walk K in rotated order: at any moment they read different columns of the (shared) activation
     // matrix, instead of all hitting the same few L2 lines. (Not where the last slot is only partly used: it comes last.)
     const int rot = total_ksteps % per ? 0 : (int)((blockIdx.x * 7u + blockIdx.y * 3u) % (unsigned)n_raw);
     auto raw_of = [&](int i) { int k = i + rot; if (k >= n_raw) k -= n_raw; return raw_begin + k; };   // i-th slot worked on
-    auto kstep_of = [&](int i) { return raw_of(i / per) * per + i % per; };
     const int slot_bytes = raw_slot_bytes(fmt);
     const int n_slots = min(G_RAW_SLOTS, g.raw_bytes / slot_bytes);
 
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)gsm + 1023) & ~(uintptr_t)1023);
-    const int b_bytes = g.n_tile * 128;
-    unsigned char* smB = base;                                  // G_STAGES x n_tile x 128 B
+    const int tile_bytes = g.n_tile * 128, b_bytes = KS * tile_bytes;
+    unsigned char* smB = base;                                  // G_STAGES x KS x n_tile x 128 B
     unsigned char* smRaw = smB + G_STAGES * b_bytes;            // raw weight slots
 
-    if (tid == 0) {
-        for (int s = 0; s < G_STAGES; ++s) {
-            mbar_init(&full[s], 5);   // the four warps of the group that owns the k-step + the TMA thread's expect_tx
-            mbar_init(&empty[s], 1);
-        }
-        for (int s = 0; s < n_slots; ++s) {
-            mbar_init(&raw_full[s], 1);
-            mbar_init(&raw_empty[s], 4 * per);   // the four warps of the group that owns each of its k-steps
-        }
-        mbar_init(&accum_bar, 1);
-        mbar_init(&resid_bar, 1);
-        mbar_init(&recv_bar, 1);
+    if (tid < N_BARS) {
+        // full: the four warps of the group that owns the stage + the activation warp's expect_tx; raw_empty: the four warps
+        // of the owning group, for every stage that takes part of the slot
+        const int i = tid - 2 * G_STAGES;
+        mbar_init(&bars[tid], tid < G_STAGES ? 5u : (i >= G_RAW_SLOTS && i < 2 * G_RAW_SLOTS ? 4u * (unsigned)(per > KS ? per / KS : 1) : 1u));
         fence_mbar_init();
-        s_failed = 0;
+        if (tid == 0) s_failed = 0;
     }
-    if (warp == 4 * G_NG + 1) tmem_alloc(&tmem_base_s, (uint32_t)g.tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -371,21 +374,6 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         float scale = 1.f;   // of the output row; requested here, used in the epilogue
         if (row_ok) scale = fmt == FMT_I8 ? __ldg(reinterpret_cast<const float*>(pb.w.scale) + row) : pb.w.tscale;
 
-        // de-quantised k-step -> operand stage (swizzled), then tell the MMA warp
-        // (j = how many k-steps this group has done before; with as many groups as stages a group always fills the
-        // same stage)
-        auto put_stage = [&](int ks, int j, const uint4* cur) {
-            const int s = G_NG == G_STAGES ? grp : ks % G_STAGES, f = G_NG == G_STAGES ? j : ks / G_STAGES;
-            if (f > 0) wait_ok(&empty[s], (f - 1) & 1);
-            tc_fence_after();   // the MMAs that read this stage are complete (their commit released it)
-            // this thread's 64 inputs = 32 registers -> 32 columns of its own TMEM lane
-            tc_st32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g.a_col0 + s * G_A_COLS),
-                    reinterpret_cast<const uint32_t*>(cur));
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);   // one arrival per warp of the owning group
-        };
-
         // One instance of the loop per weight format: chunk counts are constants in it, slots are walked with wrapping counters.
         auto produce = [&](auto fmt_c) {
             constexpr int F = decltype(fmt_c)::value;
@@ -394,37 +382,67 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             const bool own_sc = F == FMT_FP4 && !pb.scale_map;
             const unsigned char* srow = reinterpret_cast<const unsigned char*>(pb.w.scale) + (F == FMT_FP4 && row_ok ? (size_t)row * (pb.w.k / 16) : 0);
             auto scale_word = [&](int ks) -> uint32_t {
-                const int a = kstep_of(ks);
+                if (ks >= n_ksteps) return 0u;
+                const int a = raw_of(ks / P) * P + ks % P;
                 return row_ok && AB_BC(a >= 0 && a * 4 + 4 <= pb.w.k / 16) ? __ldg(reinterpret_cast<const unsigned*>(srow) + a) : 0u;
             };
-            uint32_t sc_next = own_sc && grp < n_ksteps ? scale_word(grp) : 0u;
-            int slot = grp / P, sub = grp % P;
+            uint32_t sc_next = own_sc ? scale_word(grp * KS) : 0u;
+            int slot = 0, sub = 0;
             uint32_t parity = 0;
             bool reused = false;   // the slot has held an earlier part of K
-            while (slot >= n_slots) { slot -= n_slots; parity ^= 1u; reused = true; }
-            int j = 0;
-            for (int ks = grp; ks < n_ksteps; ks += G_NG, ++j) {
-                const unsigned char* raw_slot = smRaw + slot * SB;
-                uint32_t sc4 = sc_next;
-                if (own_sc && ks + G_NG < n_ksteps) sc_next = scale_word(ks + G_NG);
-                // A slot's earlier content may have been another group's, and copies finish in any order: that copy may still
-                // be under way although this group's last one, issued after it, has landed. The phase bit alone cannot
-                // tell "two phases back" from "done", so first see that the earlier content has been used up. (Its
-                // copy had been issued by then, copies being issued in order, so this wait is at most one phase back.)
-                if (reused) wait_ok(&raw_empty[slot], parity ^ 1u);
-                wait_ok(&raw_full[slot], parity);
-                uint4 raw[8 / P], cur[8];
-                raw_fetch<F>(raw_slot, r_local, sub, raw);
-                if (F == FMT_FP4 && !own_sc) sc4 = *reinterpret_cast<const uint32_t*>(raw_slot + G_BM * G_RAW_ROW + r_local * 16 + sub * 4);
-                raw_dequant<F>(raw, sc4, cur);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[slot]);
-                sub += G_NG;
+            auto advance = [&](int n) {
+                sub += n;
                 while (sub >= P) {
                     sub -= P;
                     if (++slot == n_slots) { slot = 0; parity ^= 1u; reused = true; }
                 }
-                put_stage(ks, j, cur);
+            };
+            advance(grp * KS);
+            int stage = grp % G_STAGES;
+            uint32_t e_parity = 1;   // the first round finds every operand stage free
+            for (int st = grp; st < n_stages; st += G_NG) {
+#pragma unroll 1
+                for (int h = 0; h < KS; ++h) {
+                    const int ks = st * KS + h;
+                    if (KS > 1 && ks >= n_ksteps) {   // an odd last k-step
+                        if (P > 1 && lane == 0) mbar_arrive(&raw_empty[slot]);
+                        break;
+                    }
+                    const unsigned char* raw_slot = smRaw + slot * SB;
+                    uint32_t sc4 = sc_next;
+                    if (own_sc) sc_next = scale_word(h < KS - 1 ? ks + 1 : ks + 1 + (G_NG - 1) * KS);
+                    if (h == 0 || P == 1) {
+                        // A slot's earlier content may have been another group's, and copies finish in any order: that copy
+                        // may still be under way although this group's last one, issued after it, has landed. The phase bit
+                        // alone cannot tell "two phases back" from "done", so first see that the earlier content has been
+                        // used up. (Its copy had been issued by then - copies are issued in order and there are more slots
+                        // than the groups are apart - so this wait is at most one phase back.)
+                        if (reused) wait_ok(&raw_empty[slot], parity ^ 1u);
+                        wait_ok(&raw_full[slot], parity);
+                    }
+                    uint4 raw[8 / P], cur[8];
+                    raw_fetch<F>(raw_slot, r_local, sub, raw);
+                    if (F == FMT_FP4 && !own_sc) sc4 = *reinterpret_cast<const uint32_t*>(raw_slot + G_BM * G_RAW_ROW + r_local * 16 + sub * 4);
+                    raw_dequant<F>(raw, sc4, cur);
+                    if (h == KS - 1 || P == 1) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&raw_empty[slot]);
+                    }
+                    advance(1);
+                    if (h == 0) {
+                        if (st >= G_STAGES) wait_ok(&empty[stage], e_parity);
+                        tc_fence_after();   // the MMAs that read this stage are complete (their commit released it)
+                    }
+                    // this thread's 64 inputs = 32 registers -> 32 columns of its own TMEM lane
+                    tc_st32(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(g.a_col0 + (stage * KS + h) * G_A_COLS),
+                            reinterpret_cast<const uint32_t*>(cur));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[stage]);   // one arrival per warp of the owning group
+                advance((G_NG - 1) * KS);
+                stage += G_NG;
+                if (stage >= G_STAGES) { stage -= G_STAGES; e_parity ^= 1u; }
             }
         };
         if (fmt == FMT_I8) produce(std::integral_constant<int, FMT_I8>());
@@ -476,9 +494,16 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             auto body = [&](auto E) {
                 constexpr int EP = decltype(E)::value;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    if (EP == EPI_RESID) t[i * G_BM] = __hadd(t[i * G_BM], __float2half_rn(v[i] * scale));
-                    else t[i * G_BM] = __float2half_rn(apply_epi_t<EP>(rh(v[i] * scale)));
+                for (int i = 0; i < 32; i += 2) {   // two batch rows at a time; the same roundings as one at a time
+                    __half2 h = __floats2half2_rn(v[i] * scale, v[i + 1] * scale);
+                    if (EP == EPI_RELU2) { h = __hmax2(h, __half2(__half(0.f), __half(0.f))); h = __hmul2(h, h); }
+                    if (EP == EPI_RESID) h = __hadd2(__halves2half2(t[i * G_BM], t[(i + 1) * G_BM]), h);
+                    if (EP == EPI_TANH || EP == EPI_SIGMOID) {
+                        const float2 f = __half22float2(h);
+                        h = __floats2half2_rn(apply_epi_t<EP>(f.x), apply_epi_t<EP>(f.y));
+                    }
+                    t[i * G_BM] = __low2half(h);
+                    t[(i + 1) * G_BM] = __high2half(h);
                 }
             };
             switch (epi) {
@@ -502,7 +527,7 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             }
         };
         // With split K every block of a tile finishes the chunks ci = z, z + ksplit, ... of it.
-        auto my_chunk = [&](int ci) { return pb.ksplit == 1 || ci % pb.ksplit == z; };
+        auto my_chunk = [&](int ci) { return !split || ci % pb.ksplit == z; };
         // residual tiles on their way in
         auto fetch_resid = [&](bool wait = true) {
             if (!(staged && epi == EPI_RESID)) return;
@@ -519,7 +544,7 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             if (staged && r_local == 0) bulk_drain_reads();   // the shared memory must outlive the unit's reads
         };
 
-        if (!SPLIT || pb.ksplit == 1) {
+        if (!split) {
             fetch_resid();
             for (int ci = grp; ci < n_chunks; ci += G_NG) {
                 float v[32];
@@ -620,20 +645,26 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         const CUtensorMap* map = &maps.m[pi];
         const bool two_boxes = g.tma_rows < g.n_tile;
         const int x_begin = raw_begin * per * G_BK, x_end = raw_end * per * G_BK;
-        int x = kstep_of(0) * G_BK;   // the k-steps in rotated order, walked without divisions
-        uint32_t parity = 1;          // the first round finds every stage free
+        int x = raw_of(0) * per * G_BK;   // the k-steps in rotated order, walked without divisions
+        uint32_t parity = 1;              // the first round finds every stage free
         pdl_wait();
-        for (int ks0 = 0; ks0 < n_ksteps; ks0 += G_STAGES, parity ^= 1u) {
+        for (int st0 = 0; st0 < n_stages; st0 += G_STAGES, parity ^= 1u) {
 #pragma unroll
             for (int s = 0; s < G_STAGES; ++s) {
-                if (ks0 + s >= n_ksteps) break;
-                if (ks0 > 0) wait_ok(&empty[s], parity);
+                if (st0 + s >= n_stages) break;
+                const int n_here = KS == 1 ? 1 : min(KS, n_ksteps - (st0 + s) * KS);
+                if (st0 > 0) wait_ok(&empty[s], parity);
                 __syncwarp();
-                mbar_expect_tx_one(&full[s], (uint32_t)b_bytes);
-                tma_load_2d_one(smB + s * b_bytes, map, x, n0, &full[s]);
-                if (two_boxes) tma_load_2d_one(smB + s * b_bytes + g.tma_rows * 128, map, x, n0 + g.tma_rows, &full[s]);
-                x += G_BK;
-                if (x == x_end) x = x_begin;
+                mbar_expect_tx_one(&full[s], (uint32_t)(n_here * tile_bytes));
+#pragma unroll
+                for (int h = 0; h < KS; ++h) {
+                    if (h >= n_here) break;
+                    unsigned char* dst = smB + s * b_bytes + h * tile_bytes;
+                    tma_load_2d_one(dst, map, x, n0, &full[s]);
+                    if (KS == 1 && two_boxes) tma_load_2d_one(dst + g.tma_rows * 128, map, x, n0 + g.tma_rows, &full[s]);
+                    x += G_BK;
+                    if (x == x_end) x = x_begin;
+                }
             }
         }
     } else if (warp == 4 * G_NG + 2) {
@@ -665,27 +696,31 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
             const uint32_t idesc1 = TWO ? umma_idesc_f16(g.n_tile - g.n_first) : 0u, d1 = tmem_base + (uint32_t)g.n_first;
             const uint64_t b_half = (uint64_t)((g.n_first * 128) >> 4);
             uint32_t parity = 0;
-            for (int ks0 = 0; ks0 < n_ksteps; ks0 += G_STAGES, parity ^= 1u) {
-#pragma unroll
+            for (int st0 = 0; st0 < n_stages; st0 += G_STAGES, parity ^= 1u) {
+#pragma unroll(KS == 1 ? G_STAGES : 1)
                 for (int s = 0; s < G_STAGES; ++s) {
-                    if (ks0 + s >= n_ksteps) break;
-                    const uint64_t db = db0 + (uint64_t)s * b_stage;
-                    const uint32_t ta = tmem_base + (uint32_t)(g.a_col0 + s * G_A_COLS);
+                    if (st0 + s >= n_stages) break;
+                    const int n_here = KS == 1 ? 1 : min(KS, n_ksteps - (st0 + s) * KS);
                     wait_ok(&full[s], parity);
                     __syncwarp();
                     tc_fence_after();
-                    const uint32_t acc0 = s > 0 || ks0 > 0 ? 1u : 0u;
 #pragma unroll
-                    for (int k4 = 0; k4 < G_BK / 16; ++k4) {   // 16 inputs = 8 columns of the weight stage, 32 bytes of the swizzle row
-                        const uint32_t acc = k4 ? 1u : acc0;
-                        tc_mma_f16_one(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, acc);
-                        if (TWO) tc_mma_f16_one(d1, ta + (uint32_t)(8 * k4), db + b_half + (uint64_t)(2 * k4), idesc1, acc);
+                    for (int h = 0; h < KS; ++h) {
+                        if (h >= n_here) break;
+                        const uint64_t db = db0 + (uint64_t)s * b_stage + (uint64_t)(h * (tile_bytes >> 4));
+                        const uint32_t ta = tmem_base + (uint32_t)(g.a_col0 + (s * KS + h) * G_A_COLS);
+#pragma unroll
+                        for (int k4 = 0; k4 < G_BK / 16; ++k4) {   // 16 inputs = 8 columns of the weight stage, 32 bytes of the swizzle row
+                            const uint32_t acc = h > 0 || k4 > 0 || s > 0 || st0 > 0 ? 1u : 0u;
+                            tc_mma_f16_one(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, acc);
+                            if (TWO) tc_mma_f16_one(d1, ta + (uint32_t)(8 * k4), db + b_half + (uint64_t)(2 * k4), idesc1, acc);
+                        }
                     }
                     tc_commit_one(&empty[s]);   // the stage may be refilled once these MMAs have read it
                 }
             }
         };
-        if (g.n_first < g.n_tile) issue(std::true_type());
+        if (KS == 1 && g.n_first < g.n_tile) issue(std::true_type());
         else issue(std::false_type());
         tc_commit_one(&accum_bar);
         tc_fence_before();
@@ -695,6 +730,15 @@ __global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ 
         tc_fence_after();
         tmem_dealloc(tmem_base, (uint32_t)g.tmem_cols);
     }
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(GT, 1) gemm_tc_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup g) {
+    gemm_block<SPLIT, 1>(maps, g);
+}
+template <bool SPLIT>
+__global__ void __launch_bounds__(GT, 1) gemm_tc2_kernel(const __grid_constant__ GemmMaps maps, const __grid_constant__ GemmGroup g) {
+    gemm_block<SPLIT, 2>(maps, g);
 }
 
 // In-register de-quantisation exactly as the product kernels do it, written out as fp32.
@@ -759,8 +803,10 @@ struct GroupShape {
 // Shared memory of a block (beyond the 1 KB alignment slack): a block owns its SM (registers), so it takes all of it.
 constexpr size_t G_SMEM = 225 * 1024;
 size_t block_smem(int n_tile) { (void)n_tile; return G_SMEM; }
-// ... of which the raw weight slots get what the operand stages leave.
-size_t raw_smem(int n_tile) { return G_SMEM - (size_t)G_STAGES * n_tile * 128; }
+// k-steps per operand stage (see gemm_tc_kernel) and what the stages leave for the raw weight slots: at least 4 slots of one
+// k-step per stage, 6 of two.
+int stage_ksteps(int n_tile) { return n_tile <= 128 ? 2 : 1; }
+size_t raw_smem(int n_tile) { return G_SMEM - (size_t)G_STAGES * stage_ksteps(n_tile) * n_tile * 128; }
 // Split K: how many of its own chunks a block can fetch the other blocks' partial sums for at a time. They land
 // in the operand stages behind the output staging area.
 int split_recv_slots(int n_tile, int ks) {
@@ -772,13 +818,37 @@ int split_recv_slots(int n_tile, int ks) {
     return fit < own_max ? fit : own_max;
 }
 
-GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm) {
+// Batch rows per block tile for more rows than one tile holds. A block's time is its k-steps times what one costs (the
+// tensor core's 2.1 cycles per batch row, the hand-over's 450 below that) plus what surrounds them, and a launch takes
+// as many of those as there are rounds of blocks over the SMs: the tile with the smallest product. With the fixed tile of 256
+// that this replaces, 768 rows of a 4096-row matrix kept 96 SMs busy (192 rows: 128 SMs), and r, k, v with their adapters
+// ended in a third round of ten blocks (768 rows int8, 4096 rows of 4096 inputs: 29.2 -> 25.8 us, of 16384: 89.9 -> 85.4).
+int pick_tile(const GemmOp* ops, int n, int rows, int n_sm) {
+    long long m_tiles = 0, ksteps = 1, best = 0;
+    for (int i = 0; i < n; ++i) {
+        m_tiles += (ops[i].w.n_out + G_BM - 1) / G_BM;
+        ksteps = std::max(ksteps, (long long)(ops[i].w.k + G_BK - 1) / G_BK);
+    }
+    int pick = 256;
+    for (int t = 320; t >= 128; t -= 32) {   // whole 32-row chunks: the next tile's rows are not this one's to store
+        const long long blocks = m_tiles * ((rows + t - 1) / t), rounds = (blocks + n_sm - 1) / n_sm;
+        const long long cost = rounds * (ksteps * std::max(450, 21 * t / 10) + 6000 + 15 * t);
+        if (best == 0 || cost < best) { best = cost; pick = t; }
+    }
+    return pick;
+}
+
+// fixed_tile: the tile of more than 320 batch rows (0: the best one).
+GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int fixed_tile = 0) {
     GroupShape gs = {};
     if (rows <= 256) { gs.n_tile = (rows + 15) & ~15; gs.n_first = gs.tma_rows = gs.n_tile; }
     else if (rows <= 320) { gs.n_tile = (rows + 31) & ~31; gs.n_first = 192; gs.tma_rows = gs.n_tile / 2; }
-    else { gs.n_tile = gs.n_first = gs.tma_rows = 256; }
+    else {
+        gs.n_tile = gs.n_first = gs.tma_rows = fixed_tile ? fixed_tile : pick_tile(ops, n, rows, n_sm > 0 ? n_sm : 148);
+        if (gs.n_tile > 256) { gs.n_first = 192; gs.tma_rows = gs.n_tile / 2; }
+    }
     gs.tmem_cols = 32;
-    constexpr int a_cols = G_STAGES * G_A_COLS;   // weight stages behind the accumulators
+    const int a_cols = G_STAGES * stage_ksteps(gs.n_tile) * G_A_COLS;   // weight stages behind the accumulators
     while (gs.tmem_cols < ((gs.n_tile + 31) & ~31) + a_cols) gs.tmem_cols *= 2;
     gs.n_tiles_y = (rows + gs.n_tile - 1) / gs.n_tile;
     int base_ctas = 0, slow_ctas = 0;
@@ -829,8 +899,9 @@ size_t gemm_group_scratch_bytes(const GemmOp* ops, int n, int rows) {
     if (!ops || n < 1 || n > G_MAX_OPS || rows <= 0) return 0;
     for (int i = 0; i < n; ++i)
         if (ops[i].w.n_out <= 0 || ops[i].w.k <= 0) return 0;
-    const GroupShape gs = group_shape(ops, n, rows, current_sm_count());
-    return (size_t)G_COUNTERS * 4 + (size_t)gs.part_floats * 4 + 256;
+    // (never less than for tiles of 256 rows: what a caller's scratch area has to hold does not depend on the tile picked)
+    const long long floats = std::max(group_shape(ops, n, rows, current_sm_count()).part_floats, group_shape(ops, n, rows, current_sm_count(), 256).part_floats);
+    return (size_t)G_COUNTERS * 4 + (size_t)floats * 4 + 256;
 }
 size_t gemm_scratch_bytes(const ab_mat& m, int rows) {
     GemmOp op = {};
@@ -881,7 +952,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
         AB_CHECK_ARG(m.fmt != FMT_FP4 || (m.k % 64 == 0 && ((uintptr_t)m.scale & 3) == 0), "gemm: NVFP4 needs k %% 64 == 0");
         GemmProb& pb = g.pr[i];
         pb.w = m; pb.resid = op.resid; pb.y = op.y; pb.epi = op.epi;
-        pb.cta_base = cta; pb.ksplit = gs.ksplit[i]; pb.tile_base = tile; pb.part_base = part;
+        g.cta_base[i] = cta; pb.ksplit = gs.ksplit[i]; pb.tile_base = tile; pb.part_base = part;
         pb.recv_slots = pb.ksplit > 1 ? split_recv_slots(gs.n_tile, pb.ksplit) : 0;
         const int m_tiles = (m.n_out + G_BM - 1) / G_BM;
         cta += m_tiles * pb.ksplit;
@@ -938,6 +1009,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
             }
         }
     }
+    for (int i = n; i < G_MAX_OPS; ++i) g.cta_base[i] = 0x7fffffff;
     for (int i = n; i < G_MAX_OPS; ++i) maps.m[i] = maps.y[i] = maps.r[i] = maps.w[i] = maps.s[i] = maps.m[0];
 
     const size_t smem = 1024 + block_smem(gs.n_tile);
@@ -945,8 +1017,8 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
         static PerDeviceOnce once;
         const int s = once.run(nullptr, [](DeviceProps& d) -> int {
             // the largest dynamic size the device allows (the kernels' static shared memory is under 1 KB)
-            AB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem_optin - 1024));
-            AB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem_optin - 1024));
+            for (auto k : {gemm_tc_kernel<false>, gemm_tc_kernel<true>, gemm_tc2_kernel<false>, gemm_tc2_kernel<true>})
+                AB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem_optin - 1024));
             return OK;
         });
         if (s != OK) return s;
@@ -965,8 +1037,9 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
     }
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
-    if (gs.n_split_tiles > 0) AB_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true>, maps, g));
-    else AB_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false>, maps, g));
+    const bool two = stage_ksteps(gs.n_tile) == 2, any_split = gs.n_split_tiles > 0;
+    AB_CUDA(cudaLaunchKernelEx(&cfg, two ? (any_split ? gemm_tc2_kernel<true> : gemm_tc2_kernel<false>)
+                                         : (any_split ? gemm_tc_kernel<true> : gemm_tc_kernel<false>), maps, g));
     return OK;
 }
 

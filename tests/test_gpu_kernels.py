@@ -152,6 +152,31 @@ def test_wkv7_sequences_around_the_chunk_size(B, H, T, shift):
     assert rel_err(S.cpu(), S_ref) < 1e-5
 
 
+@pytest.mark.parametrize("T", [2, 8, 9, 40, 67])
+def test_wkv7_sequences_do_not_depend_on_the_batch(T):
+    """Few heads are shared by two blocks each, many take one: the same bits either way, and the same as step by step."""
+    from albatross_b200 import RWKV7_BATCH_OP, _lib
+    torch.manual_seed(T)
+    B, H = 40, 2                                       # 80 heads: one block each; a single sequence: two blocks per head
+    kk = torch.nn.functional.normalize(torch.randn(B, T, H, 64), dim=-1).view(B, T, H * 64)
+    vec = [torch.randn(B, T, H * 64), -torch.rand(B, T, H * 64) * 2 - 0.5, torch.randn(B, T, H * 64), torch.randn(B, T, H * 64), -kk,
+           kk * torch.rand(B, T, H * 64)]
+    vec = [v.half().cuda() for v in vec]
+    S0 = torch.randn(B, H, 64, 64, device="cuda") * 0.3
+    S_all = S0.clone()
+    y_all = RWKV7_BATCH_OP(S_all, *vec)
+    for b in (0, 17, 39):
+        S = S0[b:b + 1].clone()
+        y = RWKV7_BATCH_OP(S, *[v[b:b + 1].contiguous() for v in vec])
+        assert torch.equal(y, y_all[b:b + 1]) and torch.equal(S, S_all[b:b + 1])
+        S = S0[b:b + 1].clone()
+        for t in range(T):
+            yt = RWKV7_BATCH_OP(S, *[v[b:b + 1, t:t + 1].contiguous() for v in vec])
+            assert torch.equal(yt, y_all[b:b + 1, t:t + 1])
+        assert torch.equal(S, S_all[b:b + 1])
+    assert _lib.device_status() == 0
+
+
 def test_wkv7_operator_rejects_bad_shapes():
     from albatross_b200 import _lib
     assert _lib.lib.ab_wkv7_fwd(1, 1, 96, 2, 16, 16, 16, 16, 16, 16, 16, 16, None) == -1
@@ -209,8 +234,23 @@ def test_batched_product_split_k_batch_sizes(rows):
         assert torch.equal(_gemm(pm, x.cuda(), epi, r), got)
 
 
+@pytest.mark.parametrize("rows", [321, 400, 511, 640, 768, 1025])
+@pytest.mark.parametrize("fmt,n,k,epi", [("int8", 4096, 512, 0), ("nvfp4", 300, 1024, 4), ("none", 16384, 128, 3)])
+def test_batched_product_tall_batches(fmt, n, k, epi, rows):
+    """More rows than one tile: whatever tile height the launcher picks, with a ragged last tile, residual and relu^2."""
+    from albatross_b200 import quant
+    torch.manual_seed(rows)
+    w = torch.randn(n, k, device="cuda") * 0.02
+    x, resid = torch.randn(rows, k, device="cuda").half(), torch.randn(rows, n, device="cuda").half()
+    pm = quant.quantize(w, None if fmt == "none" else fmt)
+    want = x.double() @ pm.dequantize().double().t()
+    want = torch.relu(want) ** 2 if epi == 3 else want + resid.double() if epi == 4 else want
+    got = _gemm(pm, x, epi, resid if epi == 4 else None)
+    assert rel_err(got.float().cpu().numpy(), want.cpu().numpy()) < 4e-3     # fp16 output rounding, as in the tests above
+
+
 @pytest.mark.parametrize("fmt,rows,n,k", [("none", 320, 4096, 4096), ("int8", 320, 2048, 4096), ("nvfp4", 320, 2048, 8192),
-                                          ("none", 256, 2048, 4160), ("int8", 40, 300, 8256), ("nvfp4", 40, 300, 8512)])
+                                          ("none", 256, 2048, 4160), ("none", 100, 256, 4160), ("int8", 128, 512, 4160), ("int8", 40, 300, 8256), ("nvfp4", 40, 300, 8512)])
 def test_batched_product_recycles_its_weight_slots(fmt, rows, n, k):
     """The weight slots in shared memory are reused many times while copies complete in any order (tall batches leave the
     fewest slots; one, two or four k-steps of 64 inputs per slot, the last slot partly used): every launch gives the same
