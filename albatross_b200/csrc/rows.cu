@@ -170,6 +170,137 @@ __global__ void __launch_bounds__(RT) ln_mix_rows_kernel(const __half* __restric
     }
 }
 
+// T > 1: layer norm and token-shift lerps of sequences in one pass. A block takes p.R consecutive rows of one sequence: the
+// normalised row of step t - 1 stays in registers as the shift of step t, only the row in front of the block's first is
+// normalised twice. The block with a sequence's first rows is the only one that touches its token-shift state: it
+// reads it for step 0 and stores the sequence's last normalised row at the end.
+// What bounds it: 2 bytes in and 2 * n_mix out per element (768 rows x 4096, six lerps: 44 MB, about 7 us at the copy
+// bandwidth), then the two block-wide sums per row. Alone on a cold cache 21 us there, 13.5 us with one lerp; the three
+// passes it replaces (norm, lerps with 2-byte accesses, state hand-over) took 62 and 27 us.
+template <int V>   // 16-byte chunks per thread: D <= 8 * RT * V
+__global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict__ x, const __half* __restrict__ w,
+                                                        const __half* __restrict__ b, const __grid_constant__ MixParams p, int R,
+                                                        int use_pdl) {
+    __shared__ float red[RT / 32];
+    const int n_chunks = (p.T + R - 1) / R, seq = blockIdx.x / n_chunks, t0 = (blockIdx.x - seq * n_chunks) * R;
+    const int nv = p.D / 8;
+    const uint4* xs = reinterpret_cast<const uint4*>(x + (size_t)seq * p.T * p.D);
+    uint4* state = reinterpret_cast<uint4*>(p.x_prev + (size_t)seq * p.D);
+    if (use_pdl) pdl_launch_dependents();
+    uint4 wv_[V], bv_[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const int i = threadIdx.x + v * RT;
+        if (i < nv) {
+            wv_[v] = reinterpret_cast<const uint4*>(w)[i];
+            bv_[v] = reinterpret_cast<const uint4*>(b)[i];
+        }
+    }
+    if (use_pdl) pdl_wait();
+    auto load = [&](int t, uint4* raw) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int i = threadIdx.x + v * RT;
+            // an ordinary (coherent) load that stays behind the wait above: the row was written by the preceding kernel
+            if (i < nv)
+                asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(raw[v].x), "=r"(raw[v].y), "=r"(raw[v].z), "=r"(raw[v].w)
+                             : "l"(xs + (size_t)t * nv + i)
+                             : "memory");
+        }
+    };
+    auto norm = [&](const uint4* raw, uint4* xn) {   // same rounding points as ln_rows
+        float s = 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            if (threadIdx.x + v * RT < nv) {
+                const __half2* h = reinterpret_cast<const __half2*>(&raw[v]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(h[e]); s += f.x + f.y; }
+            }
+        }
+        const float mean = block_sum_rt(s, red) / (float)p.D;
+        float q = 0.f;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            if (threadIdx.x + v * RT < nv) {
+                const __half2* h = reinterpret_cast<const __half2*>(&raw[v]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = __half22float2(h[e]);
+                    q += (f.x - mean) * (f.x - mean) + (f.y - mean) * (f.y - mean);
+                }
+            }
+        }
+        const float rstd = rsqrtf(block_sum_rt(q, red) / (float)p.D + 1e-5f);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const __half2* h = reinterpret_cast<const __half2*>(&raw[v]);
+            const __half2* wh = reinterpret_cast<const __half2*>(&wv_[v]);
+            const __half2* bh = reinterpret_cast<const __half2*>(&bv_[v]);
+            __half2* xh = reinterpret_cast<__half2*>(&xn[v]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(h[e]), wf = __half22float2(wh[e]), bf = __half22float2(bh[e]);
+                xh[e] = __floats2half2_rn((f.x - mean) * rstd * wf.x + bf.x, (f.y - mean) * rstd * wf.y + bf.y);
+            }
+        }
+    };
+    const int t1 = min(t0 + R, p.T);
+    uint4 raw[V], prev[V];
+    if (t0 > 0) {
+        load(t0 - 1, raw);
+        norm(raw, prev);
+    } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (threadIdx.x + v * RT < nv) prev[v] = state[threadIdx.x + v * RT];
+    }
+    load(t0, raw);
+    for (int t = t0; t < t1; ++t) {
+        uint4 xn[V];
+        norm(raw, xn);
+        if (t + 1 < t1) load(t + 1, raw);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const int i = threadIdx.x + v * RT;
+            if (i < nv) {
+                const __half2* ch = reinterpret_cast<const __half2*>(&xn[v]);
+                const __half2* ph = reinterpret_cast<const __half2*>(&prev[v]);
+                float c[8], d[8];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 cf = __half22float2(ch[e]), pf = __half22float2(ph[e]);
+                    c[2 * e] = cf.x; c[2 * e + 1] = cf.y;
+                    d[2 * e] = rh(pf.x - cf.x); d[2 * e + 1] = rh(pf.y - cf.y);
+                }
+                for (int j = 0; j < p.n_mix; ++j) {
+                    const uint4 mv = reinterpret_cast<const uint4*>(p.mix[j])[i];
+                    const __half2* mh = reinterpret_cast<const __half2*>(&mv);
+                    uint4 o;
+                    __half2* oh = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 mf = __half22float2(mh[e]);
+                        oh[e] = __floats2half2_rn(c[2 * e] + rh(d[2 * e] * mf.x), c[2 * e + 1] + rh(d[2 * e + 1] * mf.y));
+                    }
+                    reinterpret_cast<uint4*>(p.out[j] + ((size_t)seq * p.T + t) * p.D)[i] = o;
+                }
+                prev[v] = xn[v];
+            }
+        }
+    }
+    if (t0 == 0) {   // the state read above is replaced by the normalised last row
+        if (t1 < p.T) {
+            load(p.T - 1, raw);
+            norm(raw, prev);
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (threadIdx.x + v * RT < nv) state[threadIdx.x + v * RT] = prev[v];
+    }
+}
+
 // Greedy / noisy-greedy sampling of one token per row: argmax over the row of logit + U(0, noise)
 // (reference/utils.py:43-45 adds uniform noise and takes the first entry of a descending argsort). Ties go to the
 // lowest index. The noise is a counter-based hash of (seed, row, column): reproducible, not torch's generator.
@@ -178,34 +309,71 @@ __device__ __forceinline__ float sample_noise(uint32_t seed, uint32_t row, uint3
     x ^= x >> 16; x *= 0x7FEB352Du; x ^= x >> 15; x *= 0x846CA68Bu; x ^= x >> 16;
     return (float)(x >> 8) * (1.0f / 16777216.0f);   // [0, 1)
 }
-// NT threads per row: 1024 when there are only a few rows (a single row of 65536 logits is otherwise read by 256 threads,
-// 32 loads one after the other: 16 us), 256 otherwise.
+// What bounds it: reading the logits. The noise hash takes some fifteen integer operations, too many to draw it for every
+// logit (320 rows of 65536: 28.8 us); so the row is read in batches of SR_U 16-byte chunks per thread, the batch's plain
+// maximum over the block is taken first, and only chunks that can still reach it are looked at value by value: noise is
+// never negative and always below `noise`, so a logit v ends up in [v, v + noise]. Skipped are chunks strictly below; ties
+// and NaNs take the long way, the result is the same id.
+// (With the maximum over a warp instead of the block, eight chunks per warp and batch still took the long way: 18.1 us, now 13.3.)
+// NT threads per row: 1024 when there are only a few rows, 256 otherwise (all rows of a batch of 320 are resident at once).
+constexpr int SR_U = 8;
 template <class OutT, int NT>
 __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restrict__ logits, int V, float noise, uint32_t seed,
                                                          OutT* __restrict__ out) {
-    __shared__ float bv[NT / 32];
+    __shared__ float bv[NT / 32], tops[2][NT / 32];
     __shared__ int bi[NT / 32];
     const size_t row = blockIdx.x;
     const __half* lr = logits + row * V;
-    float best = -INFINITY;
+    float best = -INFINITY, floor_ = -INFINITY;   // floor_: the row's result is at least this
     int idx = 0x7fffffff;
     auto take = [&](float v, int i) {
         if (noise > 0.f) v += noise * sample_noise(seed, (uint32_t)row, (uint32_t)i);
         if (v > best || (v == best && i < idx)) { best = v; idx = i; }
     };
-    const int nv = (V % 8 == 0 && ((uintptr_t)lr & 15) == 0) ? V / 8 : 0;
-#pragma unroll 4
-    for (int c = threadIdx.x; c < nv; c += NT) {
-        const uint4 q = reinterpret_cast<const uint4*>(lr)[c];
-        const __half2* h = reinterpret_cast<const __half2*>(&q);
+    // elements up to the first 16-byte boundary, chunks of eight, the rest
+    const int head = min(V, (int)((16 - ((uintptr_t)lr & 15)) & 15) / 2), nv = (V - head) / 8;
+    if ((int)threadIdx.x < head) take(__half2float(lr[threadIdx.x]), threadIdx.x);
+    const uint4* body = reinterpret_cast<const uint4*>(lr + head);
+    int buf = 0;
+    for (int c0 = 0; c0 < nv; c0 += NT * SR_U, buf ^= 1) {   // uniform in the block
+        uint4 q[SR_U];
+        __half m[SR_U];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(h[e]);
-            take(f.x, c * 8 + 2 * e);
-            take(f.y, c * 8 + 2 * e + 1);
+        for (int u = 0; u < SR_U; ++u) {
+            const int c = c0 + u * NT + threadIdx.x;
+            if (c < nv) q[u] = __ldcs(body + c);
+        }
+        __half top = __ushort_as_half((unsigned short)0xfc00u);   // -inf
+#pragma unroll
+        for (int u = 0; u < SR_U; ++u) {
+            m[u] = __ushort_as_half((unsigned short)0xfc00u);
+            if (c0 + u * NT + (int)threadIdx.x < nv) {
+                const __half2* h = reinterpret_cast<const __half2*>(&q[u]);
+                const __half2 t = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+                m[u] = __hmax(__low2half(t), __high2half(t));
+            }
+            top = __hmax(top, m[u]);
+        }
+        const float wtop = warp_max(fmaxf(__half2float(top), best));
+        if ((threadIdx.x & 31) == 0) tops[buf][threadIdx.x >> 5] = wtop;
+        __syncthreads();   // the two buffers alternate: one barrier per batch
+#pragma unroll
+        for (int i = 0; i < NT / 32; ++i) floor_ = fmaxf(floor_, tops[buf][i]);
+#pragma unroll
+        for (int u = 0; u < SR_U; ++u) {
+            const int c = c0 + u * NT + threadIdx.x;
+            if (c < nv && !(__half2float(m[u]) + noise < floor_)) {
+                const __half2* h = reinterpret_cast<const __half2*>(&q[u]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = __half22float2(h[e]);
+                    take(f.x, head + c * 8 + 2 * e);
+                    take(f.y, head + c * 8 + 2 * e + 1);
+                }
+            }
         }
     }
-    for (int i = nv * 8 + threadIdx.x; i < V; i += NT) take(__half2float(lr[i]), i);
+    for (int i = head + nv * 8 + threadIdx.x; i < V; i += NT) take(__half2float(lr[i]), i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -244,11 +412,13 @@ int ln_rows(const __half* x, const __half* w, const __half* b, int rows, int D, 
     AB_CUDA(cudaGetLastError());
     return OK;
 }
-bool ln_mix_rows_ok(const MixParams& p) { return p.T == 1 && p.D % 8 == 0 && p.D <= 8 * RT * LM_MAXV; }
+bool ln_mix_rows_ok(const MixParams& p) { return p.D % 8 == 0 && p.D <= 8 * RT * LM_MAXV; }
 int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixParams& p, cudaStream_t s, bool pdl) {
     AB_CHECK_ARG(x && w && b && p.x_prev && p.n_mix >= 1 && p.n_mix <= 6 && p.B > 0 && ln_mix_rows_ok(p), "ln_mix_rows: bad argument");
+    // rows per block of a sequence: as few as fill the GPU (each block normalises one row more than it owns)
+    const int rows = p.B * p.T, R = rows >= 2048 ? 4 : (rows >= 512 ? 2 : 1);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.B);
+    cfg.gridDim = dim3(p.T == 1 ? p.B : p.B * ((p.T + R - 1) / R));
     cfg.blockDim = dim3(RT);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -256,7 +426,9 @@ int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixPara
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    AB_CUDA(cudaLaunchKernelEx(&cfg, ln_mix_rows_kernel, x, w, b, p, pdl ? 1 : 0));
+    if (p.T == 1) AB_CUDA(cudaLaunchKernelEx(&cfg, ln_mix_rows_kernel, x, w, b, p, pdl ? 1 : 0));
+    else if (p.D <= 8 * RT * 2) AB_CUDA(cudaLaunchKernelEx(&cfg, ln_mix_seq_kernel<2>, x, w, b, p, R, pdl ? 1 : 0));
+    else AB_CUDA(cudaLaunchKernelEx(&cfg, ln_mix_seq_kernel<LM_MAXV>, x, w, b, p, R, pdl ? 1 : 0));
     return OK;
 }
 int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t seed, void* out, bool out_i64, cudaStream_t s) {
@@ -265,8 +437,8 @@ int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t see
         if (out_i64) sample_rows_kernel<long long, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (long long*)out);
         else sample_rows_kernel<int, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (int*)out);
     } else {
-        if (out_i64) sample_rows_kernel<long long, RT><<<rows, RT, 0, s>>>(logits, V, noise, seed, (long long*)out);
-        else sample_rows_kernel<int, RT><<<rows, RT, 0, s>>>(logits, V, noise, seed, (int*)out);
+        if (out_i64) sample_rows_kernel<long long, 256><<<rows, 256, 0, s>>>(logits, V, noise, seed, (long long*)out);
+        else sample_rows_kernel<int, 256><<<rows, 256, 0, s>>>(logits, V, noise, seed, (int*)out);
     }
     AB_CUDA(cudaGetLastError());
     return OK;

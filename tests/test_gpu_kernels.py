@@ -316,3 +316,69 @@ def test_device_sampler_matches_argsort():
     ret = sampler_simple_batch(logits, noise=0.0, out=pinned)
     torch.cuda.current_stream().synchronize()
     assert ret.data_ptr() == pinned.data_ptr() and pinned.flatten().tolist() == logits.float().argmax(-1).tolist()
+
+
+def _noisy_argmax(logits, noise, seed):
+    """The sampler's definition in numpy: first index of the largest logit + noise * hash(seed, row, column), in fp32."""
+    x = logits.cpu().float().numpy()
+    rows, V = x.shape
+    u32 = np.uint32
+    with np.errstate(over="ignore"):
+        h = u32(seed) ^ (np.arange(rows, dtype=u32)[:, None] * u32(0x9E3779B9)) ^ (np.arange(V, dtype=u32)[None] * u32(0x85EBCA6B))
+        h ^= h >> u32(16); h *= u32(0x7FEB352D); h ^= h >> u32(15); h *= u32(0x846CA68B); h ^= h >> u32(16)
+    u = (h >> u32(8)).astype(np.float32) * np.float32(1.0 / 16777216.0)
+    v = x + np.float32(noise) * u if noise > 0 else x
+    v = np.where(np.isnan(v), -np.inf, v)
+    best = v.max(axis=1, keepdims=True)
+    ok = (v == best) & ~np.isnan(x)
+    return ok.argmax(axis=1)
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 40])
+@pytest.mark.parametrize("V", [1, 7, 8, 37, 1000, 4096, 8191, 32776, 50277])
+@pytest.mark.parametrize("kind", ["normal", "ties", "infinite", "flat"])
+def test_device_sampler_exact(rows, V, kind):
+    """Rows on any 2-byte boundary, sizes around the 16-byte chunks and the batches, ties, infinities, NaNs: the same id
+    as the definition, for every noise."""
+    from albatross_b200 import sampler_simple_batch
+    g = torch.Generator().manual_seed(rows * V)
+    x = torch.randn(rows, V, generator=g) * 3
+    if kind == "ties":
+        x = x.round()
+    if kind == "infinite" and V > 1:
+        x[:, ::3] = -float("inf")
+        x[:, V // 2] = float("nan")
+        x[0] = -float("inf")
+        if rows > 1:
+            x[1, V - 1] = float("inf")
+    if kind == "flat":
+        x = torch.full((rows, V), -1.5)
+    x = x.half()
+    for noise in (0.0, 0.01, 1.0, 50.0):
+        got = sampler_simple_batch(x.cuda(), noise=noise, seed=9)
+        assert got.flatten().tolist() == _noisy_argmax(x, noise, 9).tolist(), (noise, kind)
+
+
+@pytest.mark.parametrize("D", [128, 256, 768, 4096, 5120])
+@pytest.mark.parametrize("B,T", [(1, 2), (3, 5), (2, 260), (5, 410)])
+def test_sequence_norm_and_lerps_through_a_model(B, T, D):
+    """The one-pass norm + token-shift kernel (1, 2 or 4 rows per block; row lengths up to its limit): the state it hands
+    over after T tokens is the normalised last row, and prompts give what the same tokens give one by one."""
+    from albatross_b200 import RWKV_x070, synth
+    import types
+    cfg = (1, D, 64, (16, 16, 16, 16))
+    args = types.SimpleNamespace(MODEL_NAME="", n_layer=1, n_embd=D, head_size=64, vocab_size=64)
+    model = RWKV_x070(args, quant="int8", state_dict=dict(synth.iter_checkpoint(cfg, seed=D, device="cuda")))
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, 64, (B, T), generator=g).tolist()
+    _, st = model.forward_batch(ids, None)
+    z = model.z
+    last = z["emb.weight"][torch.tensor([r[-1] for r in ids])].float()
+    want = torch.nn.functional.layer_norm(last, (D,), z["blocks.0.ln1.weight"].float(), z["blocks.0.ln1.bias"].float())
+    assert rel_err(st[0].float().cpu(), want.cpu()) < 1e-3          # one fp16 rounding
+    one = None
+    for t in range(min(T, 12)):                                     # a prefix, token by token through the T = 1 kernels
+        _, one = model.forward_batch([[r[t]] for r in ids], one)
+    _, pre = model.forward_batch([r[:min(T, 12)] for r in ids], None)
+    for a, b in zip(pre, one):
+        assert rel_err(a.float().cpu(), b.float().cpu()) < 1e-2     # fp16 activations along two kernel families
