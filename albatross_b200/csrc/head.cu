@@ -449,9 +449,9 @@ __global__ void __launch_bounds__(HB_THREADS, HB_BLOCKS) head_batch_kernel(const
 //     rows a lane and twice the warps shared memory is busier and the step is 12 % slower. Arithmetic on packed fp32 pairs;
 //   * "post" warps turn the read-outs of finished steps into the block output (group norm, bonus, gate).
 // Chunks travel pre -> scan -> post -> pre through a ring of SC_NBUF buffers on mbarriers. Two blocks share an SM, so that
-// one's exchanges are hidden by the other's arithmetic: 8 sequences of 128 steps, 64 heads: 104 us (one block of 512
-// threads per SM: 125 us; a 256-thread block per head without the pipeline, as it was: 611 us). One sequence of 1024 steps:
-// 252 us (1448 us).
+// one's exchanges are hidden by the other's arithmetic: 8 sequences of 128 steps, 64 heads: 93 us (a 256-thread block per
+// head without the pipeline, as it was: 631 us; before whole chunks were unrolled 104, with one block of 512 threads per
+// SM 125). One sequence of 1024 steps: 225 us (1450 us; before unrolling 252).
 // OP = true: the operator's inputs (w = pre-transform decay in w_raw, a and b in a_raw / vg_raw), y stored as it is.
 constexpr int SC_CH = 8, SC_NBUF = 4, SC_SCAN = 4, SC_PRE = 4, SC_POST = 2;
 constexpr int SC_THREADS = 32 * (SC_SCAN + SC_PRE + SC_POST);
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
             };
             auto exch2 = [&]() { y0 = (up2 ? y1 : y0) + __shfl_xor_sync(0xffffffffu, up2 ? y0 : y1, 2); };
             auto exch3 = [&]() { y0 += __shfl_xor_sync(0xffffffffu, y0, 4); };
-            for (int j = 0; j < ns; ++j) {
+            auto step = [&](int j) {
                 const ScanStep& s = ck.s[j];
                 float sa[4];
 #pragma unroll
@@ -551,6 +551,12 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                 for (int i = 0; i < 4; ++i) row_add(S[i], bb, sa[i]);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) y[i] = row_dot(S[i], r);
+            };
+            if (ns == SC_CH) {   // constant step numbers: addresses are offsets, and the compiler may overlap steps
+#pragma unroll
+                for (int j = 0; j < SC_CH; ++j) step(j);
+            } else {
+                for (int j = 0; j < ns; ++j) step(j);
             }
             exch1();
             exch2();
@@ -776,7 +782,7 @@ int wkv7_launch(int B, int T, int C, int H, float* state, const __half* r, const
     AB_CHECK_ARG(((uintptr_t)state & 15) == 0, "wkv7: state must be 16-byte aligned");
     // A single step is a pass over the state, which one small block per head streams best (64 heads, 32 sequences: 18.8 us);
     // from two steps on the pipelined kernel is ahead (T = 2: 24.3 against 26.8 us, T = 8: 37 against 77, one sequence of
-    // 1024: 255 against 1100). It reads the vectors two channels at a time: odd 2-byte boundaries take the plain kernel.
+    // 1024: 225 against 1100). It reads the vectors two channels at a time: odd 2-byte boundaries take the plain kernel.
     if (T > 1 && (((uintptr_t)r | (uintptr_t)w | (uintptr_t)k | (uintptr_t)v | (uintptr_t)a | (uintptr_t)b | (uintptr_t)y) & 3) == 0) {
         HeadParams p = {};
         p.B = B; p.T = T; p.D = C; p.H = H; p.layer0 = 1; p.state = state;
