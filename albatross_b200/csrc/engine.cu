@@ -88,6 +88,7 @@ struct Workspace {
     __half *x, *xn, *xn2, *r, *k, *v, *vfirst, *att, *kf, *hw, *ha, *hv, *hg;
     __half *mix[6], *w_raw, *a_raw, *vg_raw, *g, *xlast;
     void* gemm_scratch;
+    size_t gemm_scratch_bytes;
     size_t total;
 };
 
@@ -119,7 +120,8 @@ Workspace carve(const ab_model* m, int B, int T, unsigned char* base) {
     w.xlast = batched ? take((size_t)B * D) : nullptr;
     w.gemm_scratch = base + off;
     if (batched) {
-        size_t need = m->d.head.w ? gemm_scratch_bytes(m->d.head, (int)M) : 256;
+        // the head works on all M rows or, behind a prompt, on the B last ones (fewer rows may need more: see gemm.cuh)
+        size_t need = m->d.head.w ? std::max(gemm_scratch_bytes(m->d.head, (int)M), gemm_scratch_bytes(m->d.head, B)) : 256;
         for (const ab_layer& l : m->layers) {   // the products launched alone may be split along K
             need = std::max(need, gemm_scratch_bytes(l.output, (int)M));
             need = std::max(need, gemm_scratch_bytes(l.ffn_key, (int)M));
@@ -134,6 +136,7 @@ Workspace carve(const ab_model* m, int B, int T, unsigned char* base) {
         }
         off += al(need);
     }
+    w.gemm_scratch_bytes = off - (size_t)((unsigned char*)w.gemm_scratch - base);
     w.total = off;
     return w;
 }
@@ -461,15 +464,16 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
             AB_TRY(mix_rows(mp, st));
         }
         void* sc = ws.gemm_scratch;
+        const size_t sc_bytes = ws.gemm_scratch_bytes;
         {   // r, k, v and the adapter down-projections: one grouped launch
             GemmOp ops[8];
             const int n = time_mix_down_ops(L, gi, ws, ops);
-            AB_TRY(gemm_group_launch(ops, n, M, sc, st, m->use_pdl));
+            AB_TRY(gemm_group_launch(ops, n, M, sc, sc_bytes, st, m->use_pdl));
         }
         {   // adapter up-projections
             GemmOp ops[8];
             const int n = time_mix_up_ops(L, gi, ws, ops);
-            AB_TRY(gemm_group_launch(ops, n, M, sc, st, m->use_pdl));
+            AB_TRY(gemm_group_launch(ops, n, M, sc, sc_bytes, st, m->use_pdl));
         }
         HeadParams h = {};
         h.B = B; h.T = T; h.D = D; h.H = H; h.layer0 = (gi == 0);
@@ -480,7 +484,7 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         h.lnx_w = (const __half*)L.lnx_w; h.lnx_b = (const __half*)L.lnx_b;
         h.out = ws.att; h.use_pdl = m->use_pdl;
         AB_TRY(head_launch(h, st));
-        AB_TRY(gemm_launch(L.output, M, ws.att, ws.x, EPI_RESID, ws.x, sc, st, m->use_pdl));
+        AB_TRY(gemm_launch(L.output, M, ws.att, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl));
 
         MixParams fp = {};
         fp.xn = ws.xn; fp.x_prev = (__half*)state[3 * i + 2]; fp.B = B; fp.T = T; fp.D = D; fp.n_mix = 1;
@@ -491,8 +495,8 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
             AB_TRY(ln_rows(ws.x, (const __half*)L.ln2_w, (const __half*)L.ln2_b, M, D, 1, 0, ws.xn, st));
             AB_TRY(mix_rows(fp, st));
         }
-        AB_TRY(gemm_launch(L.ffn_key, M, ws.mix[0], ws.kf, EPI_RELU2, nullptr, sc, st, m->use_pdl));
-        AB_TRY(gemm_launch(L.ffn_value, M, ws.kf, ws.x, EPI_RESID, ws.x, sc, st, m->use_pdl));
+        AB_TRY(gemm_launch(L.ffn_key, M, ws.mix[0], ws.kf, EPI_RELU2, nullptr, sc, sc_bytes, st, m->use_pdl));
+        AB_TRY(gemm_launch(L.ffn_value, M, ws.kf, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl));
     }
     if (io && io->x_out) {
         AB_CUDA(cudaMemcpyAsync(io->x_out, ws.x, (size_t)M * D * 2, cudaMemcpyDeviceToDevice, st));
@@ -500,10 +504,10 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
     }
     if (full_output || T == 1) {
         AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, M, D, 1, 0, ws.xn, st));
-        return gemm_launch(m->d.head, M, ws.xn, logits, EPI_NONE, nullptr, ws.gemm_scratch, st, m->use_pdl);
+        return gemm_launch(m->d.head, M, ws.xn, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl);
     }
     AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, B, D, T, T - 1, ws.xlast, st));
-    return gemm_launch(m->d.head, B, ws.xlast, logits, EPI_NONE, nullptr, ws.gemm_scratch, st, m->use_pdl);
+    return gemm_launch(m->d.head, B, ws.xlast, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl);
 }
 
 }  // namespace
@@ -555,7 +559,8 @@ int ab_gemm(const ab_mat* m, int rows, const void* x, void* y, int epi, const vo
     AB_CHECK_ARG(rows > 0, "ab_gemm: rows must be positive");
     AB_TRY(check_mat(*m, "ab_gemm"));
     AB_CHECK_ARG(epi >= EPI_NONE && epi <= EPI_RESID && (epi != EPI_RESID || resid), "ab_gemm: bad epilogue");
-    return gemm_launch(*m, rows, (const __half*)x, (__half*)y, epi, (const __half*)resid, scratch, (cudaStream_t)stream);
+    // `scratch` has no size of its own here: the caller guarantees ab_gemm_scratch_bytes(m, rows)
+    return gemm_launch(*m, rows, (const __half*)x, (__half*)y, epi, (const __half*)resid, scratch, SIZE_MAX, (cudaStream_t)stream);
 }
 
 int ab_sample_rows(const void* logits, int rows, int vocab, float noise, uint32_t seed, int32_t* out, void* stream) {

@@ -909,7 +909,7 @@ size_t gemm_scratch_bytes(const ab_mat& m, int rows) {
     return gemm_group_scratch_bytes(&op, 1, rows);
 }
 
-int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStream_t stream, bool pdl) {
+int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t scratch_bytes, cudaStream_t stream, bool pdl) {
     AB_CHECK_ARG(ops && n >= 1 && n <= G_MAX_OPS && rows > 0, "gemm: bad group (n=%d rows=%d)", n, rows);
     for (int i = 0; i < n; ++i) {   // shapes first: the grid arithmetic below divides by tile counts
         const int s = check_mat(ops[i].w, "gemm");
@@ -918,9 +918,9 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
     const int n_sm = current_sm_count();
     GroupShape gs = group_shape(ops, n, rows, n_sm);
     AB_CHECK_ARG(gs.n_split_tiles <= G_COUNTERS, "gemm: too many split-K tiles");
-    if (gs.n_split_tiles > 0 && gs.grid_x * gs.n_tiles_y > n_sm) {
-        // the blocks of a split tile wait for one another, so all of them must be resident (one block per SM); a
-        // split grid that would not be is launched without the split instead
+    if (gs.n_split_tiles > 0 && (gs.grid_x * gs.n_tiles_y > n_sm || (size_t)G_COUNTERS * 4 + (size_t)gs.part_floats * 4 > scratch_bytes)) {
+        // the blocks of a split tile wait for one another, so all of them must be resident (one block per SM), and their
+        // partial sums must fit the scratch area; a split grid for which that does not hold is launched without the split
         GemmOp unsplit[G_MAX_OPS];
         for (int i = 0; i < n; ++i) unsplit[i] = ops[i];
         gs = group_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
@@ -1044,10 +1044,10 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStr
 }
 
 int gemm_launch(const ab_mat& m, int rows, const __half* x, __half* y, int epi, const __half* resid, void* scratch,
-                cudaStream_t stream, bool pdl) {
+                size_t scratch_bytes, cudaStream_t stream, bool pdl) {
     GemmOp op = {};
     op.w = m; op.x = x; op.y = y; op.epi = epi; op.resid = resid;
-    return gemm_group_launch(&op, 1, rows, scratch, stream, pdl);
+    return gemm_group_launch(&op, 1, rows, scratch, scratch_bytes, stream, pdl);
 }
 
 int dequant_launch(const ab_mat& m, float* out, cudaStream_t stream) {
@@ -1131,7 +1131,8 @@ extern "C" int ab_gemm_static(const ab_mat* m, int rows, const void* x, void* y,
     void* scratch = nullptr;
     st = static_scratch(&scratch, (cudaStream_t)stream);
     if (st != OK) return st;
-    return gemm_launch(*m, rows, (const __half*)x, (__half*)y, epi, (const __half*)resid, scratch, (cudaStream_t)stream);
+    return gemm_launch(*m, rows, (const __half*)x, (__half*)y, epi, (const __half*)resid, scratch, (size_t)AB_GEMM_STATIC_SCRATCH_BYTES,
+                       (cudaStream_t)stream);
 }
 
 extern "C" int ab_gemm_static_reset(void* stream) { return ab::static_scratch_reset((cudaStream_t)stream); }

@@ -14,15 +14,17 @@ struct GemmOp {
     int epi;
 };
 // Scratch: split-K arrival counters and fp32 partial tiles. It must be zero when first used; the kernels
-// leave the counters at zero again.
+// leave the counters at zero again. What a launch needs is not monotonic in `rows` (few rows are split along K where many
+// fill the GPU), so a caller with several launches takes the largest; a launch whose partial sums do not fit into
+// `scratch_bytes` runs without the split.
 size_t gemm_group_scratch_bytes(const GemmOp* ops, int n, int rows);
 // pdl: launch with programmatic stream serialisation (the kernel waits for the preceding grid itself, after it has
 // started its weight stream).
-int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, cudaStream_t stream, bool pdl = false);
+int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t scratch_bytes, cudaStream_t stream, bool pdl = false);
 size_t gemm_scratch_bytes(const ab_mat& m, int rows);
 int static_scratch_reset(cudaStream_t stream);   // built-in scratch of ab_gemm_static: counters back to zero
 int gemm_launch(const ab_mat& m, int rows, const __half* x, __half* y, int epi, const __half* resid, void* scratch,
-                cudaStream_t stream, bool pdl = false);
+                size_t scratch_bytes, cudaStream_t stream, bool pdl = false);
 int dequant_launch(const ab_mat& m, float* out, cudaStream_t stream);
 int check_mat(const ab_mat& m, const char* what);
 

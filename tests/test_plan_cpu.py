@@ -48,6 +48,58 @@ def test_random_segment_lists_are_covered_exactly_once(segs, n_blocks):
     _check(fmt, rows, k, n_blocks)
 
 
+def _al(v):
+    return (v + 255) & ~255
+
+
+def _model(D, V, fmt, head=True, L=2):
+    """A model handle on made-up (never followed) addresses: sizes only."""
+    layers = (_lib.Layer * L)()
+    ptr = 1 << 20
+    mat = lambda f, n, k: _lib.Mat(f, n, k, 0, ptr, None if f == F16 else ptr, None, 1.0, 0.0)
+    for ly in layers:
+        for name in _lib._LAYER_PTRS + _lib._LAYER_UPS:
+            setattr(ly, name, ptr)
+        for name in ("receptance", "key", "value", "output"):
+            setattr(ly, name, mat(fmt, D, D))
+        ly.ffn_key, ly.ffn_value = mat(fmt, 4 * D, D), mat(fmt, D, 4 * D)
+        for n in "wavg":
+            setattr(ly, n + "1t", mat(F16, 64, D))
+            setattr(ly, n + "2t", mat(F16, D, 64))
+    d = _lib.ModelDesc()
+    d.n_layer, d.n_embd, d.vocab, d.emb, d.layers = L, D, V, ptr, C.cast(layers, C.POINTER(_lib.Layer))
+    if head:
+        d.lnout_w = d.lnout_b = ptr
+        d.head = mat(fmt, V, D)
+    h = C.c_void_p()
+    _lib.check(_lib.lib.ab_model_create(C.byref(d), C.byref(h)))
+    return h, d.head
+
+
+@pytest.mark.parametrize("fmt", [I8, FP4, F16])
+@pytest.mark.parametrize("D,V", [(1024, 1024), (2048, 1024), (2560, 2048), (4096, 512), (4096, 4096), (4096, 65536)])
+def test_workspace_holds_the_partial_sums_of_a_prompts_last_product(fmt, D, V):
+    """After a prompt of T tokens the vocabulary head sees only the B last rows, and few rows are split along K where B * T
+    rows were not: the scratch part of the workspace has to hold either. What the head adds to a workspace is compared with
+    the one of the same blocks without a head, whose scratch part is at least the arrival counters' 16 KB + 256."""
+    h, head = _model(D, V, fmt)
+    bare, _ = _model(D, V, fmt, head=False)
+    ws = _lib.lib.ab_workspace_bytes
+    counters = 4096 * 4 + 256
+    for B in (1, 2, 3, 5, 8, 40):
+        for T in (2, 7, 37, 128, 513, 700, 1025, 2305, 3000):
+            need = _lib.lib.ab_gemm_scratch_bytes(C.byref(head), B)
+            rest = ws(bare, B, T) - _al(counters)       # everything else, if the blocks' own products are not split
+            if B * T >= 2305:                           # ... which holds for so many rows of these widths
+                assert ws(h, B, T) >= rest + need, (B, T)
+            assert ws(h, B, T) >= need and ws(h, B, T) >= ws(bare, B, T), (B, T)
+    # one sequence of 513 tokens, 4096 wide: no product of 513 rows is split, the head's single row is, eight ways
+    if (D, V, fmt) == (4096, 4096, I8):
+        assert ws(h, 1, 513) - ws(bare, 1, 513) >= _lib.lib.ab_gemm_scratch_bytes(C.byref(head), 1) - counters - 256 > 1 << 19
+    for x in (h, bare):
+        _lib.lib.ab_model_destroy(x)
+
+
 def test_state_list_forgets_its_checks_when_changed():
     """The list forward() hands back carries the model's validation and program key; any in-place change of the list
     drops them, so a changed list is checked from scratch (it is still a plain list to its user)."""
