@@ -225,6 +225,8 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // two adjacent fp16 channels; activations bypass L1 (written by another SM in an earlier kernel)
 __device__ __forceinline__ float2 ld2a(const __half* p) { return __half22float2(__ldcg(reinterpret_cast<const __half2*>(p))); }
 __device__ __forceinline__ float2 ld2p(const __half* p) { return __half22float2(__ldg(reinterpret_cast<const __half2*>(p))); }
+// the same for a caller's vector on any 2-byte boundary
+__device__ __forceinline__ float2 ld2u(const __half* p) { return make_float2(__half2float(__ldg(p)), __half2float(__ldg(p + 1))); }
 
 __global__ void __launch_bounds__(HB_THREADS, HB_BLOCKS) head_batch_kernel(const __grid_constant__ HeadParams p, int n_items) {
     extern __shared__ __align__(128) unsigned char dsm[];   // HB_STAGES x 16 KiB
@@ -572,18 +574,21 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         struct In { __half2 r, k, v, w, a, g, f; };   // OP: g = b; else g = v gate, f = v_first
         const int pw = warp - SC_SCAN, gc = h * 64 + 2 * lane;
         const bool gated = !OP && !p.layer0;
+        // v_first and the parameters are the caller's and may start on any 2-byte boundary; the rest is workspace (or was
+        // checked by the operator's launcher)
+        const bool vf_pairs = ((uintptr_t)p.v_first & 3) == 0;
         auto ldh = [](const __half* q) { return __ldcg(reinterpret_cast<const __half2*>(q)); };
         auto fetch = [&](int t, In& x) {
             if (t >= T) return;
             const size_t o = base + (size_t)t * p.D + 2 * lane;
             x.r = ldh(p.r + o); x.k = ldh(p.k + o); x.v = ldh(p.v + o); x.w = ldh(p.w_raw + o); x.a = ldh(p.a_raw + o);
             if (OP || gated) x.g = ldh(p.vg_raw + o);
-            if (gated) x.f = ldh(p.v_first + o);
+            if (gated) x.f = vf_pairs ? ldh(p.v_first + o) : __halves2half2(__ldcg(p.v_first + o), __ldcg(p.v_first + o + 1));
         };
         float2 w0, a0, v0, k_k, k_a, r_k;
         if (!OP) {
-            w0 = ld2p(p.w0 + gc); a0 = ld2p(p.a0 + gc); k_k = ld2p(p.k_k + gc); k_a = ld2p(p.k_a + gc); r_k = ld2p(p.r_k + gc);
-            v0 = gated ? ld2p(p.v0 + gc) : make_float2(0.f, 0.f);
+            w0 = ld2u(p.w0 + gc); a0 = ld2u(p.a0 + gc); k_k = ld2u(p.k_k + gc); k_a = ld2u(p.k_a + gc); r_k = ld2u(p.r_k + gc);
+            v0 = gated ? ld2u(p.v0 + gc) : make_float2(0.f, 0.f);
         }
         constexpr int PER = (SC_CH + SC_PRE - 1) / SC_PRE;   // steps of a chunk per pre warp
         In nxt[PER];
@@ -614,7 +619,9 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                 } else {
                     // reference/rwkv7.py:284-297, with the decay in fp32 as on its single-token path (:241)
                     if (p.layer0) {
-                        *reinterpret_cast<__half2*>(p.v_first + base + (size_t)t * p.D + 2 * lane) = cur[q].v;
+                        __half* d = p.v_first + base + (size_t)t * p.D + 2 * lane;
+                        if (vf_pairs) *reinterpret_cast<__half2*>(d) = cur[q].v;
+                        else { d[0] = __low2half(cur[q].v); d[1] = __high2half(cur[q].v); }
                     } else {
                         const float2 g = __half22float2(cur[q].g), f = __half22float2(cur[q].f);
                         v.x = rh(v.x + rh(rh(f.x - v.x) * rh(sigmoidf_(rh(v0.x + g.x)))));
@@ -642,7 +649,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         const int qw = warp - SC_SCAN - SC_PRE, gc = h * 64 + 2 * lane;
         constexpr int PER = (SC_CH + SC_POST - 1) / SC_POST;
         float2 lw, lb;
-        if (!OP) { lw = ld2p(p.lnx_w + gc); lb = ld2p(p.lnx_b + gc); }
+        if (!OP) { lw = ld2u(p.lnx_w + gc); lb = ld2u(p.lnx_b + gc); }
         for (int ch = 0; ch < n_chunks; ++ch) {
             const int buf = ch % SC_NBUF;
             const ScanChunk& ck = ring[buf];
@@ -715,7 +722,10 @@ int head_launch(const HeadParams& p, cudaStream_t stream) {
     const bool ups = p.w2 != nullptr;
     AB_CHECK_ARG(ups || (p.w_raw && p.a_raw && p.g && (p.layer0 || p.vg_raw)), "head: adapter outputs missing");
     AB_CHECK_ARG(!ups || (p.B == 1 && p.T == 1), "head: in-kernel adapter up-projection is the batch-1 path");
-    if (!ups && p.T == 1 && p.B * p.H >= 512) {
+    // head_batch_kernel reads the caller's vectors two channels at a time; on odd 2-byte boundaries the kernel below takes over
+    const bool pairs = (((uintptr_t)p.v_first | (uintptr_t)p.w0 | (uintptr_t)p.a0 | (uintptr_t)(p.layer0 ? nullptr : p.v0) | (uintptr_t)p.k_k |
+                         (uintptr_t)p.k_a | (uintptr_t)p.r_k | (uintptr_t)p.lnx_w | (uintptr_t)p.lnx_b) & 3) == 0;
+    if (!ups && p.T == 1 && p.B * p.H >= 512 && pairs) {
         // many sequences, one step each: persistent blocks with the state staged by bulk copies
         static PerDeviceOnce once;
         const DeviceProps* dp = nullptr;

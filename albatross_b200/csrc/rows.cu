@@ -392,9 +392,7 @@ __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restric
 // x_prev[b] = xn[b, T-1]
 __global__ void __launch_bounds__(RT) last_rows_kernel(const __half* __restrict__ xn, int T, int D, __half* __restrict__ x_prev) {
     const size_t b = blockIdx.x;
-    const uint4* src = reinterpret_cast<const uint4*>(xn + (b * T + T - 1) * D);
-    uint4* dst = reinterpret_cast<uint4*>(x_prev + b * D);
-    for (int i = threadIdx.x; i < D / 8; i += RT) dst[i] = src[i];
+    for (int i = threadIdx.x; i < D; i += RT) x_prev[b * D + i] = xn[(b * T + T - 1) * D + i];
 }
 
 }  // namespace
@@ -412,9 +410,13 @@ int ln_rows(const __half* x, const __half* w, const __half* b, int rows, int D, 
     AB_CUDA(cudaGetLastError());
     return OK;
 }
-bool ln_mix_rows_ok(const MixParams& p) { return p.D % 8 == 0 && p.D <= 8 * RT * LM_MAXV; }
+bool ln_mix_rows_ok(const __half* w, const __half* b, const MixParams& p) {
+    uintptr_t any = (uintptr_t)w | (uintptr_t)b | (uintptr_t)p.x_prev;
+    for (int j = 0; j < p.n_mix; ++j) any |= (uintptr_t)p.mix[j];
+    return p.D % 8 == 0 && p.D <= 8 * RT * LM_MAXV && (any & 15) == 0;
+}
 int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixParams& p, cudaStream_t s, bool pdl) {
-    AB_CHECK_ARG(x && w && b && p.x_prev && p.n_mix >= 1 && p.n_mix <= 6 && p.B > 0 && ln_mix_rows_ok(p), "ln_mix_rows: bad argument");
+    AB_CHECK_ARG(x && w && b && p.x_prev && p.n_mix >= 1 && p.n_mix <= 6 && p.B > 0 && ln_mix_rows_ok(w, b, p), "ln_mix_rows: bad argument");
     // rows per block of a sequence: as few as fill the GPU (each block normalises one row more than it owns)
     const int rows = p.B * p.T, R = rows >= 2048 ? 4 : (rows >= 512 ? 2 : 1);
     cudaLaunchConfig_t cfg = {};

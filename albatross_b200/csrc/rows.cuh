@@ -17,8 +17,9 @@ int ln_rows(const __half* x, const __half* w, const __half* b, int rows, int D, 
             cudaStream_t s);
 int mix_rows(const MixParams& p, cudaStream_t s);
 int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t seed, void* out, bool out_i64, cudaStream_t s);
-// Layer norm of x (weights w, b) fused with the lerps (p.xn is not used).
-bool ln_mix_rows_ok(const MixParams& p);
+// Layer norm of x (weights w, b) fused with the lerps (p.xn is not used). It works on 16 bytes at a time: for other row lengths
+// and for vectors or states of the caller's that are not 16-byte aligned there are ln_rows and mix_rows, which take any.
+bool ln_mix_rows_ok(const __half* w, const __half* b, const MixParams& p);
 int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixParams& p, cudaStream_t s, bool pdl = false);
 
 }  // namespace ab

@@ -164,7 +164,9 @@ int ab_forward(ab_model* m, int B, int T, const int32_t* tokens, void* const* st
  * of its first block in the whole network (block 0 defines v_first, reference/rwkv7.py:239, :292).
  * First stage: tokens != NULL (needs desc.emb), later stages: x_in fp16 [B*T, D]. v_first fp16 [B*T, D] is written
  * by the first stage and read by the others. Last stage: logits fp16 [B,V] (needs desc.head / lnout), other
- * stages: x_out fp16 [B*T, D]. State and workspace as in ab_forward (sized by ab_workspace_bytes). */
+ * stages: x_out fp16 [B*T, D]. State and workspace as in ab_forward (sized by ab_workspace_bytes). v_first may start on
+ * any 2-byte boundary, and so may a block's vectors and the fp16 state entries unless B = T = 1; the fp32 state entries
+ * must be 16-byte aligned. */
 int ab_forward_stage(ab_model* m, int B, int T, const int32_t* tokens, const void* x_in, void* v_first,
                      void* const* state, void* workspace, void* x_out, void* logits, void* stream);
 /* Batch-1 decode as ONE persistent kernel per token (same results as ab_forward with B = T = 1).

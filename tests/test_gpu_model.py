@@ -116,6 +116,83 @@ def test_pipeline_stages_chain_to_the_full_model():
     assert torch.equal(st[0][1], st_full[1]) and torch.equal(st[1][1], st_full[4]) and len(st[0]) == 3
 
 
+def _odd(t):
+    """The same values one fp16 element behind a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)
+    buf[1:1 + t.numel()] = t.reshape(-1)
+    return buf[1:1 + t.numel()].view(t.shape)
+
+
+def _run_stage(model, B, T, state, vf, tokens=None, x_in=None, x_out=None):
+    """ab_forward_stage on sequences (`forward_stage` of the class is for T = 1)."""
+    import ctypes as C
+    from albatross_b200 import _lib
+    ws = model._workspace(B, T)
+    logits = torch.empty(B, model.vocab, dtype=torch.float16, device="cuda") if x_out is None else None
+    addr = lambda t: None if t is None else t.data_ptr()
+    ptrs = (C.c_void_p * len(state))(*[t.data_ptr() for t in state])
+    _lib.check(_lib.lib.ab_forward_stage(model._handle, B, T, addr(tokens), addr(x_in), vf.data_ptr(), ptrs, (ws.data_ptr() + 255) & ~255,
+                                         addr(x_out), addr(logits), torch.cuda.current_stream().cuda_stream), "ab_forward_stage")
+    return logits
+
+
+@pytest.mark.parametrize("B,T", [(3, 1), (260, 1), (1, 2), (3, 9), (2, 40)])
+def test_stages_take_v_first_on_any_boundary(B, T):
+    """One step of few and of many sequences, and sequences: a v_first that starts on an odd 2-byte boundary gives what an
+    aligned one gives. The same kernels and the same arithmetic: the same bits, but where many single steps take the kernel for
+    few, which sums in another order: there the tolerance between kernel families."""
+    from albatross_b200 import RWKV_x070, synth
+    args = synth.make_args("tiny")
+    sd = dict(synth.iter_checkpoint("tiny", seed=0))
+    stages = [RWKV_x070(args, quant="int8", state_dict=sd, layer_range=r) for r in ((0, 1), (1, 2))]
+    toks = torch.tensor(seeded_tokens(args.vocab_size, B * T, seed=3), dtype=torch.int32, device="cuda")
+    outs = []
+    for place in (lambda t: t, _odd):
+        st = [m.new_state(B) for m in stages]
+        vf = place(torch.zeros(B * T, args.n_embd, dtype=torch.float16, device="cuda"))
+        x = torch.empty(B * T, args.n_embd, dtype=torch.float16, device="cuda")
+        _run_stage(stages[0], B, T, st[0], vf, tokens=toks, x_out=x)
+        logits = _run_stage(stages[1], B, T, st[1], vf, x_in=x)
+        outs.append([vf, logits] + [t for s in st for t in s])
+    assert outs[1][0].data_ptr() % 4 == 2
+    from albatross_b200 import _lib
+    assert _lib.device_status() == 0
+    same = not (T == 1 and B * stages[0].n_head >= 512)
+    for a, b in zip(*outs):
+        assert torch.equal(a, b) if same else rel_err(a.float().cpu(), b.float().cpu()) <= LOGIT_REL_TOL
+
+
+@pytest.mark.parametrize("B,T", [(3, 1), (260, 1), (2, 37)])
+def test_vectors_and_states_on_any_boundary(B, T):
+    """Norm weights, lerp and per-channel vectors and token-shift states on odd 2-byte boundaries take the general kernels. The
+    row sums of the two norm kernels run in another order (fp32), which moves fp16 roundings."""
+    import ctypes as C
+    from albatross_b200 import _lib
+    model, args = model_for("tiny", "int8")
+    ids = [seeded_tokens(args.vocab_size, T, seed=s) for s in range(B)]
+    want, st = model.forward_batch(ids, model.new_state(B))
+    n, keep = args.n_embd, []
+    for i, ly in enumerate(model._layers):
+        for name in _lib._LAYER_PTRS:
+            if name == "v0" and i == 0:
+                continue
+            key = {"ln1_w": "ln1.weight", "ln1_b": "ln1.bias", "ln2_w": "ln2.weight", "ln2_b": "ln2.bias", "lnx_w": "att.ln_x.weight",
+                   "lnx_b": "att.ln_x.bias", "ffn_x_k": "ffn.x_k"}.get(name, "att." + name)
+            keep.append(_odd(model.z["blocks.%d.%s" % (i, key)].view(n)))
+            setattr(ly, name, keep[-1].data_ptr())
+    h = C.c_void_p()
+    _lib.check(_lib.lib.ab_model_create(C.byref(model._desc), C.byref(h)))
+    old, model._handle = model._handle, h
+    _lib.lib.ab_model_destroy(old)
+    model._graphs.clear()
+    odd = [t if j % 3 == 1 else _odd(t) for j, t in enumerate(model.new_state(B))]
+    got, st2 = model.forward_batch(ids, odd)
+    assert _lib.device_status() == 0
+    assert rel_err(got.float().cpu(), want.float().cpu()) < LOGIT_REL_TOL
+    for a, b in zip(st2, st):
+        assert rel_err(a.float().cpu(), b.float().cpu()) < LOGIT_REL_TOL
+
+
 @pytest.mark.parametrize("option", ["merge_ups", "fuse_heads", "pair_split", "l2_prefetch_kb", "smem_prefetch", "early_slice", "barrier_prefetch"])
 def test_persistent_kernel_options_do_not_change_results(option):
     """The scheduling options of the persistent kernel move work between phases; logits stay the same: bit for bit
