@@ -10,7 +10,9 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <mutex>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "../../include/albatross_b200.h"
@@ -50,9 +52,18 @@ static GemvSeg seg_of(const ab_mat& m, const void* mix, int epi, void* out, cons
 
 using namespace ab;
 
+// Tensor maps of a block's matrices, as the batched products take them.
+struct LayerMaps {
+    WeightMaps receptance, key, value, output, ffn_key, ffn_value, w1t, a1t, v1t, g1t, w2t, a2t, v2t, g2t;
+};
+
 struct ab_model {
     ab_model_desc d;
     std::vector<ab_layer> layers;
+    // encoded by the first batched forward pass (a model can be made and sized without a GPU); the weights never move
+    std::mutex maps_mu;
+    std::vector<LayerMaps> maps;
+    WeightMaps head_maps;
     int use_pdl = 1;
     int n_sm = 0;          // blocks of the persistent decode kernel
     int layer_offset = 0;  // pipeline stage: index of this model's first block in the whole network
@@ -92,8 +103,9 @@ struct Workspace {
     size_t total;
 };
 
-int time_mix_down_ops(const ab_layer& L, int layer, const Workspace& ws, GemmOp* ops);
-int time_mix_up_ops(const ab_layer& L, int layer, const Workspace& ws, GemmOp* ops);
+// (maps: null when only sizes are asked for)
+int time_mix_down_ops(const ab_layer& L, const LayerMaps* maps, int layer, const Workspace& ws, GemmOp* ops);
+int time_mix_up_ops(const ab_layer& L, const LayerMaps* maps, int layer, const Workspace& ws, GemmOp* ops);
 
 Workspace carve(const ab_model* m, int B, int T, unsigned char* base) {
     const size_t M = (size_t)B * T, D = m->d.n_embd, F = 4 * D;
@@ -129,9 +141,9 @@ Workspace carve(const ab_model* m, int B, int T, unsigned char* base) {
         }
         for (size_t i = 0; i < m->layers.size(); ++i) {   // the two grouped launches of every block
             GemmOp ops[8];
-            int n = time_mix_down_ops(m->layers[i], (int)i + m->layer_offset, w, ops);
+            int n = time_mix_down_ops(m->layers[i], nullptr, (int)i + m->layer_offset, w, ops);
             need = std::max(need, gemm_group_scratch_bytes(ops, n, (int)M));
-            n = time_mix_up_ops(m->layers[i], (int)i + m->layer_offset, w, ops);
+            n = time_mix_up_ops(m->layers[i], nullptr, (int)i + m->layer_offset, w, ops);
             need = std::max(need, gemm_group_scratch_bytes(ops, n, (int)M));
         }
         off += al(need);
@@ -416,34 +428,54 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
     return OK;
 }
 
-GemmOp gemm_op(const ab_mat& w, const __half* x, __half* y, int epi, const __half* resid = nullptr) {
+GemmOp gemm_op(const ab_mat& w, const __half* x, __half* y, int epi, const WeightMaps* maps) {
     GemmOp o = {};
-    o.w = w; o.x = x; o.y = y; o.epi = epi; o.resid = resid;
+    o.w = w; o.x = x; o.y = y; o.epi = epi; o.maps = maps;
     return o;
 }
-int time_mix_down_ops(const ab_layer& L, int layer, const Workspace& ws, GemmOp* ops) {
+int encode_maps(ab_model* m) {
+    std::lock_guard<std::mutex> lock(m->maps_mu);
+    if (!m->maps.empty()) return OK;
+    std::vector<LayerMaps> maps(m->layers.size());
+    for (size_t i = 0; i < maps.size(); ++i) {
+        const ab_layer& l = m->layers[i];
+        LayerMaps& o = maps[i];
+        const ab_mat* from[14] = {&l.receptance, &l.key, &l.value, &l.output, &l.ffn_key, &l.ffn_value, &l.w1t,
+                                  &l.a1t, &l.v1t, &l.g1t, &l.w2t, &l.a2t, &l.v2t, &l.g2t};
+        WeightMaps* to[14] = {&o.receptance, &o.key, &o.value, &o.output, &o.ffn_key, &o.ffn_value, &o.w1t,
+                              &o.a1t, &o.v1t, &o.g1t, &o.w2t, &o.a2t, &o.v2t, &o.g2t};
+        for (int j = 0; j < 14; ++j) AB_TRY(encode_weight_maps(*from[j], to[j]));
+    }
+    AB_TRY(encode_weight_maps(m->d.head, &m->head_maps));
+    m->maps = std::move(maps);
+    return OK;
+}
+int time_mix_down_ops(const ab_layer& L, const LayerMaps* maps, int layer, const Workspace& ws, GemmOp* ops) {
+    auto mp = [&](WeightMaps LayerMaps::*which) { return maps ? &(maps->*which) : nullptr; };
     int n = 0;
-    ops[n++] = gemm_op(L.receptance, ws.mix[0], ws.r, EPI_NONE);
-    ops[n++] = gemm_op(L.key, ws.mix[1], ws.k, EPI_NONE);
-    ops[n++] = gemm_op(L.value, ws.mix[2], ws.v, EPI_NONE);
-    ops[n++] = gemm_op(L.w1t, ws.mix[3], ws.hw, EPI_TANH);
-    ops[n++] = gemm_op(L.a1t, ws.mix[4], ws.ha, EPI_NONE);
-    ops[n++] = gemm_op(L.g1t, ws.mix[5], ws.hg, EPI_SIGMOID);
-    if (layer > 0) ops[n++] = gemm_op(L.v1t, ws.mix[2], ws.hv, EPI_NONE);
+    ops[n++] = gemm_op(L.receptance, ws.mix[0], ws.r, EPI_NONE, mp(&LayerMaps::receptance));
+    ops[n++] = gemm_op(L.key, ws.mix[1], ws.k, EPI_NONE, mp(&LayerMaps::key));
+    ops[n++] = gemm_op(L.value, ws.mix[2], ws.v, EPI_NONE, mp(&LayerMaps::value));
+    ops[n++] = gemm_op(L.w1t, ws.mix[3], ws.hw, EPI_TANH, mp(&LayerMaps::w1t));
+    ops[n++] = gemm_op(L.a1t, ws.mix[4], ws.ha, EPI_NONE, mp(&LayerMaps::a1t));
+    ops[n++] = gemm_op(L.g1t, ws.mix[5], ws.hg, EPI_SIGMOID, mp(&LayerMaps::g1t));
+    if (layer > 0) ops[n++] = gemm_op(L.v1t, ws.mix[2], ws.hv, EPI_NONE, mp(&LayerMaps::v1t));
     return n;
 }
-int time_mix_up_ops(const ab_layer& L, int layer, const Workspace& ws, GemmOp* ops) {
+int time_mix_up_ops(const ab_layer& L, const LayerMaps* maps, int layer, const Workspace& ws, GemmOp* ops) {
+    auto mp = [&](WeightMaps LayerMaps::*which) { return maps ? &(maps->*which) : nullptr; };
     int n = 0;
-    ops[n++] = gemm_op(L.w2t, ws.hw, ws.w_raw, EPI_NONE);
-    ops[n++] = gemm_op(L.a2t, ws.ha, ws.a_raw, EPI_NONE);
-    ops[n++] = gemm_op(L.g2t, ws.hg, ws.g, EPI_NONE);
-    if (layer > 0) ops[n++] = gemm_op(L.v2t, ws.hv, ws.vg_raw, EPI_NONE);
+    ops[n++] = gemm_op(L.w2t, ws.hw, ws.w_raw, EPI_NONE, mp(&LayerMaps::w2t));
+    ops[n++] = gemm_op(L.a2t, ws.ha, ws.a_raw, EPI_NONE, mp(&LayerMaps::a2t));
+    ops[n++] = gemm_op(L.g2t, ws.hg, ws.g, EPI_NONE, mp(&LayerMaps::g2t));
+    if (layer > 0) ops[n++] = gemm_op(L.v2t, ws.hv, ws.vg_raw, EPI_NONE, mp(&LayerMaps::v2t));
     return n;
 }
 
 int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* state, const Workspace& ws_in,
                  __half* logits, int full_output, cudaStream_t st, const StageIO* io = nullptr) {
     const int D = m->d.n_embd, H = D / HEAD, M = B * T;
+    AB_TRY(encode_maps(m));
     Workspace ws = ws_in;
     if (io && io->v_first) ws.vfirst = io->v_first;
     if (io && io->x_in) AB_CUDA(cudaMemcpyAsync(ws.x, io->x_in, (size_t)M * D * 2, cudaMemcpyDeviceToDevice, st));
@@ -453,6 +485,7 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         const int i = li;
         const int gi = g0 + li;
         const ab_layer& L = m->layers[i];
+        const LayerMaps& LM = m->maps[i];
         MixParams mp = {};
         mp.xn = ws.xn; mp.x_prev = (__half*)state[3 * i]; mp.B = B; mp.T = T; mp.D = D; mp.n_mix = 6;
         const void* mv[6] = {L.x_r, L.x_k, L.x_v, L.x_w, L.x_a, L.x_g};
@@ -467,12 +500,12 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         const size_t sc_bytes = ws.gemm_scratch_bytes;
         {   // r, k, v and the adapter down-projections: one grouped launch
             GemmOp ops[8];
-            const int n = time_mix_down_ops(L, gi, ws, ops);
+            const int n = time_mix_down_ops(L, &LM, gi, ws, ops);
             AB_TRY(gemm_group_launch(ops, n, M, sc, sc_bytes, st, m->use_pdl));
         }
         {   // adapter up-projections
             GemmOp ops[8];
-            const int n = time_mix_up_ops(L, gi, ws, ops);
+            const int n = time_mix_up_ops(L, &LM, gi, ws, ops);
             AB_TRY(gemm_group_launch(ops, n, M, sc, sc_bytes, st, m->use_pdl));
         }
         HeadParams h = {};
@@ -484,7 +517,7 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         h.lnx_w = (const __half*)L.lnx_w; h.lnx_b = (const __half*)L.lnx_b;
         h.out = ws.att; h.use_pdl = m->use_pdl;
         AB_TRY(head_launch(h, st));
-        AB_TRY(gemm_launch(L.output, M, ws.att, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl));
+        AB_TRY(gemm_launch(L.output, M, ws.att, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl, &LM.output));
 
         MixParams fp = {};
         fp.xn = ws.xn; fp.x_prev = (__half*)state[3 * i + 2]; fp.B = B; fp.T = T; fp.D = D; fp.n_mix = 1;
@@ -495,8 +528,8 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
             AB_TRY(ln_rows(ws.x, (const __half*)L.ln2_w, (const __half*)L.ln2_b, M, D, 1, 0, ws.xn, st));
             AB_TRY(mix_rows(fp, st));
         }
-        AB_TRY(gemm_launch(L.ffn_key, M, ws.mix[0], ws.kf, EPI_RELU2, nullptr, sc, sc_bytes, st, m->use_pdl));
-        AB_TRY(gemm_launch(L.ffn_value, M, ws.kf, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl));
+        AB_TRY(gemm_launch(L.ffn_key, M, ws.mix[0], ws.kf, EPI_RELU2, nullptr, sc, sc_bytes, st, m->use_pdl, &LM.ffn_key));
+        AB_TRY(gemm_launch(L.ffn_value, M, ws.kf, ws.x, EPI_RESID, ws.x, sc, sc_bytes, st, m->use_pdl, &LM.ffn_value));
     }
     if (io && io->x_out) {
         AB_CUDA(cudaMemcpyAsync(io->x_out, ws.x, (size_t)M * D * 2, cudaMemcpyDeviceToDevice, st));
@@ -504,10 +537,10 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
     }
     if (full_output || T == 1) {
         AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, M, D, 1, 0, ws.xn, st));
-        return gemm_launch(m->d.head, M, ws.xn, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl);
+        return gemm_launch(m->d.head, M, ws.xn, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl, &m->head_maps);
     }
     AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, B, D, T, T - 1, ws.xlast, st));
-    return gemm_launch(m->d.head, B, ws.xlast, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl);
+    return gemm_launch(m->d.head, B, ws.xlast, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl, &m->head_maps);
 }
 
 }  // namespace

@@ -63,7 +63,8 @@ constexpr int G_BK = 64;         // inputs per k-step (128 bytes of fp16 = one s
 constexpr int G_RAW_ROW = 128;            // bytes of each weight row per raw slot: 1 / 2 / 4 k-steps of fp16 / int8 / NVFP4
 constexpr int G_RAW_SLOTS = 12;           // at most this many raw slots
 constexpr int G_REGS_PROD = 136, G_REGS_REST = 96;   // (136 - 128) * 384 producer threads <= (128 - 96) * 128 others
-constexpr int G_MAX_OPS = 8;
+constexpr int G_MAX_OPS = 7;
+constexpr int G_MAX_MAPS = 24;            // tensor maps of a launch
 constexpr int G_COUNTERS = 4096;         // split-K arrival counters at the start of the scratch area
 
 // One matrix product of a grouped launch.
@@ -75,8 +76,10 @@ struct GemmProb {
     int ksplit;       // blocks that share one output tile along K
     int tile_base;    // first split-K tile id (counter / partial index)
     long long part_base;   // float offset of its split-K partial sums in the scratch area
-    int tma_out;      // output (and residual) tiles go through shared memory and the TMA unit
-    int scale_map;    // NVFP4: the block scales come by TMA with the weights (else each thread loads its own)
+    // which of the launch's tensor maps: activations X; weights as bytes, boxes of 128 rows x 128 bytes; NVFP4 block scales,
+    // boxes of 128 rows x 16 bytes (-1: each thread loads its own); outputs Y and residuals, boxes of 32 batch rows x 128
+    // features (-1: straight from and to global memory)
+    signed char x_map, w_map, s_map, y_map, r_map;
     int recv_slots;   // split K: own chunks whose slices fit the receive area at a time
 };
 struct GemmGroup {
@@ -94,13 +97,13 @@ struct GemmGroup {
     int raw_bytes;  // shared memory for the raw slots
     int recv_off;   // split K: byte offset of the area the partial sums are fetched to, in the block's shared memory
 };
+// A launch with more than 4 KB of parameters costs the host more, so the maps share one table; products that find it full do
+// without the optional ones. The host's part of an eager step of 12 blocks (61 launches of products): 283 us with five maps
+// for every product (6 KB) and the weights' encoded for each launch, 256 like this; a prompt of 37 tokens 345 and 320.
 struct GemmMaps {
-    CUtensorMap m[G_MAX_OPS];   // activations X
-    CUtensorMap y[G_MAX_OPS];   // outputs Y, boxes of 32 batch rows x 128 features
-    CUtensorMap r[G_MAX_OPS];   // residuals, same boxes
-    CUtensorMap w[G_MAX_OPS];   // weights as bytes, boxes of 128 rows x 128 bytes
-    CUtensorMap s[G_MAX_OPS];   // NVFP4 block scales, boxes of 128 rows x 16 bytes (k a multiple of 256)
+    CUtensorMap t[G_MAX_MAPS];
 };
+static_assert(2 * G_MAX_OPS <= G_MAX_MAPS && sizeof(GemmMaps) + sizeof(GemmGroup) <= 4096, "parameters of the product kernels");
 
 // ---------------------------------------------------------------------------------------------
 // PTX wrappers (tcgen05 / TMA)
@@ -379,7 +382,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
             constexpr int F = decltype(fmt_c)::value;
             constexpr int P = raw_ksteps(F), SB = raw_slot_bytes(F);
             // block scales without a tensor map (k not a multiple of 256): this thread's own words, one own k-step ahead
-            const bool own_sc = F == FMT_FP4 && !pb.scale_map;
+            const bool own_sc = F == FMT_FP4 && pb.s_map < 0;
             const unsigned char* srow = reinterpret_cast<const unsigned char*>(pb.w.scale) + (F == FMT_FP4 && row_ok ? (size_t)row * (pb.w.k / 16) : 0);
             auto scale_word = [&](int ks) -> uint32_t {
                 if (ks >= n_ksteps) return 0u;
@@ -488,7 +491,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
         // operand stages are idle by now) and leaves through the TMA unit in full lines; the unit clips rows and
         // features beyond the matrix. A residual tile comes in the same way and is updated in place.
         __half* stg = reinterpret_cast<__half*>(base);
-        const bool staged = pb.tma_out != 0;
+        const bool staged = pb.y_map >= 0;
         auto stage32 = [&](int ci, const float* v) {
             __half* t = stg + (size_t)ci * 32 * G_BM + r_local;
             auto body = [&](auto E) {
@@ -522,7 +525,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
             fence_proxy_async();
             group_sync(grp);
             if (r_local == 0) {
-                tma_store_2d(&maps.y[pi], m0, n0 + ci * 32, stg + (size_t)ci * 32 * G_BM);
+                tma_store_2d(&maps.t[pb.y_map], m0, n0 + ci * 32, stg + (size_t)ci * 32 * G_BM);
                 bulk_commit();
             }
         };
@@ -536,7 +539,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
                 for (int ci = 0; ci < n_chunks; ++ci) n_mine += my_chunk(ci) ? 1 : 0;
                 mbar_expect_tx(&resid_bar, (uint32_t)(n_mine * 32 * G_BM * 2));
                 for (int ci = 0; ci < n_chunks; ++ci)
-                    if (my_chunk(ci)) tma_load_2d(stg + (size_t)ci * 32 * G_BM, &maps.r[pi], m0, n0 + ci * 32, &resid_bar);
+                    if (my_chunk(ci)) tma_load_2d(stg + (size_t)ci * 32 * G_BM, &maps.t[pb.r_map], m0, n0 + ci * 32, &resid_bar);
             }
             if (wait) wait_ok(&resid_bar, 0);
         };
@@ -642,7 +645,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
         tc_fence_before();
     } else if (warp == 4 * G_NG) {
         // ===== activation tiles by TMA =====
-        const CUtensorMap* map = &maps.m[pi];
+        const CUtensorMap* map = &maps.t[pb.x_map];
         const bool two_boxes = g.tma_rows < g.n_tile;
         const int x_begin = raw_begin * per * G_BK, x_end = raw_end * per * G_BK;
         int x = raw_of(0) * per * G_BK;   // the k-steps in rotated order, walked without divisions
@@ -669,7 +672,8 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
         }
     } else if (warp == 4 * G_NG + 2) {
         // ===== raw weights by TMA: never written by anybody, so they start before the preceding grid is done =====
-        const uint32_t bytes = (uint32_t)(G_BM * G_RAW_ROW + (pb.scale_map ? G_BM * 16 : 0));
+        const uint32_t bytes = (uint32_t)(G_BM * G_RAW_ROW + (pb.s_map >= 0 ? G_BM * 16 : 0));
+        const CUtensorMap *w_map = &maps.t[pb.w_map], *s_map = pb.s_map >= 0 ? &maps.t[pb.s_map] : nullptr;
         int slot = 0;
         uint32_t parity = 1;   // the first round finds every slot free
         for (int i = 0; i < n_raw; ++i) {
@@ -678,8 +682,8 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
             unsigned char* dst = smRaw + slot * slot_bytes;
             const int ra = raw_of(i);
             mbar_expect_tx_one(&raw_full[slot], bytes);
-            tma_load_2d_one(dst, &maps.w[pi], ra * G_RAW_ROW, m0, &raw_full[slot]);
-            if (pb.scale_map) tma_load_2d_one(dst + G_BM * G_RAW_ROW, &maps.s[pi], ra * 16, m0, &raw_full[slot]);
+            tma_load_2d_one(dst, w_map, ra * G_RAW_ROW, m0, &raw_full[slot]);
+            if (s_map) tma_load_2d_one(dst + G_BM * G_RAW_ROW, s_map, ra * 16, m0, &raw_full[slot]);
             if (++slot == n_slots) { slot = 0; parity ^= 1u; }
         }
     } else if (warp == 4 * G_NG + 1) {
@@ -787,6 +791,33 @@ int check_mat(const ab_mat& m, const char* what) {
     AB_CHECK_ARG(m.w && m.n_out > 0 && m.k > 0, "%s: empty matrix", what);
     AB_CHECK_ARG(m.fmt == FMT_F16 || m.scale, "%s: scales missing", what);
     AB_CHECK_ARG(m.fmt != FMT_FP4 || m.k % 32 == 0, "%s: NVFP4 needs k %% 32 == 0", what);
+    return OK;
+}
+
+int encode_weight_maps(const ab_mat& m, WeightMaps* out) {
+    out->valid = out->scale_map = 0;
+    if (!m.w || m.n_out <= 0 || m.k <= 0 || m.k % 16 != 0 || ((uintptr_t)m.w & 15) != 0 || (m.fmt == FMT_FP4 && (m.k % 64 != 0 || !m.scale)))
+        return OK;
+    EncodeTiledFn encode;
+    const int st = get_encode_fn(&encode);
+    if (st != OK) return st;
+    // rows as they are stored; the block scales need a row pitch of a multiple of 16 bytes
+    out->scale_map = m.fmt == FMT_FP4 && m.k % 256 == 0 && ((uintptr_t)m.scale & 15) == 0 ? 1 : 0;
+    const cuuint32_t estr[2] = {1, 1};
+    for (int which = 0; which < 1 + out->scale_map; ++which) {
+        const cuuint64_t pitch = which ? m.k / 16 : (m.fmt == FMT_F16 ? 2ull * m.k : m.fmt == FMT_I8 ? (cuuint64_t)m.k : m.k / 2);
+        const cuuint64_t wdim[2] = {pitch, (cuuint64_t)m.n_out};
+        const cuuint32_t wbox[2] = {which ? 16u : (cuuint32_t)G_RAW_ROW, (cuuint32_t)G_BM};
+        const CUresult cw = encode(which ? &out->s : &out->w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                                   const_cast<void*>(which ? m.scale : m.w), wdim, &pitch, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   which ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cw != CUDA_SUCCESS) {
+            set_error("gemm: cuTensorMapEncodeTiled (weights) failed with %d (n_out=%d k=%d fmt=%d)", (int)cw, m.n_out, m.k, m.fmt);
+            return ERR_CUDA;
+        }
+    }
+    out->valid = 1;
     return OK;
 }
 
@@ -938,7 +969,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
     g.recv_off = (gs.n_tile + 31) / 32 * 32 * G_BM * 2;
     g.counters = reinterpret_cast<unsigned*>(scratch);
     g.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + (size_t)G_COUNTERS * 4) : nullptr;
-    int cta = 0, tile = 0;
+    int cta = 0, tile = 0, n_maps = 0;
     long long part = 0;
     for (int i = 0; i < n; ++i) {
         const GemmOp& op = ops[i];
@@ -964,43 +995,37 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
         const cuuint64_t gstride[1] = {(cuuint64_t)m.k * 2};
         const cuuint32_t box[2] = {(cuuint32_t)G_BK, (cuuint32_t)gs.tma_rows};
         const cuuint32_t estr[2] = {1, 1};
-        const CUresult cr = encode(&maps.m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(op.x), gdim, gstride, box,
+        const CUresult cr = encode(&maps.t[pb.x_map = (signed char)n_maps++], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(op.x), gdim, gstride, box,
                                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) {
             set_error("gemm: cuTensorMapEncodeTiled failed with %d (rows=%d k=%d)", (int)cr, rows, m.k);
             return ERR_CUDA;
         }
-        // weights: rows as they are stored; the block scales need a row pitch of a multiple of 16 bytes
-        pb.scale_map = m.fmt == FMT_FP4 && m.k % 256 == 0 && ((uintptr_t)m.scale & 15) == 0 ? 1 : 0;
-        for (int which = 0; which < 1 + pb.scale_map; ++which) {
-            const cuuint64_t pitch = which ? m.k / 16 : (m.fmt == FMT_F16 ? 2ull * m.k : m.fmt == FMT_I8 ? (cuuint64_t)m.k : m.k / 2);
-            const cuuint64_t wdim[2] = {pitch, (cuuint64_t)m.n_out};
-            const cuuint32_t wbox[2] = {which ? 16u : (cuuint32_t)G_RAW_ROW, (cuuint32_t)G_BM};
-            const CUresult cw = encode(which ? &maps.s[i] : &maps.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
-                                       const_cast<void*>(which ? m.scale : m.w), wdim, &pitch, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                       which ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
-                                       CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (cw != CUDA_SUCCESS) {
-                set_error("gemm: cuTensorMapEncodeTiled (weights) failed with %d (n_out=%d k=%d fmt=%d)", (int)cw, m.n_out, m.k, m.fmt);
-                return ERR_CUDA;
-            }
+        WeightMaps own;
+        const WeightMaps* wm = op.maps && op.maps->valid ? op.maps : &own;
+        if (wm == &own) {
+            st = encode_weight_maps(m, &own);
+            if (st != OK) return st;
         }
-        if (!pb.scale_map) maps.s[i] = maps.w[i];
+        maps.t[pb.w_map = (signed char)n_maps++] = wm->w;
+        // (the obligatory maps of the products behind this one keep their places)
+        const int room = G_MAX_MAPS - n_maps - 2 * (n - 1 - i);
+        pb.s_map = pb.y_map = pb.r_map = -1;
         // output / residual tiles through the TMA unit when the row pitch and the pointers allow it
-        pb.tma_out = (m.n_out % 8 == 0 && m.n_out >= G_BM && ((uintptr_t)op.y & 15) == 0 &&
-                      (op.epi != EPI_RESID || ((uintptr_t)op.resid & 15) == 0)) ? 1 : 0;
-        maps.y[i] = maps.m[i];
-        maps.r[i] = maps.m[i];
-        if (pb.tma_out) {
+        const int out_maps = op.epi == EPI_RESID ? 2 : 1;
+        if (m.n_out % 8 == 0 && m.n_out >= G_BM && ((uintptr_t)op.y & 15) == 0 && (op.epi != EPI_RESID || ((uintptr_t)op.resid & 15) == 0) &&
+            out_maps <= room) {
+            pb.y_map = (signed char)n_maps++;
+            if (op.epi == EPI_RESID) pb.r_map = (signed char)n_maps++;
             const cuuint64_t odim[2] = {(cuuint64_t)m.n_out, (cuuint64_t)rows};
             const cuuint64_t ostride[1] = {(cuuint64_t)m.n_out * 2};
             const cuuint32_t obox[2] = {(cuuint32_t)G_BM, 32};
-            CUresult c2 = encode(&maps.y[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, op.y, odim, ostride, obox, estr,
+            CUresult c2 = encode(&maps.t[pb.y_map], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, op.y, odim, ostride, obox, estr,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (c2 == CUDA_SUCCESS && op.epi == EPI_RESID)
-                c2 = encode(&maps.r[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(op.resid), odim, ostride, obox,
+                c2 = encode(&maps.t[pb.r_map], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(op.resid), odim, ostride, obox,
                             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (c2 != CUDA_SUCCESS) {
@@ -1008,9 +1033,9 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
                 return ERR_CUDA;
             }
         }
+        if (wm->scale_map && (pb.y_map < 0 ? room : room - out_maps) > 0) maps.t[pb.s_map = (signed char)n_maps++] = wm->s;
     }
     for (int i = n; i < G_MAX_OPS; ++i) g.cta_base[i] = 0x7fffffff;
-    for (int i = n; i < G_MAX_OPS; ++i) maps.m[i] = maps.y[i] = maps.r[i] = maps.w[i] = maps.s[i] = maps.m[0];
 
     const size_t smem = 1024 + block_smem(gs.n_tile);
     {
@@ -1044,9 +1069,9 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
 }
 
 int gemm_launch(const ab_mat& m, int rows, const __half* x, __half* y, int epi, const __half* resid, void* scratch,
-                size_t scratch_bytes, cudaStream_t stream, bool pdl) {
+                size_t scratch_bytes, cudaStream_t stream, bool pdl, const WeightMaps* maps) {
     GemmOp op = {};
-    op.w = m; op.x = x; op.y = y; op.epi = epi; op.resid = resid;
+    op.w = m; op.x = x; op.y = y; op.epi = epi; op.resid = resid; op.maps = maps;
     return gemm_group_launch(&op, 1, rows, scratch, scratch_bytes, stream, pdl);
 }
 
