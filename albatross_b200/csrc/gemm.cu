@@ -849,33 +849,13 @@ int split_recv_slots(int n_tile, int ks) {
     return fit < own_max ? fit : own_max;
 }
 
-// Batch rows per block tile for more rows than one tile holds. A block's time is its k-steps times what one costs (the
-// tensor core's 2.1 cycles per batch row, the hand-over's 450 below that) plus what surrounds them, and a launch takes
-// as many of those as there are rounds of blocks over the SMs: the tile with the smallest product. With the fixed tile of 256
-// that this replaces, 768 rows of a 4096-row matrix kept 96 SMs busy (192 rows: 128 SMs), and r, k, v with their adapters
-// ended in a third round of ten blocks (768 rows int8, 4096 rows of 4096 inputs: 29.2 -> 25.8 us, of 16384: 89.9 -> 85.4).
-int pick_tile(const GemmOp* ops, int n, int rows, int n_sm) {
-    long long m_tiles = 0, ksteps = 1, best = 0;
-    for (int i = 0; i < n; ++i) {
-        m_tiles += (ops[i].w.n_out + G_BM - 1) / G_BM;
-        ksteps = std::max(ksteps, (long long)(ops[i].w.k + G_BK - 1) / G_BK);
-    }
-    int pick = 256;
-    for (int t = 320; t >= 128; t -= 32) {   // whole 32-row chunks: the next tile's rows are not this one's to store
-        const long long blocks = m_tiles * ((rows + t - 1) / t), rounds = (blocks + n_sm - 1) / n_sm;
-        const long long cost = rounds * (ksteps * std::max(450, 21 * t / 10) + 6000 + 15 * t);
-        if (best == 0 || cost < best) { best = cost; pick = t; }
-    }
-    return pick;
-}
-
-// fixed_tile: the tile of more than 320 batch rows (0: the best one).
-GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int fixed_tile = 0) {
+// tall_tile: the batch rows per tile for more rows than one tile holds.
+GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int tall_tile) {
     GroupShape gs = {};
     if (rows <= 256) { gs.n_tile = (rows + 15) & ~15; gs.n_first = gs.tma_rows = gs.n_tile; }
     else if (rows <= 320) { gs.n_tile = (rows + 31) & ~31; gs.n_first = 192; gs.tma_rows = gs.n_tile / 2; }
     else {
-        gs.n_tile = gs.n_first = gs.tma_rows = fixed_tile ? fixed_tile : pick_tile(ops, n, rows, n_sm > 0 ? n_sm : 148);
+        gs.n_tile = gs.n_first = gs.tma_rows = tall_tile;
         if (gs.n_tile > 256) { gs.n_first = 192; gs.tma_rows = gs.n_tile / 2; }
     }
     gs.tmem_cols = 32;
@@ -916,6 +896,34 @@ GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int fixed_t
     return gs;
 }
 
+// The shape a launch runs with. For more than 320 rows the tile height is a choice: fewer, taller tiles read the weights fewer
+// times and may be split along K, more and lower ones fill the SMs without an exchange. A block's time is its k-steps times
+// what one costs (420 cycles up to 128 rows, where two share a hand-over; above, the tensor core's 2.1 per row, 450 at least)
+// plus what surrounds them; a launch takes as many of those as there are rounds of blocks over the SMs, and the exchange where
+// it is split. The height with the smallest sum; over 96 products of 400 - 768 rows that is within 10 % of the fastest and level
+// with it on average. 400 rows, int8, a fixed tile of 256, this rule, and one that leaves the split out: 4096 x 4096 inputs 22.9, 21.1
+// (128 rows), 20.8 us; 2560 x 10240 inputs 29.8, 28.9 (224 rows, three ways), 38.8 (128 rows, 80 blocks of 160 k-steps).
+// A height whose partial sums need more scratch than 256 rows do is left out: what a caller's scratch area has to hold, and
+// which products the built-in one takes, does not depend on the choice.
+constexpr int G_TALL = 256;
+GroupShape launch_shape(const GemmOp* ops, int n, int rows, int n_sm) {
+    const GroupShape ref = group_shape(ops, n, rows, n_sm, G_TALL);
+    if (rows <= 320) return ref;
+    const int sms = n_sm > 0 ? n_sm : 148;
+    GroupShape pick = ref;
+    long long best = 0;
+    for (int t = 320; t >= 128; t -= 32) {   // whole 32-row chunks: the next tile's rows are not this one's to store
+        const GroupShape gs = t == G_TALL ? ref : group_shape(ops, n, rows, n_sm, t);
+        if (gs.part_floats > ref.part_floats) continue;
+        int ksteps = 1;
+        for (int i = 0; i < n; ++i) ksteps = std::max(ksteps, ((ops[i].w.k + G_BK - 1) / G_BK + gs.ksplit[i] - 1) / gs.ksplit[i]);
+        const int rounds = (gs.grid_x * gs.n_tiles_y + sms - 1) / sms, per_step = t <= 128 ? 420 : std::max(450, 21 * t / 10);
+        const long long cost = rounds * ((long long)ksteps * per_step + 6000 + 30 * t) + (gs.n_split_tiles ? 4000 + 30 * t : 0);
+        if (best == 0 || cost < best) { best = cost; pick = gs; }
+    }
+    return pick;
+}
+
 }  // namespace
 
 // SMs of the current device (148 on B200); the split-K decisions depend on it.
@@ -930,9 +938,8 @@ size_t gemm_group_scratch_bytes(const GemmOp* ops, int n, int rows) {
     if (!ops || n < 1 || n > G_MAX_OPS || rows <= 0) return 0;
     for (int i = 0; i < n; ++i)
         if (ops[i].w.n_out <= 0 || ops[i].w.k <= 0) return 0;
-    // (never less than for tiles of 256 rows: what a caller's scratch area has to hold does not depend on the tile picked)
-    const long long floats = std::max(group_shape(ops, n, rows, current_sm_count()).part_floats, group_shape(ops, n, rows, current_sm_count(), 256).part_floats);
-    return (size_t)G_COUNTERS * 4 + (size_t)floats * 4 + 256;
+    // (launch_shape never takes more)
+    return (size_t)G_COUNTERS * 4 + (size_t)group_shape(ops, n, rows, current_sm_count(), G_TALL).part_floats * 4 + 256;
 }
 size_t gemm_scratch_bytes(const ab_mat& m, int rows) {
     GemmOp op = {};
@@ -947,14 +954,14 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
         if (s != OK) return s;
     }
     const int n_sm = current_sm_count();
-    GroupShape gs = group_shape(ops, n, rows, n_sm);
+    GroupShape gs = launch_shape(ops, n, rows, n_sm);
     AB_CHECK_ARG(gs.n_split_tiles <= G_COUNTERS, "gemm: too many split-K tiles");
     if (gs.n_split_tiles > 0 && (gs.grid_x * gs.n_tiles_y > n_sm || (size_t)G_COUNTERS * 4 + (size_t)gs.part_floats * 4 > scratch_bytes)) {
         // the blocks of a split tile wait for one another, so all of them must be resident (one block per SM), and their
         // partial sums must fit the scratch area; a split grid for which that does not hold is launched without the split
         GemmOp unsplit[G_MAX_OPS];
         for (int i = 0; i < n; ++i) unsplit[i] = ops[i];
-        gs = group_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
+        gs = launch_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
     }
     AB_CHECK_ARG(gs.part_floats == 0 || (scratch && ((uintptr_t)scratch & 15) == 0), "gemm: split-K needs a 16-byte aligned scratch area");
     EncodeTiledFn encode;
@@ -1138,6 +1145,25 @@ int static_scratch_reset(cudaStream_t stream) {
 namespace {
 }  // namespace
 }  // namespace ab
+
+extern "C" int ab_gemm_plan_selftest(const int32_t* fmt, const int32_t* n_out, const int32_t* k, int n, int rows, int n_sm, int32_t* tile,
+                                     int32_t* blocks, int32_t* ksplit) {
+    using namespace ab;
+    AB_CHECK_ARG(fmt && n_out && k && tile && blocks && ksplit && n >= 1 && n <= G_MAX_OPS && rows > 0 && n_sm >= 0, "ab_gemm_plan_selftest: bad argument");
+    GemmOp ops[G_MAX_OPS] = {};
+    for (int i = 0; i < n; ++i) {
+        AB_CHECK_ARG(n_out[i] > 0 && k[i] > 0, "ab_gemm_plan_selftest: empty matrix");
+        ops[i].w.fmt = fmt[i]; ops[i].w.n_out = n_out[i]; ops[i].w.k = k[i];
+    }
+    const GroupShape gs = launch_shape(ops, n, rows, n_sm), ref = group_shape(ops, n, rows, n_sm, G_TALL);
+    AB_CHECK_ARG(gs.part_floats <= ref.part_floats, "ab_gemm_plan_selftest: %lld partial sums, scratch for %lld", gs.part_floats, ref.part_floats);
+    AB_CHECK_ARG(gs.n_split_tiles == 0 || gs.grid_x * gs.n_tiles_y <= n_sm, "ab_gemm_plan_selftest: %d blocks of a split grid", gs.grid_x * gs.n_tiles_y);
+    AB_CHECK_ARG(gs.n_tiles_y * gs.n_tile >= rows && (gs.n_tiles_y == 1 || gs.n_tile % 32 == 0), "ab_gemm_plan_selftest: tiles of %d rows", gs.n_tile);
+    *tile = gs.n_tile;
+    *blocks = gs.grid_x * gs.n_tiles_y;
+    for (int i = 0; i < n; ++i) ksplit[i] = gs.ksplit[i];
+    return OK;
+}
 
 extern "C" int ab_gemm_static(const ab_mat* m, int rows, const void* x, void* y, int epi, const void* resid, void* stream) {
     using namespace ab;

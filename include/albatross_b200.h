@@ -109,6 +109,12 @@ size_t ab_gemm_scratch_bytes(const ab_mat* m, int rows);
 int ab_gemm(const ab_mat* m, int rows, const void* x, void* y, int epi, const void* resid, void* scratch,
             void* stream);
 
+/* Host-only self-check of how a launch of `n` products (HOST arrays: weight format, output rows, inputs) of `rows` batch rows
+ * is cut up on a GPU of `n_sm` SMs: batch rows per tile, blocks, and into how many parts each product's K is split. Fails if
+ * the partial sums would not fit ab_gemm_scratch_bytes or a split grid would not be resident at once. Runs without a GPU. */
+int ab_gemm_plan_selftest(const int32_t* fmt, const int32_t* n_out, const int32_t* k, int n, int rows, int n_sm, int32_t* tile,
+                          int32_t* blocks, int32_t* ksplit);
+
 /* ab_gemm without a scratch argument (no counterpart in the reference). The split-K counters and partial tiles
  * live in a fixed AB_GEMM_STATIC_SCRATCH_BYTES array inside the library, so the call neither receives nor makes
  * any device allocation. It is for callers that have no device memory to hand over and must not create any at

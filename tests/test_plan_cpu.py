@@ -100,6 +100,37 @@ def test_workspace_holds_the_partial_sums_of_a_prompts_last_product(fmt, D, V):
         _lib.lib.ab_model_destroy(x)
 
 
+def _gemm_plan(ops, rows, n_sm=148):
+    n = len(ops)
+    arr = lambda v: (C.c_int32 * n)(*v)
+    tile, blocks, ks = C.c_int32(0), C.c_int32(0), (C.c_int32 * n)()
+    rc = _lib.lib.ab_gemm_plan_selftest(arr([o[0] for o in ops]), arr([o[1] for o in ops]), arr([o[2] for o in ops]), n, rows, n_sm,
+                                        C.byref(tile), C.byref(blocks), ks)
+    assert rc == 0, _lib.lib.ab_last_error().decode()
+    return tile.value, blocks.value, list(ks)
+
+
+@pytest.mark.parametrize("fmt", [I8, FP4, F16])
+@pytest.mark.parametrize("n_out,k,rows,blocks,ksteps", [
+    (2560, 10240, 400, 100, 54), (2560, 10240, 512, 100, 54), (4096, 16384, 400, 100, 128), (2048, 8192, 640, 100, 43),   # long K: split
+    (2560, 2560, 400, 80, 40), (768, 768, 768, 36, 12),                                                                    # short: low tiles
+    (16384, 4096, 400, 256, 64), (4096, 4096, 768, 128, 64)])
+def test_tile_height_weighs_the_split_along_k(fmt, n_out, k, rows, blocks, ksteps):
+    """The k-steps a block is left with and the SMs at work, for products on both sides of the choice between low tiles and
+    tall ones that are split (bounds: the fastest of the seven heights, timed)."""
+    _, b, (ks,) = _gemm_plan([(fmt, n_out, k)], rows)
+    assert b >= blocks and -(-(k // 64) // ks) <= ksteps, (b, ks)
+
+
+@settings(max_examples=200, deadline=None)
+@given(st.lists(st.tuples(st.sampled_from([F16, I8, FP4]), st.integers(1, 20000), st.integers(1, 300)), min_size=1, max_size=7),
+       st.integers(1, 4000), st.sampled_from([148, 132, 1]))
+def test_every_plan_of_products_fits_its_scratch_and_the_gpu(segs, rows, n_sm):
+    """Checked inside: partial sums within the scratch area, a split grid resident at once, tiles of whole chunks."""
+    tile, _, _ = _gemm_plan([(f, n, 64 * k) for f, n, k in segs], rows, n_sm)
+    assert 16 <= tile <= 320
+
+
 def test_state_list_forgets_its_checks_when_changed():
     """The list forward() hands back carries the model's validation and program key; any in-place change of the list
     drops them, so a changed list is checked from scratch (it is still a plain list to its user)."""
