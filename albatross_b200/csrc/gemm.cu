@@ -51,7 +51,7 @@ namespace {
 #endif
 constexpr int G_NG = G_NG_;      // producer groups
 constexpr int G_PROD = 128 * G_NG;
-constexpr int GT = G_PROD + 128; // threads per block: producers + a warpgroup holding the TMA warp, the MMA warp and two idle warps
+constexpr int GT = G_PROD + 128; // threads per block: producers + a warpgroup of the activation, MMA and weight warps and an idle one
                                  // (register re-allocation works on whole, aligned warpgroups)
 #ifndef G_STAGES_
 #define G_STAGES_ 4
@@ -350,8 +350,8 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
-    // Registers go where the work is: the producers' de-quantisation needs more than an even share, the two single-thread
-    // warps and the idle ones far less. (Whole warpgroups execute these: warps 0-3, 4-7, 8-11 / 12-15.)
+    // Registers go where the work is: the producers' de-quantisation needs more than an even share, the warps that only issue
+    // copies and MMAs far less. (Whole warpgroups execute these: warps 0-3, 4-7, 8-11 / 12-15.)
     if (warp < 4 * G_NG) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(G_REGS_PROD));
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G_REGS_REST));
     // Under programmatic stream serialisation the next grid may start now; like this one it begins with its weight
@@ -877,8 +877,10 @@ GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int tall_ti
             if (ks > ksteps / 8) ks = ksteps / 8;
             if (ks < 1) ks = 1;
         } else if (base_ctas < n_sm && slow_ctas > 0 && ops[i].w.fmt == FMT_F16 && ksteps >= 32) {
-            // A nearly full grid whose fp16 products (twice to four times the bytes per k-step of the quantised
-            // ones, fetched only two k-steps ahead) would finish last: the idle SMs take slices of their K loops.
+            // A nearly full grid whose fp16 products move two to four times the bytes per k-step of the quantised ones: they
+            // would finish last, and the idle SMs take slices of their K loops. A step of two blocks, 4096 wide, with and
+            // without (us): int8 8 rows 242, 248; 100 rows 324, 333; 320 rows 621, 644; nvfp4 8 rows 228, 227; 64 rows
+            // 281, 285; 320 rows 603, 620; all fp16 up to 160 rows alike, 320 rows 664, 676.
             ks = 1 + (n_sm - base_ctas) / slow_ctas;
             if (ks > 8) ks = 8;
             if (ks > ksteps / 8) ks = ksteps / 8;
