@@ -418,8 +418,8 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
                         // A slot's earlier content may have been another group's, and copies finish in any order: that copy
                         // may still be under way although this group's last one, issued after it, has landed. The phase bit
                         // alone cannot tell "two phases back" from "done", so first see that the earlier content has been
-                        // used up. (Its copy had been issued by then - copies are issued in order and there are more slots
-                        // than the groups are apart - so this wait is at most one phase back.)
+                        // used up. (Its copy had been issued by then - copies are issued in order and there are enough slots,
+                        // see slots_suffice - so this wait is at most one phase back.)
                         if (reused) wait_ok(&raw_empty[slot], parity ^ 1u);
                         wait_ok(&raw_full[slot], parity);
                     }
@@ -832,18 +832,27 @@ struct GroupShape {
 };
 
 // Shared memory of a block (beyond the 1 KB alignment slack): a block owns its SM (registers), so it takes all of it.
-constexpr size_t G_SMEM = 225 * 1024;
-size_t block_smem(int n_tile) { (void)n_tile; return G_SMEM; }
-// k-steps per operand stage (see gemm_tc_kernel) and what the stages leave for the raw weight slots: at least 4 slots of one
-// k-step per stage, 6 of two.
-int stage_ksteps(int n_tile) { return n_tile <= 128 ? 2 : 1; }
-size_t raw_smem(int n_tile) { return G_SMEM - (size_t)G_STAGES * stage_ksteps(n_tile) * n_tile * 128; }
+constexpr int G_SMEM = 225 * 1024;
+// k-steps per operand stage (see gemm_block) and what the stages leave for the raw weight slots.
+constexpr int stage_ksteps(int n_tile) { return n_tile <= 128 ? 2 : 1; }
+constexpr int raw_smem(int n_tile) { return G_SMEM - G_STAGES * stage_ksteps(n_tile) * n_tile * 128; }
+// What the phase bits of the slots rely on (see the wait in gemm_block): when a producer group comes to a k-step, the copy
+// that filled its slot the time before has been issued. Copies are issued in order, so that holds if there are at least as
+// many slots as lie between two k-steps that the group visits one after the other. The tallest tiles leave the fewest: 320
+// rows 4 slots (fp16: 3 needed, int8: 2) or 3 (NVFP4 with its scales: 1), 128 rows, two k-steps a stage, 6 (5, 3) or 5 (2).
+constexpr bool slots_suffice(int fmt, int n_tile) {
+    const int ks = stage_ksteps(n_tile), apart = G_NG * ks - (ks - 1), per = raw_ksteps(fmt);
+    return raw_smem(n_tile) / raw_slot_bytes(fmt) >= (apart + per - 1) / per;
+}
+static_assert(slots_suffice(FMT_F16, 320) && slots_suffice(FMT_I8, 320) && slots_suffice(FMT_FP4, 320) && slots_suffice(FMT_F16, 128) &&
+                  slots_suffice(FMT_I8, 128) && slots_suffice(FMT_FP4, 128),
+              "too few raw weight slots for this number of operand stages and producer groups");
 // Split K: how many of its own chunks a block can fetch the other blocks' partial sums for at a time. They land
 // in the operand stages behind the output staging area.
 int split_recv_slots(int n_tile, int ks) {
     const int n_chunks = (n_tile + 31) / 32;
     const size_t stage_bytes = (size_t)n_chunks * 32 * G_BM * 2;
-    const size_t avail = block_smem(n_tile) - stage_bytes;
+    const size_t avail = G_SMEM - stage_bytes;
     const int own_max = (n_chunks + ks - 1) / ks;
     const int fit = (int)(avail / ((size_t)(ks - 1) * G_CHUNK_F32));
     return fit < own_max ? fit : own_max;
@@ -974,7 +983,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
     GemmMaps maps;
     g.n_prob = n; g.rows = rows; g.n_tile = gs.n_tile; g.n_first = gs.n_first; g.tma_rows = gs.tma_rows; g.tmem_cols = gs.tmem_cols;
     g.a_col0 = (gs.n_tile + 31) & ~31;
-    g.raw_bytes = (int)raw_smem(gs.n_tile);
+    g.raw_bytes = raw_smem(gs.n_tile);
     g.recv_off = (gs.n_tile + 31) / 32 * 32 * G_BM * 2;
     g.counters = reinterpret_cast<unsigned*>(scratch);
     g.partials = scratch ? reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + (size_t)G_COUNTERS * 4) : nullptr;
@@ -1046,7 +1055,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
     }
     for (int i = n; i < G_MAX_OPS; ++i) g.cta_base[i] = 0x7fffffff;
 
-    const size_t smem = 1024 + block_smem(gs.n_tile);
+    const size_t smem = 1024 + G_SMEM;
     {
         static PerDeviceOnce once;
         const int s = once.run(nullptr, [](DeviceProps& d) -> int {
