@@ -85,7 +85,6 @@ struct GemmProb {
 struct GemmGroup {
     int cta_base[G_MAX_OPS];   // first blockIdx.x of each product (unused ones: INT_MAX)
     GemmProb pr[G_MAX_OPS];
-    int n_prob;
     int rows;       // batch rows (B*T)
     int n_tile;     // batch rows per block tile
     int n_first;    // batch rows of the first MMA of a k-substep (n_tile, or 192 when a second MMA takes the rest)
@@ -981,7 +980,7 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
 
     GemmGroup g = {};
     GemmMaps maps;
-    g.n_prob = n; g.rows = rows; g.n_tile = gs.n_tile; g.n_first = gs.n_first; g.tma_rows = gs.tma_rows; g.tmem_cols = gs.tmem_cols;
+    g.rows = rows; g.n_tile = gs.n_tile; g.n_first = gs.n_first; g.tma_rows = gs.tma_rows; g.tmem_cols = gs.tmem_cols;
     g.a_col0 = (gs.n_tile + 31) & ~31;
     g.raw_bytes = raw_smem(gs.n_tile);
     g.recv_off = (gs.n_tile + 31) / 32 * 32 * G_BM * 2;
@@ -1153,8 +1152,6 @@ int static_scratch_reset(cudaStream_t stream) {
     return OK;
 }
 
-namespace {
-}  // namespace
 }  // namespace ab
 
 extern "C" int ab_gemm_plan_selftest(const int32_t* fmt, const int32_t* n_out, const int32_t* k, int n, int rows, int n_sm, int32_t* tile,
