@@ -504,8 +504,10 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         const int c = lane & 7, row0 = (warp * 4 + (lane >> 3)) * 4;
         float* sbase = p.state + (size_t)bh * 4096;
         f32x2 S[4][4];
+        const bool mine = AB_BC(bh < p.B * p.H && row0 + 4 <= 64 && 32 + 4 * c + 4 <= 64);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ld_cols(S[i], sbase + (row0 + i) * 64, c);
+        for (int i = 0; i < 4; ++i)
+            if (mine) ld_cols(S[i], sbase + (row0 + i) * 64, c);
         for (int ch = 0; ch < n_chunks; ++ch) {
             const int buf = ch % SC_NBUF, ns = min(SC_CH, T - ch * SC_CH);
             ScanChunk& ck = ring[buf];
@@ -548,7 +550,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
 #pragma unroll
                 for (int i = 0; i < 4; ++i) sa[i] += __shfl_xor_sync(0xffffffffu, sa[i], 4);
                 exch3();
-                if (j > 0 && !(lane & 4)) ck.y[j - 1][yrow] = y0;
+                if (j > 0 && !(lane & 4) && AB_BC(j <= SC_CH && yrow < 64)) ck.y[j - 1][yrow] = y0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) row_add(S[i], bb, sa[i]);
 #pragma unroll
@@ -563,12 +565,13 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
             exch1();
             exch2();
             exch3();
-            if (!(lane & 4)) ck.y[ns - 1][yrow] = y0;
+            if (!(lane & 4) && AB_BC(ns >= 1 && ns <= SC_CH)) ck.y[ns - 1][yrow] = y0;
             __syncwarp();
             if (lane == 0) mbar_arrive(&done[buf]);
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) st_cols(sbase + (row0 + i) * 64, c, S[i]);
+        for (int i = 0; i < 4; ++i)
+            if (mine) st_cols(sbase + (row0 + i) * 64, c, S[i]);
     } else if (warp < SC_SCAN + SC_PRE) {
         // lane = channels 2 * lane and 2 * lane + 1
         struct In { __half2 r, k, v, w, a, g, f; };   // OP: g = b; else g = v gate, f = v_first
@@ -581,6 +584,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         auto fetch = [&](int t, In& x) {
             if (t >= T) return;
             const size_t o = base + (size_t)t * p.D + 2 * lane;
+            if (!AB_BC(o + 2 <= (size_t)p.B * T * p.D && gc + 2 <= p.D)) return;
             x.r = ldh(p.r + o); x.k = ldh(p.k + o); x.v = ldh(p.v + o); x.w = ldh(p.w_raw + o); x.a = ldh(p.a_raw + o);
             if (OP || gated) x.g = ldh(p.vg_raw + o);
             if (gated) x.f = vf_pairs ? ldh(p.v_first + o) : __halves2half2(__ldcg(p.v_first + o), __ldcg(p.v_first + o + 1));
@@ -607,6 +611,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
             for (int q = 0; q < PER; ++q) {
                 const int j = pw + q * SC_PRE, t = ch * SC_CH + j;
                 if (j >= SC_CH || t >= T) break;
+                if (!AB_BC(t >= 0 && base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) continue;
                 ScanStep& s = ring[buf].s[j];
                 auto put = [&](float* d, float x, float y) { *reinterpret_cast<float2*>(d + 2 * lane) = make_float2(x, y); };
                 const float2 r = __half22float2(cur[q].r), k = __half22float2(cur[q].k), w = __half22float2(cur[q].w), a = __half22float2(cur[q].a);
@@ -668,6 +673,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                 if (j >= SC_CH || t >= T) break;
                 const float2 y = *reinterpret_cast<const float2*>(&ck.y[j][2 * lane]);
                 __half2* out = reinterpret_cast<__half2*>(p.out + base + (size_t)t * p.D + 2 * lane);
+                if (!AB_BC(base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) continue;
                 if (OP) {
                     *out = __floats2half2_rn(y.x, y.y);
                 } else {

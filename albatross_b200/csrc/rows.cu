@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
         for (int v = 0; v < V; ++v) {
             const int i = threadIdx.x + v * RT;
             // an ordinary (coherent) load that stays behind the wait above: the row was written by the preceding kernel
-            if (i < nv)
+            if (i < nv && AB_BC(seq < p.B && t >= 0 && t < p.T && 8 * (i + 1) <= p.D))
                 asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                              : "=r"(raw[v].x), "=r"(raw[v].y), "=r"(raw[v].z), "=r"(raw[v].w)
                              : "l"(xs + (size_t)t * nv + i)
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
     } else {
 #pragma unroll
         for (int v = 0; v < V; ++v)
-            if (threadIdx.x + v * RT < nv) prev[v] = state[threadIdx.x + v * RT];
+            if (threadIdx.x + v * RT < nv && AB_BC(seq < p.B)) prev[v] = state[threadIdx.x + v * RT];
     }
     load(t0, raw);
     for (int t = t0; t < t1; ++t) {
@@ -284,7 +284,8 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
                         const float2 mf = __half22float2(mh[e]);
                         oh[e] = __floats2half2_rn(c[2 * e] + rh(d[2 * e] * mf.x), c[2 * e + 1] + rh(d[2 * e + 1] * mf.y));
                     }
-                    reinterpret_cast<uint4*>(p.out[j] + ((size_t)seq * p.T + t) * p.D)[i] = o;
+                    if (AB_BC(seq < p.B && t >= t0 && t < p.T && j < 6 && 8 * (i + 1) <= p.D))
+                        reinterpret_cast<uint4*>(p.out[j] + ((size_t)seq * p.T + t) * p.D)[i] = o;
                 }
                 prev[v] = xn[v];
             }
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
         }
 #pragma unroll
         for (int v = 0; v < V; ++v)
-            if (threadIdx.x + v * RT < nv) state[threadIdx.x + v * RT] = prev[v];
+            if (threadIdx.x + v * RT < nv && AB_BC(seq < p.B && 8 * (int)(threadIdx.x + v * RT + 1) <= p.D)) state[threadIdx.x + v * RT] = prev[v];
     }
 }
 
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restric
     };
     // elements up to the first 16-byte boundary, chunks of eight, the rest
     const int head = min(V, (int)((16 - ((uintptr_t)lr & 15)) & 15) / 2), nv = (V - head) / 8;
-    if ((int)threadIdx.x < head) take(__half2float(lr[threadIdx.x]), threadIdx.x);
+    if ((int)threadIdx.x < head && AB_BC((int)threadIdx.x < V)) take(__half2float(lr[threadIdx.x]), threadIdx.x);
     const uint4* body = reinterpret_cast<const uint4*>(lr + head);
     int buf = 0;
     for (int c0 = 0; c0 < nv; c0 += NT * SR_U, buf ^= 1) {   // uniform in the block
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restric
 #pragma unroll
         for (int u = 0; u < SR_U; ++u) {
             const int c = c0 + u * NT + threadIdx.x;
-            if (c < nv) q[u] = __ldcs(body + c);
+            if (c < nv && AB_BC(c >= 0 && head + 8 * (c + 1) <= V)) q[u] = __ldcs(body + c);
         }
         __half top = __ushort_as_half((unsigned short)0xfc00u);   // -inf
 #pragma unroll
@@ -373,7 +374,8 @@ __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restric
             }
         }
     }
-    for (int i = head + nv * 8 + threadIdx.x; i < V; i += NT) take(__half2float(lr[i]), i);
+    for (int i = head + nv * 8 + threadIdx.x; i < V; i += NT)
+        if (AB_BC(i >= 0)) take(__half2float(lr[i]), i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
