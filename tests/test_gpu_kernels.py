@@ -154,10 +154,11 @@ def test_wkv7_sequences_around_the_chunk_size(B, H, T, shift):
 
 @pytest.mark.parametrize("T", [2, 8, 9, 40, 67])
 def test_wkv7_sequences_do_not_depend_on_the_batch(T):
-    """Few heads are shared by two blocks each, many take one: the same bits either way, and the same as step by step."""
+    """A head's result does not depend on the other sequences of the call or on where its block runs, and a sequence cut into
+    calls of any length gives the same bits: step by step (the plain kernel), and in two calls that end inside a chunk."""
     from albatross_b200 import RWKV7_BATCH_OP, _lib
     torch.manual_seed(T)
-    B, H = 40, 2                                       # 80 heads: one block each; a single sequence: two blocks per head
+    B, H = 40, 2
     kk = torch.nn.functional.normalize(torch.randn(B, T, H, 64), dim=-1).view(B, T, H * 64)
     vec = [torch.randn(B, T, H * 64), -torch.rand(B, T, H * 64) * 2 - 0.5, torch.randn(B, T, H * 64), torch.randn(B, T, H * 64), -kk,
            kk * torch.rand(B, T, H * 64)]
@@ -174,6 +175,10 @@ def test_wkv7_sequences_do_not_depend_on_the_batch(T):
             yt = RWKV7_BATCH_OP(S, *[v[b:b + 1, t:t + 1].contiguous() for v in vec])
             assert torch.equal(yt, y_all[b:b + 1, t:t + 1])
         assert torch.equal(S, S_all[b:b + 1])
+        cut = 3 * T // 5                               # 67 = 40 + 27, 40 = 24 + 16, 9 = 5 + 4, 8 = 4 + 4, 2 = 1 + 1
+        S = S0[b:b + 1].clone()
+        ys = [RWKV7_BATCH_OP(S, *[v[b:b + 1, t0:t1].contiguous() for v in vec]) for t0, t1 in ((0, cut), (cut, T))]
+        assert torch.equal(torch.cat(ys, 1), y_all[b:b + 1]) and torch.equal(S, S_all[b:b + 1])
     assert _lib.device_status() == 0
 
 
@@ -359,11 +364,13 @@ def test_device_sampler_exact(rows, V, kind):
         assert got.flatten().tolist() == _noisy_argmax(x, noise, 9).tolist(), (noise, kind)
 
 
-@pytest.mark.parametrize("D", [128, 256, 768, 4096, 5120])
-@pytest.mark.parametrize("B,T", [(1, 2), (3, 5), (2, 260), (5, 410)])
+@pytest.mark.parametrize("D,B,T", [(D, B, T) for D in (128, 256, 768, 4096, 5120) for B, T in ((1, 2), (3, 5), (2, 260), (5, 410))] +
+                         [(256, 3, 171), (4096, 3, 171), (8192, 3, 5), (8192, 3, 171), (8192, 5, 410)])
 def test_sequence_norm_and_lerps_through_a_model(B, T, D):
-    """The one-pass norm + token-shift kernel (1, 2 or 4 rows per block; row lengths up to its limit): the state it hands
-    over after T tokens is the normalised last row, and prompts give what the same tokens give one by one."""
+    """The one-pass norm + token-shift kernel (1 row per block, 2 from 512 rows, 4 from 2048; row lengths up to its limit of
+    8192): the state it hands over after T tokens is the normalised last row; a prefix gives what its tokens give one by one
+    (other kernels); and a prompt gives, at every position and in every state, what it gives in pieces of under 512 rows,
+    which one-row blocks work on (171 = 3 mod 4 tokens and 410 = 2 mod 4: the last block of a sequence is not full)."""
     from albatross_b200 import RWKV_x070, synth
     import types
     cfg = (1, D, 64, (16, 16, 16, 16))
@@ -382,3 +389,15 @@ def test_sequence_norm_and_lerps_through_a_model(B, T, D):
     _, pre = model.forward_batch([r[:min(T, 12)] for r in ids], None)
     for a, b in zip(pre, one):
         assert rel_err(a.float().cpu(), b.float().cpu()) < 1e-2     # fp16 activations along two kernel families
+    if B * T >= 512:
+        whole, st = model.forward_batch(ids, None, True)            # logits of every position
+        parts, pst, n = [], None, 500 // B
+        for t in range(0, T, n):
+            lg, pst = model.forward_batch([r[t:t + n] for r in ids], pst, True)
+            parts.append(lg.view(B, -1, 64))
+        parts = torch.cat(parts, 1).float()
+        # The products of other row counts sum in another order, which moves fp16 roundings of the block's dozen stages (2**-11
+        # each, of the largest value at most); a wrong token-shift row changes its position by as much as the logits themselves.
+        assert rel_err(whole.view(B, T, 64).float().cpu(), parts.cpu()) < 2e-2
+        for a, b in zip(st, pst):
+            assert rel_err(a.float().cpu(), b.float().cpu()) < 2e-2
