@@ -32,8 +32,8 @@
 // that the memory and the hand-over between the warps, about 390 cycles a k-step whatever the batch (int8 rows at the
 // copy bandwidth: 350). Around the main loop a block spends 1 us before it (tensor memory, barriers, first rows on their
 // way) and 1 - 3 us behind it; the exchange of a split K costs 5 us.
-// 16384 x 4096, back to back: 320 rows nvfp4 39.2 -> 33.3 us, 64 rows nvfp4 32.0 -> 17.9, 8 rows int8 32.6 -> 19.7, against
-// the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below).
+// 16384 x 4096, back to back: 320 rows nvfp4 41.2 -> 35.4 us (1214 TFLOP/s), 64 rows nvfp4 32.0 -> 17.9, 8 rows int8 32.6 ->
+// 19.7, against the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below).
 #include <cuda.h>
 
 #include <algorithm>
@@ -108,11 +108,10 @@ static_assert(2 * G_MAX_OPS <= G_MAX_MAPS && sizeof(GemmMaps) + sizeof(GemmGroup
 // PTX wrappers (tcgen05 / TMA)
 // ---------------------------------------------------------------------------------------------
 // The wrappers named *_one are called by a whole, converged warp; one elected lane performs the operation. The election
-// sits inside the assembly on purpose: tcgen05 and TMA instructions take their operands from registers shared by the
-// warp, and in code that only one lane runs (`if (lane == 0)`) the compiler wraps every one of them in a loop that
-// moves the operands over lane by lane. An MMA issued that way took 95 - 120 cycles, which bounded every product here
-// whatever its batch (a k-step of four: 480 cycles at 16 batch rows as at 192); elected it takes 34 (N <= 64) and runs
-// at the tensor core's rate above (4 x N = 128: 257 cycles).
+// sits inside the assembly on purpose: an MMA issued from code that only one lane runs (`if (lane == 0)`) took 95 - 120
+// cycles, timed by the kernel's own clock, which bounded every product here whatever its batch (a k-step of four: 480 cycles
+// at 16 batch rows as at 192); elected like this it takes 34 (N <= 64) and runs at the tensor core's rate above (4 x N = 128:
+// 257 cycles).
 __device__ __forceinline__ void tma_load_2d_one(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
