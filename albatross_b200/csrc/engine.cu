@@ -436,7 +436,13 @@ GemmOp gemm_op(const ab_mat& w, const __half* x, __half* y, int epi, const Weigh
 int encode_maps(ab_model* m) {
     std::lock_guard<std::mutex> lock(m->maps_mu);
     if (!m->maps.empty()) return OK;
-    std::vector<LayerMaps> maps(m->layers.size());
+    std::vector<LayerMaps> maps;
+    try {   // (called from C)
+        maps.resize(m->layers.size());
+    } catch (const std::bad_alloc&) {
+        set_error("out of host memory for the tensor maps of %zu blocks", m->layers.size());
+        return ERR_TOO_LARGE;
+    }
     for (size_t i = 0; i < maps.size(); ++i) {
         const ab_layer& l = m->layers[i];
         LayerMaps& o = maps[i];
