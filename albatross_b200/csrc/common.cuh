@@ -229,7 +229,33 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // fp16 rounding points: the reference computes its glue in fp16 tensors, so each torch op rounds.
 __device__ __forceinline__ float rh(float v) { return __half2float(__float2half_rn(v)); }
-__device__ __forceinline__ float sigmoidf_(float v) { return 1.0f / (1.0f + __expf(-v)); }
+// Reciprocal, quotient and square root without branches. The compiler's own end in a test and a call for operands at the ends
+// of the range; nine of them in the per-step glue cut it into pieces that cannot overlap (4000 cycles for two steps whose
+// arithmetic is some 600 instructions; 2000 like this). These take the approximation of the hardware and one Newton step on
+// its residual, computed exactly by a fused multiply-add. The operands they are given stay clear of the range's ends; there
+// the results were the same as the compiler's for every float (reciprocal, root) and for 2^31 pairs of fp16 values
+// (quotient). Infinities and NaNs come out as they should. Two blocks of the network, 4096 wide: 8 sequences one step 250 -> 243 us, a
+// prompt of 768 tokens 1385 -> 1360, 5 of 37 tokens 398 -> 384.
+__device__ __forceinline__ float recip_(float d) {   // 1 <= d < 2^126, or NaN
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.f), r);
+}
+__device__ __forceinline__ float quot_(float x, float d) {   // 1e-12 <= d <= 65504, infinite or NaN
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = x * r;
+    return d > 65504.f ? q : fmaf(r, fmaf(-d, q, x), q);
+}
+__device__ __forceinline__ float root_(float x) {   // 0, 2^-60 <= x < 2^60, infinite or NaN
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    const float s = x * r, y = fmaf(0.5f * r, fmaf(-s, s, x), s);
+    return x > 0.f && x < 3e38f ? y : x;
+}
+__device__ __forceinline__ float sigmoidf_(float v) {   // (below -80 the result is 0 in fp16, and 1 is what it adds to in an exponent)
+    return recip_(1.0f + __expf(v < -80.f ? 80.f : -v));
+}
 
 constexpr int HEAD = 64;
 

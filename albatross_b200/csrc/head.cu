@@ -326,10 +326,10 @@ __global__ void __launch_bounds__(HB_THREADS, HB_BLOCKS) head_batch_kernel(const
             }
             ssq = warp_sum(ssq);
             rkr = rh(warp_sum(rkr));
-            const float nrm = fmaxf(rh(sqrtf(ssq)), 1e-12f);
+            const float nrm = fmaxf(rh(root_(ssq)), 1e-12f);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float kk = rh(kk0[e] / nrm);
+                const float kk = rh(quot_(kk0[e], nrm));
                 o.a[2 * lane + e] = __float2half_rn(-kk);
                 o.b[2 * lane + e] = __float2half_rn(kk * av[e]);
             }
@@ -640,8 +640,8 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                     put(s.v, v.x, v.y);
                     const float ssq = warp_sum(fmaf(ky, ky, kx * kx));
                     const float rkr = warp_sum(rh(rh(r.x * k2x) * r_k.x) + rh(rh(r.y * k2y) * r_k.y));
-                    const float nrm = fmaxf(rh(sqrtf(ssq)), 1e-12f);
-                    const float kkx = rh(kx / nrm), kky = rh(ky / nrm);
+                    const float nrm = fmaxf(rh(root_(ssq)), 1e-12f);
+                    const float kkx = rh(quot_(kx, nrm)), kky = rh(quot_(ky, nrm));
                     put(s.a, -kkx, -kky);
                     put(s.b, rh(kkx * ax), rh(kky * ay));
                     if (lane == 0) s.rkr = rh(rkr);

@@ -348,11 +348,11 @@ __device__ __forceinline__ void head_step(const HeadParams& p, int b, int h, int
         }
         ssq = warp_sum(ssq);
         rkr = rh(warp_sum(rkr));
-        const float nrm = fmaxf(rh(sqrtf(ssq)), 1e-12f);
+        const float nrm = fmaxf(rh(root_(ssq)), 1e-12f);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int c = lane + 32 * e;
-            const float kk = rh(kk0[e] / nrm);
+            const float kk = rh(quot_(kk0[e], nrm));
             sa_[c] = -kk;
             sb[c] = rh(kk * av[e]);
         }

@@ -415,3 +415,32 @@ def test_persistent_kernel_tags_wrap_around():
         if i % 100 == 99 or i >= 2290 or 1070 <= i <= 1080 or 2145 <= i <= 2155:
             assert torch.equal(lp, le), f"token {i}"
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 1), (260, 1), (3, 19)])
+def test_glue_at_the_ends_of_its_range(B, T):
+    """The branch-free reciprocal, quotient and root of the per-step glue where they could go wrong, in the batch-1, the few-
+    and many-sequence and the sequence kernels: gates and decays far beyond the exponential's range on both sides, a head whose
+    k is zero (norm 1e-12), and small ones. The tolerance is that of the logits everywhere (fp16 activations)."""
+    raw = synth.make_checkpoint("tiny", seed=0)
+    D = raw["emb.weight"].shape[1]
+    sign = torch.tensor([1.0, -1.0]).repeat(D // 2)
+    for name in list(raw):
+        if name.endswith((".a0", ".w0", ".v0")):
+            raw[name] = (sign * {"a": 300.0, "w": 90.0, "v": 6e4}[name[-2]]).view_as(raw[name])
+        if name.endswith(".k_k"):
+            kk = raw[name].clone().view(-1)
+            kk[:64] = 0.0
+            kk[64:128] *= 2e-3
+            raw[name] = kk.view_as(raw[name])
+    model, args = model_for("tiny", "int8", raw=raw)
+    o, _ = oracle_for("tiny", "int8", raw=raw)
+    ids = [seeded_tokens(args.vocab_size, T + 1, seed=b) for b in range(B)]
+    ref, st = new_state(args.n_layer, args.n_embd, batch=B), None if B > 1 else model.new_state()
+    for part in ([r[:T] for r in ids], [r[T:] for r in ids]):
+        want, ref = o.forward_tokens(part, ref)
+        if B > 1: got, st = model.forward_batch(part, st)
+        else: got, st = model.forward(part[0], st)
+        assert torch.isfinite(got).all() and rel_err(got.float().cpu().numpy().reshape(want.shape), want.numpy()) <= LOGIT_REL_TOL
+    for i in range(args.n_layer):
+        assert rel_err(st[3 * i + 1].cpu().numpy().reshape(ref[3 * i + 1].shape), ref[3 * i + 1].numpy()) <= LOGIT_REL_TOL
