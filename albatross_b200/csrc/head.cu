@@ -455,8 +455,18 @@ __global__ void __launch_bounds__(HB_THREADS, HB_BLOCKS) head_batch_kernel(const
 // head without the pipeline, as it was: 631 us; before whole chunks were unrolled 104, with one block of 512 threads per
 // SM 125). One sequence of 1024 steps: 225 us (1450 us; before unrolling 252).
 // OP = true: the operator's inputs (w = pre-transform decay in w_raw, a and b in a_raw / vg_raw), y stored as it is.
-constexpr int SC_CH = 8, SC_NBUF = 4, SC_SCAN = 4, SC_PRE = 4, SC_POST = 2;
-constexpr int SC_THREADS = 32 * (SC_SCAN + SC_PRE + SC_POST);
+//
+// WIDE: one block per SM with eight preparing and four finishing warps, for no more heads than SMs. The preparing warps keep two
+// or four steps apart in flight, which takes registers: within the 96 that two blocks per SM leave, a step's glue waited for
+// itself 2300 cycles (the model's step 311 ns where the operator's took 216, whose inputs need little preparation); with 120
+// registers and twice the warps it is off the chain. 768 steps of two blocks of the network, 4096 wide, int8: 1385 us, 1360
+// with glue free of branches (quot_ and its like), 1353 with a warp's steps side by side, 1156 with the registers, 1088 with
+// the warps; the operator, 1024 steps: 222 -> 210. 5 prompts of 37 tokens (320 heads) 384 in blocks of ten warps, two per SM,
+// 390 in wide ones.
+constexpr int SC_CH = 8, SC_NBUF = 4, SC_SCAN = 4;
+__host__ __device__ constexpr int scan_pre(bool wide) { return wide ? 8 : 4; }
+__host__ __device__ constexpr int scan_post(bool wide) { return wide ? 4 : 2; }
+__host__ __device__ constexpr int scan_threads(bool wide) { return 32 * (SC_SCAN + scan_pre(wide) + scan_post(wide)); }
 struct ScanStep {
     float a[64], w[64], k[64], b[64], r[64], v[64];
     float rkr, pad[3];
@@ -466,8 +476,9 @@ struct ScanChunk {
     float y[SC_CH][64];
 };
 
-template <bool OP>
-__global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_constant__ HeadParams p) {
+template <bool OP, bool WIDE>
+__global__ void __launch_bounds__(scan_threads(WIDE), WIDE ? 1 : 2) scan_kernel(const __grid_constant__ HeadParams p) {
+    constexpr int SC_PRE = scan_pre(WIDE), SC_POST = scan_post(WIDE);
     extern __shared__ __align__(128) unsigned char dsm[];   // SC_NBUF chunks
     __shared__ uint64_t full[SC_NBUF], done[SC_NBUF], vacant[SC_NBUF];
     __shared__ int s_failed;
@@ -582,19 +593,22 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         const bool vf_pairs = ((uintptr_t)p.v_first & 3) == 0;
         auto ldh = [](const __half* q) { return __ldcg(reinterpret_cast<const __half2*>(q)); };
         auto fetch = [&](int t, In& x) {
-            if (t >= T) return;
+            if (t >= T) { x = In{}; return; }
             const size_t o = base + (size_t)t * p.D + 2 * lane;
-            if (!AB_BC(o + 2 <= (size_t)p.B * T * p.D && gc + 2 <= p.D)) return;
+            if (!AB_BC(o + 2 <= (size_t)p.B * T * p.D && gc + 2 <= p.D)) { x = In{}; return; }
             x.r = ldh(p.r + o); x.k = ldh(p.k + o); x.v = ldh(p.v + o); x.w = ldh(p.w_raw + o); x.a = ldh(p.a_raw + o);
             if (OP || gated) x.g = ldh(p.vg_raw + o);
-            if (gated) x.f = vf_pairs ? ldh(p.v_first + o) : __halves2half2(__ldcg(p.v_first + o), __ldcg(p.v_first + o + 1));
+            if (gated) {
+                if (vf_pairs) x.f = ldh(p.v_first + o);
+                else x.f = __halves2half2(__ldcg(p.v_first + o), __ldcg(p.v_first + o + 1));
+            }
         };
         float2 w0, a0, v0, k_k, k_a, r_k;
         if (!OP) {
             w0 = ld2u(p.w0 + gc); a0 = ld2u(p.a0 + gc); k_k = ld2u(p.k_k + gc); k_a = ld2u(p.k_a + gc); r_k = ld2u(p.r_k + gc);
             v0 = gated ? ld2u(p.v0 + gc) : make_float2(0.f, 0.f);
         }
-        constexpr int PER = (SC_CH + SC_PRE - 1) / SC_PRE;   // steps of a chunk per pre warp
+        constexpr int PER = SC_CH / SC_PRE;   // steps of a chunk per pre warp
         In nxt[PER];
 #pragma unroll
         for (int q = 0; q < PER; ++q) fetch(pw + q * SC_PRE, nxt[q]);
@@ -607,11 +621,11 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                 fetch((ch + 1) * SC_CH + pw + q * SC_PRE, nxt[q]);
             }
             if (ch >= SC_NBUF) wait_for(&vacant[buf], (uint32_t)(ch / SC_NBUF - 1) & 1u);
+            // (steps beyond T are prepared from zeros and read by nobody; the steps of a warp run side by side)
+            float kx[PER], ky[PER], ax[PER], ay[PER], ssq[PER], rkr[PER];
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const int j = pw + q * SC_PRE, t = ch * SC_CH + j;
-                if (j >= SC_CH || t >= T) break;
-                if (!AB_BC(t >= 0 && base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) continue;
                 ScanStep& s = ring[buf].s[j];
                 auto put = [&](float* d, float x, float y) { *reinterpret_cast<float2*>(d + 2 * lane) = make_float2(x, y); };
                 const float2 r = __half22float2(cur[q].r), k = __half22float2(cur[q].k), w = __half22float2(cur[q].w), a = __half22float2(cur[q].a);
@@ -625,26 +639,41 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
                     // reference/rwkv7.py:284-297, with the decay in fp32 as on its single-token path (:241)
                     if (p.layer0) {
                         __half* d = p.v_first + base + (size_t)t * p.D + 2 * lane;
-                        if (vf_pairs) *reinterpret_cast<__half2*>(d) = cur[q].v;
-                        else { d[0] = __low2half(cur[q].v); d[1] = __high2half(cur[q].v); }
+                        if (t < T && AB_BC(base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) {
+                            if (vf_pairs) *reinterpret_cast<__half2*>(d) = cur[q].v;
+                            else { d[0] = __low2half(cur[q].v); d[1] = __high2half(cur[q].v); }
+                        }
                     } else {
                         const float2 g = __half22float2(cur[q].g), f = __half22float2(cur[q].f);
                         v.x = rh(v.x + rh(rh(f.x - v.x) * rh(sigmoidf_(rh(v0.x + g.x)))));
                         v.y = rh(v.y + rh(rh(f.y - v.y) * rh(sigmoidf_(rh(v0.y + g.y)))));
                     }
-                    const float ax = rh(sigmoidf_(rh(a0.x + a.x))), ay = rh(sigmoidf_(rh(a0.y + a.y)));
-                    const float kx = rh(k.x * k_k.x), ky = rh(k.y * k_k.y);
-                    const float k2x = rh(k.x * rh(1.f + rh(rh(ax - 1.f) * k_a.x))), k2y = rh(k.y * rh(1.f + rh(rh(ay - 1.f) * k_a.y)));
+                    ax[q] = rh(sigmoidf_(rh(a0.x + a.x))), ay[q] = rh(sigmoidf_(rh(a0.y + a.y)));
+                    kx[q] = rh(k.x * k_k.x), ky[q] = rh(k.y * k_k.y);
+                    const float k2x = rh(k.x * rh(1.f + rh(rh(ax[q] - 1.f) * k_a.x))), k2y = rh(k.y * rh(1.f + rh(rh(ay[q] - 1.f) * k_a.y)));
                     put(s.w, __expf(-0.606531f * sigmoidf_(rh(w0.x + w.x))), __expf(-0.606531f * sigmoidf_(rh(w0.y + w.y))));
                     put(s.k, k2x, k2y);
                     put(s.v, v.x, v.y);
-                    const float ssq = warp_sum(fmaf(ky, ky, kx * kx));
-                    const float rkr = warp_sum(rh(rh(r.x * k2x) * r_k.x) + rh(rh(r.y * k2y) * r_k.y));
-                    const float nrm = fmaxf(rh(root_(ssq)), 1e-12f);
-                    const float kkx = rh(quot_(kx, nrm)), kky = rh(quot_(ky, nrm));
-                    put(s.a, -kkx, -kky);
-                    put(s.b, rh(kkx * ax), rh(kky * ay));
-                    if (lane == 0) s.rkr = rh(rkr);
+                    ssq[q] = fmaf(ky[q], ky[q], kx[q] * kx[q]);
+                    rkr[q] = rh(rh(r.x * k2x) * r_k.x) + rh(rh(r.y * k2y) * r_k.y);
+                }
+            }
+            if (!OP) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)   // (warp_sum of all of them)
+#pragma unroll
+                    for (int q = 0; q < PER; ++q) {
+                        ssq[q] += __shfl_xor_sync(0xffffffffu, ssq[q], o);
+                        rkr[q] += __shfl_xor_sync(0xffffffffu, rkr[q], o);
+                    }
+#pragma unroll
+                for (int q = 0; q < PER; ++q) {
+                    ScanStep& s = ring[buf].s[pw + q * SC_PRE];
+                    const float nrm = fmaxf(rh(root_(ssq[q])), 1e-12f);
+                    const float kkx = rh(quot_(kx[q], nrm)), kky = rh(quot_(ky[q], nrm));
+                    *reinterpret_cast<float2*>(s.a + 2 * lane) = make_float2(-kkx, -kky);
+                    *reinterpret_cast<float2*>(s.b + 2 * lane) = make_float2(rh(kkx * ax[q]), rh(kky * ay[q]));
+                    if (lane == 0) s.rkr = rh(rkr[q]);
                 }
             }
             __syncwarp();
@@ -652,7 +681,7 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
         }
     } else {
         const int qw = warp - SC_SCAN - SC_PRE, gc = h * 64 + 2 * lane;
-        constexpr int PER = (SC_CH + SC_POST - 1) / SC_POST;
+        constexpr int PER = SC_CH / SC_POST;
         float2 lw, lb;
         if (!OP) { lw = ld2u(p.lnx_w + gc); lb = ld2u(p.lnx_b + gc); }
         for (int ch = 0; ch < n_chunks; ++ch) {
@@ -662,30 +691,50 @@ __global__ void __launch_bounds__(SC_THREADS, 2) scan_kernel(const __grid_consta
             if (!OP) {
 #pragma unroll
                 for (int q = 0; q < PER; ++q) {
-                    const int j = qw + q * SC_POST, t = ch * SC_CH + j;
-                    if (j < SC_CH && t < T) g[q] = ld2a(p.g + base + (size_t)t * p.D + 2 * lane);
+                    const int t = ch * SC_CH + qw + q * SC_POST;
+                    g[q] = t < T ? ld2a(p.g + base + (size_t)t * p.D + 2 * lane) : make_float2(0.f, 0.f);
                 }
             }
             wait_for(&done[buf], (uint32_t)(ch / SC_NBUF) & 1u);
+            // (rows of y beyond T hold what an earlier chunk left there, or nothing: computed with, never stored)
+            float2 y[PER];
+            float mean[PER], var[PER];
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                y[q] = *reinterpret_cast<const float2*>(&ck.y[qw + q * SC_POST][2 * lane]);
+                if (!OP) { y[q].x = rh(y[q].x); y[q].y = rh(y[q].y); }
+                mean[q] = y[q].x + y[q].y;
+            }
+            if (!OP) {   // group norm over the head's 64 channels (eps 64e-5), bonus, gate (reference/rwkv7.py:297-299)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int q = 0; q < PER; ++q) mean[q] += __shfl_xor_sync(0xffffffffu, mean[q], o);
+#pragma unroll
+                for (int q = 0; q < PER; ++q) {
+                    mean[q] *= 1.f / 64.f;
+                    y[q].x -= mean[q];
+                    y[q].y -= mean[q];
+                    var[q] = y[q].x * y[q].x + y[q].y * y[q].y;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int q = 0; q < PER; ++q) var[q] += __shfl_xor_sync(0xffffffffu, var[q], o);
+            }
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 const int j = qw + q * SC_POST, t = ch * SC_CH + j;
-                if (j >= SC_CH || t >= T) break;
-                const float2 y = *reinterpret_cast<const float2*>(&ck.y[j][2 * lane]);
                 __half2* out = reinterpret_cast<__half2*>(p.out + base + (size_t)t * p.D + 2 * lane);
-                if (!AB_BC(base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) continue;
+                if (t >= T || !AB_BC(base + (size_t)t * p.D + 2 * lane + 2 <= (size_t)p.B * T * p.D)) continue;
                 if (OP) {
-                    *out = __floats2half2_rn(y.x, y.y);
+                    *out = __floats2half2_rn(y[q].x, y[q].y);
                 } else {
-                    // group norm over the head's 64 channels (eps 64e-5), bonus, gate (reference/rwkv7.py:297-299)
-                    const float yx = rh(y.x), yy = rh(y.y);
-                    const float mean = warp_sum(yx + yy) * (1.f / 64.f);
-                    const float d0 = yx - mean, d1 = yy - mean;
-                    const float rstd = rsqrtf(warp_sum(d0 * d0 + d1 * d1) * (1.f / 64.f) + 64e-5f);
-                    const float rkr = ck.s[j].rkr;
+                    const float rstd = rsqrtf(var[q] * (1.f / 64.f) + 64e-5f);
+                    const float bonus = ck.s[j].rkr;
                     const float2 v = *reinterpret_cast<const float2*>(&ck.s[j].v[2 * lane]);
-                    const float o0 = rh(rh(d0 * rstd * lw.x + lb.x) + rh(rkr * v.x));
-                    const float o1 = rh(rh(d1 * rstd * lw.y + lb.y) + rh(rkr * v.y));
+                    const float o0 = rh(rh(y[q].x * rstd * lw.x + lb.x) + rh(bonus * v.x));
+                    const float o1 = rh(rh(y[q].y * rstd * lw.y + lb.y) + rh(bonus * v.y));
                     *out = __floats2half2_rn(o0 * g[q].x, o1 * g[q].y);
                 }
             }
@@ -699,15 +748,17 @@ int scan_launch(const HeadParams& p, bool op, cudaStream_t stream) {
     AB_CHECK_ARG(((uintptr_t)p.state & 15) == 0, "head: state must be 16-byte aligned");
     constexpr int smem = SC_NBUF * (int)sizeof(ScanChunk);
     static PerDeviceOnce once;
-    const int s = once.run(nullptr, [](DeviceProps&) -> int {
-        AB_CUDA(cudaFuncSetAttribute(scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        AB_CUDA(cudaFuncSetAttribute(scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const DeviceProps* dp = nullptr;
+    const int s = once.run(&dp, [](DeviceProps&) -> int {
+        for (auto k : {scan_kernel<false, false>, scan_kernel<false, true>, scan_kernel<true, false>, scan_kernel<true, true>})
+            AB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         return OK;
     });
     if (s != OK) return s;
+    const bool wide = p.B * p.H <= dp->n_sm;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(p.B * p.H));
-    cfg.blockDim = dim3(SC_THREADS);
+    cfg.blockDim = dim3(scan_threads(wide));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -715,8 +766,8 @@ int scan_launch(const HeadParams& p, bool op, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.use_pdl ? 1 : 0;
-    if (op) AB_CUDA(cudaLaunchKernelEx(&cfg, scan_kernel<true>, p));
-    else AB_CUDA(cudaLaunchKernelEx(&cfg, scan_kernel<false>, p));
+    AB_CUDA(cudaLaunchKernelEx(&cfg, op ? (wide ? scan_kernel<true, true> : scan_kernel<true, false>)
+                                        : (wide ? scan_kernel<false, true> : scan_kernel<false, false>), p));
     return OK;
 }
 
