@@ -6,3 +6,4 @@
 #include "gemv.cu"
 #include "head.cu"
 #include "rows.cu"
+#include "stream.cu"

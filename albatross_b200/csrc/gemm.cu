@@ -973,8 +973,21 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
         gs = launch_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
     }
     AB_CHECK_ARG(gs.part_floats == 0 || (scratch && ((uintptr_t)scratch & 15) == 0), "gemm: split-K needs a 16-byte aligned scratch area");
+    int st = OK;
+    for (int i = 0; i < n; ++i) {
+        const GemmOp& op = ops[i];
+        const ab_mat& m = op.w;
+        AB_CHECK_ARG(op.x && op.y, "gemm: null activation pointer");
+        AB_CHECK_ARG(op.epi >= EPI_NONE && op.epi <= EPI_RESID && (op.epi != EPI_RESID || op.resid), "gemm: bad epilogue");
+        AB_CHECK_ARG(m.col_scale == nullptr, "gemm: per-input-column scales are a batch-1 feature");
+        AB_CHECK_ARG(m.k % 16 == 0 && ((uintptr_t)op.x & 15) == 0 && ((uintptr_t)m.w & 15) == 0, "gemm: k %% 16 and 16-byte alignment needed");
+        AB_CHECK_ARG(m.fmt != FMT_FP4 || (m.k % 64 == 0 && ((uintptr_t)m.scale & 3) == 0), "gemm: NVFP4 needs k %% 64 == 0");
+    }
+    bool taken = false;
+    st = stream_group_launch(ops, n, rows, stream, pdl, &taken);
+    if (st != OK || taken) return st;
     EncodeTiledFn encode;
-    int st = get_encode_fn(&encode);
+    st = get_encode_fn(&encode);
     if (st != OK) return st;
 
     GemmGroup g = {};
@@ -990,13 +1003,6 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
     for (int i = 0; i < n; ++i) {
         const GemmOp& op = ops[i];
         const ab_mat& m = op.w;
-        st = check_mat(m, "gemm");
-        if (st != OK) return st;
-        AB_CHECK_ARG(op.x && op.y, "gemm: null activation pointer");
-        AB_CHECK_ARG(op.epi >= EPI_NONE && op.epi <= EPI_RESID && (op.epi != EPI_RESID || op.resid), "gemm: bad epilogue");
-        AB_CHECK_ARG(m.col_scale == nullptr, "gemm: per-input-column scales are a batch-1 feature");
-        AB_CHECK_ARG(m.k % 16 == 0 && ((uintptr_t)op.x & 15) == 0 && ((uintptr_t)m.w & 15) == 0, "gemm: k %% 16 and 16-byte alignment needed");
-        AB_CHECK_ARG(m.fmt != FMT_FP4 || (m.k % 64 == 0 && ((uintptr_t)m.scale & 3) == 0), "gemm: NVFP4 needs k %% 64 == 0");
         GemmProb& pb = g.pr[i];
         pb.w = m; pb.resid = op.resid; pb.y = op.y; pb.epi = op.epi;
         g.cta_base[i] = cta; pb.ksplit = gs.ksplit[i]; pb.tile_base = tile; pb.part_base = part;

@@ -33,6 +33,8 @@ size_t gemm_group_scratch_bytes(const GemmOp* ops, int n, int rows);
 // pdl: launch with programmatic stream serialisation (the kernel waits for the preceding grid itself, after it has
 // started its weight stream).
 int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t scratch_bytes, cudaStream_t stream, bool pdl = false);
+// The same for few rows (stream.cu): *taken tells whether it took the launch.
+int stream_group_launch(const GemmOp* ops, int n, int rows, cudaStream_t stream, bool pdl, bool* taken);
 size_t gemm_scratch_bytes(const ab_mat& m, int rows);
 int static_scratch_reset(cudaStream_t stream);   // built-in scratch of ab_gemm_static: counters back to zero
 int gemm_launch(const ab_mat& m, int rows, const __half* x, __half* y, int epi, const __half* resid, void* scratch,

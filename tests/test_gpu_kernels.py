@@ -401,3 +401,41 @@ def test_sequence_norm_and_lerps_through_a_model(B, T, D):
         assert rel_err(whole.view(B, T, 64).float().cpu(), parts.cpu()) < 2e-2
         for a, b in zip(st, pst):
             assert rel_err(a.float().cpu(), b.float().cpu()) < 2e-2
+
+
+@pytest.mark.parametrize("fmt", ["int8", "nvfp4", "none"])
+@pytest.mark.parametrize("rows,n,k", [(1, 64, 64), (7, 300, 192), (8, 4096, 320), (8, 129, 4096), (5, 4100, 448), (8, 1024, 16384), (9, 1000, 1024),
+                                      (16, 96, 4096), (13, 2560, 2560), (17, 768, 768), (24, 1000, 2048), (24, 31, 12288)])
+def test_products_of_few_rows(fmt, rows, n, k):
+    """The kernel for up to 24 rows at its edges: ragged weight tiles (32 rows) and row pieces (128 bytes: 64, 128 or 256
+    inputs), one to three groups of eight batch rows, K split over the blocks of a cluster, NVFP4 scales with and without a
+    tensor map (k a multiple of 256 or not), every epilogue; a second call gives the same bits. Bound: one fp16 rounding of the
+    product (2**-11), one more by the epilogue, and fp32 sums."""
+    from albatross_b200 import quant
+    torch.manual_seed(rows * 7 + n + k)
+    pm = quant.quantize((torch.randn(n, k) * 0.02).cuda(), None if fmt == "none" else fmt)
+    x, r = torch.randn(rows, k).half().cuda(), torch.randn(rows, n).half().cuda()
+    want = x.double() @ pm.dequantize().double().t()
+    fns = [lambda t: t, torch.tanh, torch.sigmoid, lambda t: torch.relu(t) ** 2, lambda t: t + r.double()]
+    for epi, fn in enumerate(fns):
+        got = _gemm(pm, x, epi, r if epi == 4 else None)
+        ref = fn(want)
+        assert rel_err(got.double().cpu(), ref.cpu()) < 2e-3, epi
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -10.5, epi
+        assert torch.equal(_gemm(pm, x, epi, r if epi == 4 else None), got)
+
+
+def test_products_of_few_rows_leave_their_neighbours_alone():
+    """Outputs beyond the last row and column stay as they were (ragged rows and columns are clipped, not written)."""
+    from albatross_b200 import _lib, quant
+    torch.manual_seed(3)
+    for rows, n, k in ((3, 70, 512), (9, 33, 256), (8, 4099, 128)):
+        pm = quant.quantize((torch.randn(n, k) * 0.02).cuda(), "int8")
+        mat, x = pm.as_mat(), torch.randn(rows, k).half().cuda()
+        buf = torch.full((rows * n + 64,), 7.0, dtype=torch.float16, device="cuda")
+        scratch = torch.zeros(max(256, _lib.lib.ab_gemm_scratch_bytes(C.byref(mat), rows)), dtype=torch.uint8, device="cuda")
+        _lib.check(_lib.lib.ab_gemm(C.byref(mat), rows, x.data_ptr(), buf.data_ptr(), 0, None, scratch.data_ptr(), _stream()), "ab_gemm")
+        torch.cuda.synchronize()
+        assert _lib.device_status() == 0
+        assert torch.equal(buf[rows * n:], torch.full_like(buf[rows * n:], 7.0))
+        assert rel_err(buf[:rows * n].view(rows, n).double().cpu(), (x.double() @ pm.dequantize().double().t()).cpu()) < 2e-3
