@@ -477,7 +477,7 @@ struct ScanChunk {
 };
 
 template <bool OP, bool WIDE>
-__global__ void __launch_bounds__(scan_threads(WIDE), WIDE ? 1 : 2) scan_kernel(const __grid_constant__ HeadParams p) {
+__device__ __forceinline__ void scan_block(const HeadParams& p) {
     constexpr int SC_PRE = scan_pre(WIDE), SC_POST = scan_post(WIDE);
     extern __shared__ __align__(128) unsigned char dsm[];   // SC_NBUF chunks
     __shared__ uint64_t full[SC_NBUF], done[SC_NBUF], vacant[SC_NBUF];
@@ -744,13 +744,18 @@ __global__ void __launch_bounds__(scan_threads(WIDE), WIDE ? 1 : 2) scan_kernel(
     }
 }
 
+template <bool OP>
+__global__ void __launch_bounds__(scan_threads(false), 2) scan_kernel(const __grid_constant__ HeadParams p) { scan_block<OP, false>(p); }
+template <bool OP>
+__global__ void __launch_bounds__(scan_threads(true), 1) scan_wide_kernel(const __grid_constant__ HeadParams p) { scan_block<OP, true>(p); }
+
 int scan_launch(const HeadParams& p, bool op, cudaStream_t stream) {
     AB_CHECK_ARG(((uintptr_t)p.state & 15) == 0, "head: state must be 16-byte aligned");
     constexpr int smem = SC_NBUF * (int)sizeof(ScanChunk);
     static PerDeviceOnce once;
     const DeviceProps* dp = nullptr;
     const int s = once.run(&dp, [](DeviceProps&) -> int {
-        for (auto k : {scan_kernel<false, false>, scan_kernel<false, true>, scan_kernel<true, false>, scan_kernel<true, true>})
+        for (auto k : {scan_kernel<false>, scan_kernel<true>, scan_wide_kernel<false>, scan_wide_kernel<true>})
             AB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         return OK;
     });
@@ -766,8 +771,7 @@ int scan_launch(const HeadParams& p, bool op, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.use_pdl ? 1 : 0;
-    AB_CUDA(cudaLaunchKernelEx(&cfg, op ? (wide ? scan_kernel<true, true> : scan_kernel<true, false>)
-                                        : (wide ? scan_kernel<false, true> : scan_kernel<false, false>), p));
+    AB_CUDA(cudaLaunchKernelEx(&cfg, op ? (wide ? scan_wide_kernel<true> : scan_kernel<true>) : (wide ? scan_wide_kernel<false> : scan_kernel<false>), p));
     return OK;
 }
 
