@@ -315,12 +315,16 @@ __device__ __forceinline__ float sample_noise(uint32_t seed, uint32_t row, uint3
 // maximum over the block is taken first, and only chunks that can still reach it are looked at value by value: noise is
 // never negative and always below `noise`, so a logit v ends up in [v, v + noise]. Skipped are chunks strictly below; ties
 // and NaNs take the long way, the result is the same id.
-// (With the maximum over a warp instead of the block, eight chunks per warp and batch still took the long way: 18.1 us, now 13.3.)
-// NT threads per row: 1024 when there are only a few rows, 256 otherwise (all rows of a batch of 320 are resident at once).
-constexpr int SR_U = 8;
+// (With the maximum over a warp instead of the block, eight chunks per warp and batch still took the long way: 18.1 us, then 13.3.)
+// NT threads per row: 1024 for up to 16 rows, whose rows are a batch of eight chunks per thread (8 rows of 65536: 4.5 us); more
+// threads than that do not share an SM, so further rows take 512 threads as long as every row has an SM to itself and 256
+// beyond, in batches of four chunks of which the next travels while one is looked at (100 rows of 65536 8.9 -> 6.1 us, 200 of
+// 50277 9.5 -> 8.0, 320 of 65536 11.0 -> 10.5, in a graph).
 template <class OutT, int NT>
 __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restrict__ logits, int V, float noise, uint32_t seed,
                                                          OutT* __restrict__ out) {
+    constexpr bool AHEAD = NT < 1024;
+    constexpr int SR_U = AHEAD ? 4 : 8;
     __shared__ float bv[NT / 32], tops[2][NT / 32];
     __shared__ int bi[NT / 32];
     const size_t row = blockIdx.x;
@@ -336,14 +340,22 @@ __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restric
     if ((int)threadIdx.x < head && AB_BC((int)threadIdx.x < V)) take(__half2float(lr[threadIdx.x]), threadIdx.x);
     const uint4* body = reinterpret_cast<const uint4*>(lr + head);
     int buf = 0;
-    for (int c0 = 0; c0 < nv; c0 += NT * SR_U, buf ^= 1) {   // uniform in the block
-        uint4 q[SR_U];
-        __half m[SR_U];
+    uint4 nxt[SR_U];
+    auto request = [&](int c0) {
 #pragma unroll
         for (int u = 0; u < SR_U; ++u) {
             const int c = c0 + u * NT + threadIdx.x;
-            if (c < nv && AB_BC(c >= 0 && head + 8 * (c + 1) <= V)) q[u] = __ldcs(body + c);
+            if (c < nv && AB_BC(c >= 0 && head + 8 * (c + 1) <= V)) nxt[u] = __ldcs(body + c);
         }
+    };
+    if (AHEAD) request(0);
+    for (int c0 = 0; c0 < nv; c0 += NT * SR_U, buf ^= 1) {   // uniform in the block
+        uint4 q[SR_U];
+        __half m[SR_U];
+        if (!AHEAD) request(c0);
+#pragma unroll
+        for (int u = 0; u < SR_U; ++u) q[u] = nxt[u];
+        if (AHEAD) request(c0 + NT * SR_U);   // the next batch travels while this one is looked at
         __half top = __ushort_as_half((unsigned short)0xfc00u);   // -inf
 #pragma unroll
         for (int u = 0; u < SR_U; ++u) {
@@ -440,6 +452,9 @@ int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t see
     if (rows <= 16) {
         if (out_i64) sample_rows_kernel<long long, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (long long*)out);
         else sample_rows_kernel<int, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (int*)out);
+    } else if (rows <= 148) {
+        if (out_i64) sample_rows_kernel<long long, 512><<<rows, 512, 0, s>>>(logits, V, noise, seed, (long long*)out);
+        else sample_rows_kernel<int, 512><<<rows, 512, 0, s>>>(logits, V, noise, seed, (int*)out);
     } else {
         if (out_i64) sample_rows_kernel<long long, 256><<<rows, 256, 0, s>>>(logits, V, noise, seed, (long long*)out);
         else sample_rows_kernel<int, 256><<<rows, 256, 0, s>>>(logits, V, noise, seed, (int*)out);

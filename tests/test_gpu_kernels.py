@@ -439,3 +439,19 @@ def test_products_of_few_rows_leave_their_neighbours_alone():
         assert _lib.device_status() == 0
         assert torch.equal(buf[rows * n:], torch.full_like(buf[rows * n:], 7.0))
         assert rel_err(buf[:rows * n].view(rows, n).double().cpu(), (x.double() @ pm.dequantize().double().t()).cpu()) < 2e-3
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 148, 149])
+@pytest.mark.parametrize("V", [1, 9, 8191, 8200, 16384, 16393, 32777])
+def test_sampler_at_the_edges_of_its_batches(rows, V):
+    """Row lengths around a batch of each kernel (16 K logits of 512 threads, 8 K of 256, 64 K of 1024), rows that start off a
+    16-byte boundary, and the row counts where the kernel changes. Whole numbers: the same ids as torch."""
+    from albatross_b200 import sampler_simple_batch
+    g = torch.Generator().manual_seed(rows + V)
+    logits = (torch.randn(rows, V, generator=g) * 3).half()
+    logits[:, V // 3] = logits.max() + 1                     # a winner whose position is known ...
+    logits[rows // 2, V - 1] = logits.max() + 1              # ... and one in the last place
+    dev = logits.cuda()
+    assert torch.equal(sampler_simple_batch(dev, noise=0.0).flatten().cpu(), logits.float().argmax(1))
+    a = sampler_simple_batch(dev, noise=0.5, seed=3).flatten().cpu()     # noise below the winner's margin of 1
+    assert torch.equal(a, logits.float().argmax(1))
