@@ -388,6 +388,12 @@ class RWKV_x070:
             ev = self._tok_events[slot] = torch.cuda.Event()
         ev.record()
 
+    def _send_ids(self, ids: torch.Tensor) -> torch.Tensor:
+        """A prompt's ids on the device, sent from page-locked memory: a copy from ordinary memory would wait for the stream
+        to drain, and the launches of this call would start behind the last one of the call before. (torch's allocator
+        hands a page-locked block out again when the copies that read it have completed.)"""
+        return ids.pin_memory().to(self.device, non_blocking=True)
+
     def _hand_back(self, state: List[torch.Tensor], batch: Optional[int]):
         """The caller's next state: the same tensors (updated in place) in a list that remembers this model's checks."""
         return _State(state, (self, batch, self._state_key(state)))
@@ -475,7 +481,7 @@ class RWKV_x070:
         self._check_state(state, None)
         T = len(idx)
         self._check_ids(idx)
-        tok = torch.tensor([self._wrap_id(t) for t in idx], dtype=torch.int32, device=self.device)
+        tok = self._send_ids(torch.tensor([self._wrap_id(t) for t in idx], dtype=torch.int32))
         logits = torch.empty((T, self.vocab) if full_output else (self.vocab,), dtype=DTYPE, device=self.device)
         self._run(1, T, tok, state, logits, full_output)
         return logits, self._hand_back(state, None)
@@ -491,7 +497,7 @@ class RWKV_x070:
         tok = torch.where(tok < 0, tok + self.vocab, tok).to(torch.int32)
         if T == 1 and B > 1 and self.use_graph:
             return self._forward_batch_graph(B, tok, state)
-        tok = tok.to(self.device)
+        tok = self._send_ids(tok)
         shape = (B, T, self.vocab) if full_output else (B, self.vocab)
         logits = torch.empty(shape, dtype=DTYPE, device=self.device)
         self._run(B, T, tok, state, logits, full_output)
