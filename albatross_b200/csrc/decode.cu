@@ -73,17 +73,17 @@ __device__ __forceinline__ void stage_phase(DecodePhase* dst, const DecodePhase*
 
 // The per-head phase of one network block. Its own function (not inlined) so that the register allocation of the
 // matrix-vector phases, which run at the kernel's register cap, does not have to make room for it.
-__device__ __noinline__ void head_phase(const HeadParams& hp, int bid, int nb, int tid, unsigned char* smem, unsigned char* pref,
+__device__ __noinline__ void head_phase(const HeadParams& hp, int my_head, int bid, int nb, int tid, unsigned char* smem, unsigned char* pref,
                                         const __half* xn, HeadShared& hsh, uint32_t epoch, unsigned long long* htl) {
     // adapter up-projections inside the phase: block h needs only the 64 channels of head h, so the
     // matrix-vector phase (and the grid barrier) that would produce them for everybody is not needed
     const bool ups = hp.w2 != nullptr;
-    // Dataflow mode (pair_mode): no barrier among all blocks came before this phase. Block 2h runs head h; its
+    // Dataflow mode (pair_mode): no barrier among all blocks came before this phase. Block P h runs head h; its
     // inputs (the head's r / k / v rows, the adapter hidden vectors) are tagged words and the loads wait for
     // them one by one. Everybody else goes straight on to the next phase.
     const bool pair = hp.pair_mode != 0;
-    const bool mine = !pair || (bid < 2 * hp.H && (bid & 1) == 0);
-    for (int h = pair ? (bid >> 1) : bid; mine && h < hp.H; h += pair ? hp.H : nb) {   // block-uniform
+    const bool mine = !pair || my_head > 0;
+    for (int h = pair ? my_head - 1 : bid; mine && h < hp.H; h += pair ? hp.H : nb) {   // block-uniform
         if (tid < HT) {
             unsigned char* dsm = pair ? pref : smem;   // pair mode: staged during the phase before
             if (ups && !pair) head_ups_stage(hp, h, tid, dsm);   // the matrix-vector buffers are idle in this phase
@@ -167,14 +167,15 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
                          // the first-slice prefetch uses the area that the phase before a paired head phase stages into
                          (i + 1 < n_phases && phs[(i + 1) & 3].type == PHASE_HEAD && phs[(i + 1) & 3].h.pair_mode) ? 0 : prog->early_slice,
                          [&]() {
-                             if (ph.no_barrier == 2 && tid < HT && bid < 2 * phs[(i + 1) & 3].h.H && (bid & 1) == 0) {
-                                 // "fused heads": this block runs head bid / 2 right after the phase. Its slices of the
+                             const int my_head = plans[(i + 1) & 3].head;   // (0 unless the next phase is a head phase in dataflow mode)
+                             if (tid < HT && my_head > 0) {
+                                 // "fused heads": this block runs a head right after the phase. Its slices of the
                                  // four adapter up-projection matrices (weights: no dependency) move into the idle
                                  // prefetch area while the phase's own weights stream; requested any earlier they would
                                  // sit in front of the loads of the phase's input vector. The head's per-channel
                                  // parameters and its state (last touched a token ago) are pulled towards the SM as well.
                                  const HeadParams& nh = phs[(i + 1) & 3].h;
-                                 const int h = bid >> 1;
+                                 const int h = my_head - 1;
                                  head_ups_stage(nh, h, tid, m.pref);
                                  head_par_stage(nh, h, tid, m.pref);
                                  asm volatile("cp.async.commit_group;" ::: "memory");
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
             // sit in front of the loads that wait for the inputs).
             if (tid == 32 && j >= 0 && prog->l2_prefetch_bytes > 0) prefetch_share(phs[j & 3].g, plans[j & 3], 0, prog->l2_prefetch_bytes);
         } else {
-            head_phase(ph.h, bid, nb, tid, smem, m.pref, m.xn, hsh, epoch,
+            head_phase(ph.h, plans[i & 3].head, bid, nb, tid, smem, m.pref, m.xn, hsh, epoch,
                        (tid == 0 && tl_base()) ? tl_base() + 2 * n_phases + 4 * i : nullptr);
         }
         if (tid == 0 && tl_base()) tl_base()[2 * i + 1] = global_ns();

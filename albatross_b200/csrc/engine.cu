@@ -81,10 +81,10 @@ struct ab_model {
                            // while the block waits for its input anyway; with barriers it delays the input loads and is slower)
     int barrier_prefetch = 0;   // measured slower: the polls of the barrier queue behind the prefetch traffic
     int stage_gemv = 0;  // ab_forward_stage at B = T = 1 runs the batch-1 matrix-vector kernels instead of the row-wise program
-    int fuse_heads = 1;  // persistent decode kernel: r/k/v rows of head h on blocks 2h, 2h+1, the adapter down-projections on
-                         // the remaining blocks; block 2h runs the head (up-projections from pre-staged weights, WKV step)
+    int fuse_heads = 1;  // persistent decode kernel: r/k/v rows of head h on P blocks (two or more) from P h on, the adapter down-projections on
+                         // the remaining blocks; block P h runs the head (up-projections from pre-staged weights, WKV step)
                          // as soon as those producers have signalled: two barriers among all blocks fewer per network block
-    int pair_split = 16; // ... row groups (of 4 rows) of a head's 48 (r, k, v) that go to block 2h (which also stages the up-projections)
+    int pair_split = 16; // ... row groups (of 4 rows) of a head's 48 (r, k, v) that go to its first block (which also stages the up-projections) of two, in proportion of more
     int merge_ups = 0;   // persistent decode kernel: block h computes the adapter up-projections of head h inside the head
                          // phase: one phase and barrier fewer per block and the same arithmetic as the per-phase
                          // launches (identical logits), but 3 % slower per token than the phase of matrix-vector rows
@@ -331,7 +331,7 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
         if (fused) {
             DecodePhase& p1 = prog->phases[n - 1];
             p1.no_barrier = 2;         // dataflow: tagged outputs, no barrier among all blocks
-            p1.rows_per_block = -1;    // marks the head-aligned plan
+            p1.rows_per_block = -blocks_per_head(p1.g, m->n_sm, H);   // marks the head-aligned plan
             // layer 0 reads the embedding row (weights) and block 0 publishes it as the tagged hidden state
             p1.g.tag_in = i == 0 ? n : x_tag;
             if (i == 0) x_tag = n;
@@ -365,7 +365,7 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
             h.lnx_w = (const __half*)Ly.lnx_w; h.lnx_b = (const __half*)Ly.lnx_b;
             h.out = ws.att; h.copy_src = ws.xn; h.copy_dst = att_prev;
             if (fused) {
-                h.pair_mode = 1; h.tag_in = n - 1; h.tag_out = n;   // n - 1: the phase before (1-based), n: this one
+                h.pair_mode = -prog->phases[n - 2].rows_per_block; h.tag_in = n - 1; h.tag_out = n;   // n - 1: the phase before (1-based), n: this one
                 ph.no_barrier = 2;
             }
             if (ups_in_head) {   // block h computes the adapter outputs of head h itself (no phase, no barrier for them)
@@ -418,11 +418,17 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
     m->prog_xq_bytes = prog->xq_bytes;
     BlockPlan* host_plans = reinterpret_cast<BlockPlan*>(buf.data() + plans_off);
     for (int i = 0; i < n; ++i)
-        if (prog->phases[i].type == PHASE_GEMV)
+        if (prog->phases[i].type == PHASE_HEAD) {
+            const int P = prog->phases[i].h.pair_mode;
+            for (int hd = 0; P > 0 && hd < H; ++hd) host_plans[(size_t)i * m->n_sm + hd * P].head = hd + 1;
+        } else if (prog->phases[i].type == PHASE_GEMV)
             for (int b = 0; b < m->n_sm; ++b) {
                 BlockPlan& bp = host_plans[(size_t)i * m->n_sm + b];
                 if (prog->phases[i].rows_per_block > 0) compute_plan_rows(prog->phases[i].g, b, prog->phases[i].rows_per_block, bp);
-                else if (prog->phases[i].rows_per_block < 0) compute_plan_heads(prog->phases[i].g, b, m->n_sm, H, m->pair_split, bp);
+                else if (prog->phases[i].rows_per_block < 0) {
+                    const int P = -prog->phases[i].rows_per_block;
+                    compute_plan_heads(prog->phases[i].g, b, m->n_sm, H, P, first_block_groups(P, m->pair_split), bp);
+                }
                 else compute_plan(prog->phases[i].g, b, m->n_sm, bp);
             }
     return OK;

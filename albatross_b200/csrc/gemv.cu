@@ -184,6 +184,29 @@ extern "C" int ab_gemv_plan_selftest(const int32_t* fmt, const int32_t* n_rows, 
     for (int s = 0; s < nseg; ++s)
         AB_CHECK_ARG(next[s] == gemv_groups_of(n_rows[s]), "plan selftest: segment %d covered up to group %d of %d", s, next[s],
                      gemv_groups_of(n_rows[s]));
+    // The head-aligned plan of the persistent kernel, where the launch has its form: r, k, v of whole heads, then adapters.
+    const int H = n_rows[0] / HEAD;
+    if (nseg >= 4 && n_rows[0] % HEAD == 0 && n_rows[1] == n_rows[0] && n_rows[2] == n_rows[0] && 2 * H + 4 <= n_blocks) {
+        const int P = blocks_per_head(p, n_blocks, H), gph = HEAD / GEMV_ROWS;
+        AB_CHECK_ARG(P >= 2 && P * H + 4 <= n_blocks, "plan selftest: %d blocks per head", P);
+        for (int split : {1, gph, 3 * gph - 1}) {
+            std::vector<std::vector<int>> seen(nseg);
+            for (int s = 0; s < nseg; ++s) seen[s].assign(gemv_groups_of(n_rows[s]), 0);
+            for (int b = 0; b < n_blocks; ++b) {
+                BlockPlan bp = {};
+                compute_plan_heads(p, b, n_blocks, H, P, first_block_groups(P, split), bp);
+                AB_CHECK_ARG(bp.n_rows <= GEMV_MAX_ROWS_PER_BLOCK, "plan selftest: %d rows in block %d", bp.n_rows, b);
+                for (int s = 0; s < nseg; ++s)
+                    for (int g = bp.sp[s].lo; g < bp.sp[s].lo + bp.sp[s].n_groups; ++g) {
+                        AB_CHECK_ARG(g >= 0 && g < (int)seen[s].size() && (s >= 3 ? b >= P * H : b / P == g / gph && b < P * H),
+                                     "plan selftest: block %d has group %d of segment %d (%d blocks per head)", b, g, s, P);
+                        ++seen[s][g];
+                    }
+            }
+            for (int s = 0; s < nseg; ++s)
+                for (int c : seen[s]) AB_CHECK_ARG(c == 1, "plan selftest: a group of segment %d is in %d blocks (%d per head, split %d)", s, c, P, split);
+        }
+    }
     if (max_items) *max_items = items_max;
     if (max_cost_spread_pct) {
         const double mean = (double)total_cost / n_blocks;

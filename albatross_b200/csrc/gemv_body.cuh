@@ -189,6 +189,7 @@ struct SegPlan {
 struct __align__(16) BlockPlan {
     SegPlan sp[GEMV_MAX_SEG];
     int n_items, n_rows, nseg, valid;
+    int head;   // persistent kernel, the plan of a head phase in dataflow mode: 1 + the head this block runs (0: none)
 };
 
 // 32-bit arithmetic on purpose (one thread computes this while the others run the prologue): costs are at
@@ -270,11 +271,31 @@ __host__ __device__ inline void compute_plan_rows(const GemvParams& p, int bid, 
     bp.valid = 1;
 }
 
-// Plan of the r/k/v + adapter phase of the persistent kernel in dataflow mode. Segments 0..2 are the r, k, v matrices,
-// the rest the adapter down-projections. Blocks 2h and 2h + 1 compute the 64 rows of head h of each of r, k, v (48 row
-// groups in the order r, k, v: the first `split` go to block 2h, which also runs the head afterwards and holds its
-// up-projection weights, the others to block 2h + 1); blocks 2H .. nb - 1 share the adapter rows by cost.
-__host__ inline void compute_plan_heads(const GemvParams& p, int bid, int nb, int H, int split, BlockPlan& bp) {
+// Blocks per head of the r/k/v + adapter phase of the persistent kernel in dataflow mode (segments 0..2 are the r, k, v
+// matrices, the rest the adapter down-projections): as many as leave the adapters their share of the work. With two for every
+// head a model of 12 heads streamed r, k and v with 24 of 148 blocks (0.1B int8 381 -> 370 us a token; four blocks, 2560 wide, fp16
+// 298 -> 278); 64 heads get two.
+__host__ inline int blocks_per_head(const GemvParams& p, int nb, int H) {
+    long long heads = 0, all = 0;
+    for (int s = 0; s < p.nseg; ++s) {
+        const long long c = (long long)gemv_groups_of(p.seg[s].n_rows) * gemv_group_cost(p.seg[s].fmt, p.seg[s].K);
+        all += c;
+        if (s < 3) heads += c;
+    }
+    const int most = 3 * (HEAD / GEMV_ROWS);   // a row group each
+    int n = (int)(nb * heads / (all * H));
+    if (n > (nb - 4) / H) n = (nb - 4) / H;
+    return n < 2 ? 2 : (n > most ? most : n);
+}
+// Row groups of a head's 48 that its first block takes, of `split` when there are two: that block stages the head's
+// up-projections meanwhile, so it gets half of what the others do.
+__host__ inline int first_block_groups(int blocks, int split) {
+    return blocks == 2 ? split : (3 * split) / (2 * blocks - 1);
+}
+// The plan of that phase. Blocks P h .. P h + P - 1 compute the 64 rows of head h of each of r, k, v (48 row groups in the order
+// r, k, v: the first `split` go to the first of them, which also runs the head afterwards and holds its up-projection
+// weights, the others share the rest evenly); blocks P H .. nb - 1 share the adapter rows by cost.
+__host__ inline void compute_plan_heads(const GemvParams& p, int bid, int nb, int H, int P, int split, BlockPlan& bp) {
     int items = 0, rows = 0, part = 0, xq = 0;
     auto fill = [&](int s, int lo, int n_groups) {
         const GemvSeg& sg = p.seg[s];
@@ -298,11 +319,10 @@ __host__ inline void compute_plan_heads(const GemvParams& p, int bid, int nb, in
         if (q.n_groups > 0) xq += gemv_xq_bytes(sg.K);
     };
     const int gph = HEAD / GEMV_ROWS;   // row groups per head and matrix
-    if (bid < 2 * H) {
-        // the head's 3 * gph row groups in the order r, k, v: block 2h takes the first `split`, block 2h + 1 the rest, so
-        // that each of them prepares the inputs of two matrices at most
-        const int h = bid >> 1, odd = bid & 1;
-        const int g0 = odd ? split : 0, g1 = odd ? 3 * gph : split;
+    if (bid < P * H) {
+        // the head's 3 * gph row groups in the order r, k, v, so that few blocks prepare the inputs of more than one matrix
+        const int h = bid / P, j = bid - h * P, rest = 3 * gph - split;
+        const int g0 = j ? split + rest * (j - 1) / (P - 1) : 0, g1 = split + rest * j / (P - 1);
         for (int s = 0; s < p.nseg; ++s) {
             int lo = 0, n = 0;
             if (s < 3) {
@@ -312,7 +332,7 @@ __host__ inline void compute_plan_heads(const GemvParams& p, int bid, int nb, in
             fill(s, lo, n);
         }
     } else {
-        const int b = bid - 2 * H, nd = nb - 2 * H;
+        const int b = bid - P * H, nd = nb - P * H;
         unsigned total = 0;
         for (int s = 3; s < p.nseg; ++s)
             total += (unsigned)gemv_groups_of(p.seg[s].n_rows) * (unsigned)gemv_group_cost(p.seg[s].fmt, p.seg[s].K);
@@ -377,7 +397,7 @@ __device__ __forceinline__ Item make_item(const GemvParams& p, const BlockPlan& 
     const SegPlan& q = bp.sp[s];
     const GemvSeg& sg = p.seg[s];
     const int it = i - q.item_base;
-    const int gl = it / q.npc, sl = it - gl * q.npc;
+    const int gl = q.npc == 1 ? it : it / q.npc, sl = it - gl * q.npc;
     const int row0 = (q.lo + gl) * GEMV_ROWS;
     Item t;
     t.row_bytes = q.row_bytes;
@@ -391,6 +411,9 @@ __device__ __forceinline__ Item make_item(const GemvParams& p, const BlockPlan& 
     return t;
 }
 
+// Sweep u of a slice lies beyond the row: the whole warp skips it (a row of 768 bytes has two sweeps of a slice's four:
+// 0.1B int8 370 -> 365 us a token).
+__device__ __forceinline__ bool sweep_beyond(const Item& t, int slice, int u) { return t.sb + slice * GEMV_SLICE_BYTES + u * 512 >= t.row_bytes; }
 // Issue the 16 (+ scale) loads of slice `slice` of an item; nothing waits for them here.
 // FULL: all four rows exist and the slice lies inside the row, so no load is predicated.
 template <bool FULL>
@@ -427,6 +450,7 @@ __device__ __forceinline__ void load_item(const Item& t, int slice, int lane, It
 __device__ __forceinline__ void prefetch_item(const Item& t, int lane, unsigned char* slot) {
 #pragma unroll
     for (int u = 0; u < GEMV_SWEEPS; ++u) {
+        if (sweep_beyond(t, 0, u)) break;
         const int o = t.sb + u * 512 + lane * 16;
 #pragma unroll
         for (int r = 0; r < GEMV_ROWS; ++r) {
@@ -471,6 +495,7 @@ __device__ __forceinline__ void compute_item(const Item& t, int slice, const Ite
                                              const float* sx, int lane, float* acc) {
 #pragma unroll
     for (int u = 0; u < GEMV_SWEEPS; ++u) {
+        if (!FULL && sweep_beyond(t, slice, u)) break;
         const int o = t.sb + slice * GEMV_SLICE_BYTES + u * 512 + lane * 16;
         if (FULL || o < t.row_bytes) {
             if (FMT == FMT_I8) {

@@ -19,6 +19,16 @@ def _check(fmt, rows, k, n_blocks):
     return items.value, spread.value
 
 
+@pytest.mark.parametrize("D", [64, 128, 256, 768, 1024, 2048, 2560, 4096])
+@pytest.mark.parametrize("big", [F16, I8, FP4])
+@pytest.mark.parametrize("n_blocks", [148, 132, 80])
+def test_head_aligned_plan_covers_every_row_once(D, big, n_blocks):
+    """r, k, v and the adapters over two or more blocks per head: the library's self-check goes over that plan as well when a
+    launch has this form and the blocks suffice (with the fewest, the default and the most row groups on a head's first block)."""
+    for ranks in ((64, 64, 32, 128), (4, 4, 4), (128, 128, 96, 480)):
+        _check([big] * 3 + [F16] * len(ranks), [D] * 3 + list(ranks), [D] * (3 + len(ranks)), n_blocks)
+
+
 @pytest.mark.parametrize("cfg", ["tiny", "0.1b", "7.2b"])
 @pytest.mark.parametrize("big", [I8, FP4])
 def test_every_phase_of_the_decode_program_is_covered(cfg, big):
