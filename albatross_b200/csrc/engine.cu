@@ -491,7 +491,8 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
     Workspace ws = ws_in;
     if (io && io->v_first) ws.vfirst = io->v_first;
     if (io && io->x_in) AB_CUDA(cudaMemcpyAsync(ws.x, io->x_in, (size_t)M * D * 2, cudaMemcpyDeviceToDevice, st));
-    else AB_TRY(gather_rows((const __half*)m->d.emb, tokens, M, D, m->d.vocab, ws.x, st));
+    // (the embedding rows are read by the first block's norm, or gathered in a pass of their own where that takes the general path)
+    bool rows_from_ids = !(io && io->x_in);
     const int g0 = m->layer_offset;   // index of this model's first block in the whole network
     for (int li = 0; li < m->d.n_layer; ++li) {
         const int i = li;
@@ -502,8 +503,18 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         mp.xn = ws.xn; mp.x_prev = (__half*)state[3 * i]; mp.B = B; mp.T = T; mp.D = D; mp.n_mix = 6;
         const void* mv[6] = {L.x_r, L.x_k, L.x_v, L.x_w, L.x_a, L.x_g};
         for (int j = 0; j < 6; ++j) { mp.mix[j] = (const __half*)mv[j]; mp.out[j] = ws.mix[j]; }
-        if (ln_mix_rows_ok((const __half*)L.ln1_w, (const __half*)L.ln1_b, mp)) {
-            AB_TRY(ln_mix_rows(ws.x, (const __half*)L.ln1_w, (const __half*)L.ln1_b, mp, st, m->use_pdl));
+        const bool fused = ln_mix_rows_ok((const __half*)L.ln1_w, (const __half*)L.ln1_b, mp);
+        const bool first = rows_from_ids;   // nothing of this pass runs yet that the launch could overlap with
+        if (rows_from_ids) {
+            rows_from_ids = false;
+            if (fused && ((uintptr_t)m->d.emb & 15) == 0) {
+                mp.table = (const __half*)m->d.emb; mp.ids = tokens; mp.vocab = m->d.vocab; mp.x_copy = ws.x;
+            } else {
+                AB_TRY(gather_rows((const __half*)m->d.emb, tokens, M, D, m->d.vocab, ws.x, st));
+            }
+        }
+        if (fused) {
+            AB_TRY(ln_mix_rows(ws.x, (const __half*)L.ln1_w, (const __half*)L.ln1_b, mp, st, m->use_pdl && !first));
         } else {
             AB_TRY(ln_rows(ws.x, (const __half*)L.ln1_w, (const __half*)L.ln1_b, M, D, 1, 0, ws.xn, st));
             AB_TRY(mix_rows(mp, st));
@@ -548,10 +559,10 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         return OK;
     }
     if (full_output || T == 1) {
-        AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, M, D, 1, 0, ws.xn, st));
+        AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, M, D, 1, 0, ws.xn, st, m->use_pdl));
         return gemm_launch(m->d.head, M, ws.xn, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl, &m->head_maps);
     }
-    AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, B, D, T, T - 1, ws.xlast, st));
+    AB_TRY(ln_rows(ws.x, (const __half*)m->d.lnout_w, (const __half*)m->d.lnout_b, B, D, T, T - 1, ws.xlast, st, m->use_pdl));
     return gemm_launch(m->d.head, B, ws.xlast, logits, EPI_NONE, nullptr, ws.gemm_scratch, ws.gemm_scratch_bytes, st, m->use_pdl, &m->head_maps);
 }
 

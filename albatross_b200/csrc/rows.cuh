@@ -10,11 +10,16 @@ struct MixParams {
     const __half* mix[6]; // lerp vectors [D]
     __half* out[6];       // [B*T, D] each
     int n_mix, B, T, D;
+    // first layer: the rows are those of `table` (vocab rows) that the ids name (null: x); their copy goes to x_copy
+    const __half* table;
+    const int* ids;
+    __half* x_copy;
+    int vocab;
 };
 
 int gather_rows(const __half* table, const int* idx, int rows, int D, int vocab, __half* out, cudaStream_t s);
 int ln_rows(const __half* x, const __half* w, const __half* b, int rows, int D, int stride, int offset, __half* out,
-            cudaStream_t s);
+            cudaStream_t s, bool pdl = false);
 int mix_rows(const MixParams& p, cudaStream_t s);
 int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t seed, void* out, bool out_i64, cudaStream_t s);
 // Layer norm of x (weights w, b) fused with the lerps (p.xn is not used). It works on 16 bytes at a time: for other row lengths

@@ -444,3 +444,22 @@ def test_glue_at_the_ends_of_its_range(B, T):
         assert torch.isfinite(got).all() and rel_err(got.float().cpu().numpy().reshape(want.shape), want.numpy()) <= LOGIT_REL_TOL
     for i in range(args.n_layer):
         assert rel_err(st[3 * i + 1].cpu().numpy().reshape(ref[3 * i + 1].shape), ref[3 * i + 1].numpy()) <= LOGIT_REL_TOL
+
+
+@pytest.mark.parametrize("B,T", [(2, 1), (260, 1), (1, 2), (3, 9), (2, 300), (5, 500)])
+def test_first_norm_reads_the_embedding_rows(B, T):
+    """The first block's norm takes its rows straight from the embedding table: the same bits as when the rows are handed over as
+    a stage's input, for single steps and for sequences over several rows per block (1, 2 and 4), an id beyond the table (clamped and
+    reported) among them."""
+    from albatross_b200 import _lib
+    model, args = model_for("tiny", "int8")
+    toks = torch.tensor(seeded_tokens(args.vocab_size, B * T, seed=B + T), dtype=torch.int32, device="cuda")
+    toks[-1] = args.vocab_size + 3
+    rows = model.z["emb.weight"][toks.long().clamp(max=args.vocab_size - 1)].contiguous()
+    outs = []
+    for kw in ({"tokens": toks}, {"x_in": rows}):
+        st = model.new_state(B)
+        vf = torch.zeros(B * T, args.n_embd, dtype=torch.float16, device="cuda")
+        outs.append([_run_stage(model, B, T, st, vf, **kw), vf] + list(st))
+        assert _lib.device_status() == (8 if "tokens" in kw else 0)
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
