@@ -172,6 +172,8 @@ extern "C" int ab_gemv_plan_selftest(const int32_t* fmt, const int32_t* n_rows, 
             if (q.n_groups > 0) next[s] = q.lo + q.n_groups;
             AB_CHECK_ARG(q.npc * q.chunk == q.nks && q.item_base == items && q.row_base == rows,
                          "plan selftest: inconsistent item layout (block %d segment %d)", b, s);
+            for (int it = 0; it < q.n_items; ++it)
+                AB_CHECK_ARG(group_of_item(it, q.npc_inv) == it / q.npc, "plan selftest: item %d of %d per group", it, q.npc);
             items += q.n_groups * q.npc;
             rows += q.n_groups * GEMV_ROWS;
             cost += (long long)q.n_groups * gemv_group_cost(fmt[s], k[s]);
