@@ -33,7 +33,8 @@
 // copy bandwidth: 350). Around the main loop a block spends 1 us before it (tensor memory, barriers, first rows on their
 // way) and 1 - 3 us behind it; the exchange of a split K costs 5 us.
 // 16384 x 4096, back to back: 320 rows nvfp4 41.2 -> 35.4 us (1214 TFLOP/s), 64 rows nvfp4 32.0 -> 17.9, 8 rows int8 32.6 ->
-// 19.7, against the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below).
+// 19.7, against the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below). Launches of
+// few rows, which none of this hides, go to stream.cu.
 #include <cuda.h>
 
 #include <algorithm>
@@ -886,8 +887,8 @@ GroupShape group_shape(const GemmOp* ops, int n, int rows, int n_sm, int tall_ti
         } else if (base_ctas < n_sm && slow_ctas > 0 && ops[i].w.fmt == FMT_F16 && ksteps >= 32) {
             // A nearly full grid whose fp16 products move two to four times the bytes per k-step of the quantised ones: they
             // would finish last, and the idle SMs take slices of their K loops. A step of two blocks, 4096 wide, with and
-            // without (us): int8 8 rows 242, 248; 100 rows 324, 333; 320 rows 621, 644; nvfp4 8 rows 228, 227; 64 rows
-            // 281, 285; 320 rows 603, 620; all fp16 up to 160 rows alike, 320 rows 664, 676.
+            // without (us): int8 100 rows 324, 333; 320 rows 621, 644; nvfp4 64 rows 281, 285; 320 rows 603, 620; all fp16 up to
+            // 160 rows alike, 320 rows 664, 676.
             ks = 1 + (n_sm - base_ctas) / slow_ctas;
             if (ks > 8) ks = 8;
             if (ks > ksteps / 8) ks = ksteps / 8;

@@ -199,7 +199,7 @@ int ab_decode_run(ab_model* m, void* program, void* stream);
  *                         of matrix-vector rows of their own (bit-identical to ab_forward at B = T = 1, 3 % slower;
  *                         switches "smem_prefetch" and "barrier_prefetch" off)
  *   "fuse_heads" (1)      persistent kernel in dataflow mode: no barrier among all blocks; the vectors that cross
- *                         blocks are tagged words their readers wait for, and block 2h runs head h right after its
+ *                         blocks are tagged words their readers wait for, and the first block of a head runs it after its
  *                         share of the r/k/v rows (needs 2 * heads + 4 blocks; else the barrier mode is used)
  *   "pair_split" (16)     dataflow mode: how many of a head's 48 r/k/v row groups its first block takes (of two; in proportion of more)
  *   "early_slice" (-1)    first weight slice of every warp requested into shared memory ahead of the phase's input
