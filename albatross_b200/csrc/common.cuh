@@ -174,6 +174,16 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
     return p;
 }
 
+// Before a stage of shared memory is handed back to a copy engine (bulk or tensor copies write through the asynchronous
+// proxy): what this thread read of the stage has arrived in its registers. An arrival on a barrier does not say that by
+// itself: loads that were issued before it but whose results nobody has used yet may still be on their way when the refill
+// lands, and then deliver bytes of it. (Seen with fp16 weights, whose words went into tensor memory only after the arrival: one 16-byte
+// piece of one weight row in some ten million was that of the slot's next content.) `used` combines a word of each load, so that
+// the comparison cannot be made before all of them are there; the store it guards hardly ever happens and means nothing.
+__device__ __forceinline__ void loads_returned(uint32_t used, volatile uint32_t* nobody) {
+    if (used == 0x9e3779b9u) *nobody = used;
+}
+
 // Programmatic dependent launch: wait for the preceding grid in the stream / let the next one start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

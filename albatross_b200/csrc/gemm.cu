@@ -306,6 +306,7 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
     uint64_t &accum_bar = bars[N_BARS - 3], &resid_bar = bars[N_BARS - 2], &recv_bar = bars[N_BARS - 1];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_failed;
+    __shared__ uint32_t s_nobody;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 4 * G_NG + 1) tmem_alloc(&tmem_base_s, (uint32_t)g.tmem_cols);
     // ---- which product, which tile, which K split
@@ -425,11 +426,15 @@ __device__ __forceinline__ void gemm_block(const GemmMaps& maps, const GemmGroup
                     uint4 raw[8 / P], cur[8];
                     raw_fetch<F>(raw_slot, r_local, sub, raw);
                     if (F == FMT_FP4 && !own_sc) sc4 = *reinterpret_cast<const uint32_t*>(raw_slot + G_BM * G_RAW_ROW + r_local * 16 + sub * 4);
-                    raw_dequant<F>(raw, sc4, cur);
                     if (h == KS - 1 || P == 1) {
+                        uint32_t used = F == FMT_FP4 && !own_sc ? sc4 : 0u;
+#pragma unroll
+                        for (int q = 0; q < 8 / P; ++q) used ^= raw[q].x;
+                        loads_returned(used, &s_nobody);
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&raw_empty[slot]);
                     }
+                    raw_dequant<F>(raw, sc4, cur);
                     advance(1);
                     if (h == 0) {
                         if (st >= G_STAGES) wait_ok(&empty[stage], e_parity);

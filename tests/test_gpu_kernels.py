@@ -272,6 +272,22 @@ def test_batched_product_recycles_its_weight_slots(fmt, rows, n, k):
         assert torch.equal(_gemm(pm, x), got)
 
 
+@pytest.mark.parametrize("fmt,rows,n,k", [("none", 768, 12288, 4096), ("none", 320, 8192, 4096), ("none", 100, 16384, 2048), ("int8", 768, 12288, 4096),
+                                          ("nvfp4", 768, 12288, 4096)])
+def test_batched_product_reads_its_weight_slots_before_it_gives_them_back(fmt, rows, n, k):
+    """A slot of weights is refilled as soon as the warps that read it say so. With fp16 weights a piece of a row was now and
+    then that of the refill (768 x 12288 x 4096: in one call of two); so call after call has to give the same bits, and those within
+    one rounding of the product (fp16: 2**-11 of a value) plus fp32 sums (k / 16 additions, each off by 2**-23 of a sum below 8)."""
+    from albatross_b200 import quant
+    torch.manual_seed(n + rows)
+    pm = quant.quantize((torch.randn(n, k, device="cuda") * 0.02), None if fmt == "none" else fmt)
+    x = torch.randn(rows, k, device="cuda").half()
+    first = _gemm(pm, x, 0, None)
+    want = x.double() @ pm.dequantize().double().t()
+    assert ((first.double() - want).abs() <= 2 ** -11 * 1.02 * want.abs() + k / 16 * 8 * 2 ** -23).all()
+    assert all(torch.equal(_gemm(pm, x, 0, None), first) for _ in range(60))
+
+
 def test_batched_product_small_k_and_epilogues():
     """Adapter-sized products (K = 16 ... 480, not multiples of the 64-input k-step) and the fused epilogues."""
     from albatross_b200 import _lib, quant
