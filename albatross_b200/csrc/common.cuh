@@ -179,9 +179,10 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
 // itself: loads that were issued before it but whose results nobody has used yet may still be on their way when the refill
 // lands, and then deliver bytes of it. (Seen with fp16 weights, whose words went into tensor memory only after the arrival: one 16-byte
 // piece of one weight row in some ten million was that of the slot's next content.) `used` combines a word of each load, so that
-// the comparison cannot be made before all of them are there; the store it guards hardly ever happens and means nothing.
-__device__ __forceinline__ void loads_returned(uint32_t used, volatile uint32_t* nobody) {
-    if (used == 0x9e3779b9u) *nobody = used;
+// the comparison cannot be made before all of them are there; the store it guards hardly ever happens and means nothing. (One
+// predicated store: as a branch it cost the step of 8 sequences 3.3 us of 174, so it costs 0.8.)
+__device__ __forceinline__ void loads_returned(uint32_t used, uint32_t* nobody) {
+    asm volatile("{\n .reg .pred p;\n setp.eq.u32 p, %0, 0x9e3779b9;\n @p st.volatile.shared.u32 [%1], %0;\n}" ::"r"(used), "r"(smem_u32(nobody)) : "memory");
 }
 
 // Programmatic dependent launch: wait for the preceding grid in the stream / let the next one start.

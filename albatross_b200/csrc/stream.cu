@@ -98,6 +98,7 @@ template <int NT>
 __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_constant__ SgMaps maps, const __grid_constant__ SgGroup g) {
     extern __shared__ __align__(1024) unsigned char ssm[];
     __shared__ uint64_t x_full[SG_WARPS], w_full[SG_WARPS][SG_STAGES];
+    __shared__ uint32_t s_nobody;
     constexpr int N = 8 * NT, TILE_F = N * SG_COL;   // floats of a tile's partial sums: [batch row][weight row]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q = lane & 3;
     const int cl = (int)blockIdx.x / g.ks, rank = (int)blockIdx.x - cl * g.ks;
@@ -169,8 +170,10 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
                 }
             }
         };
-        auto piece = [&](const unsigned char* w, const unsigned char* sc, int c, int row0) {
+        // (returns a combination of a word of each load from the stage)
+        auto piece = [&](const unsigned char* w, const unsigned char* sc, int c, int row0) -> uint32_t {
             (void)sc; (void)row0;
+            uint32_t used = 0;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {   // halves of the 128 bytes: a lane's 16 bytes of four rows
                 uint4 lo[2], hi[2];
@@ -178,6 +181,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
                 for (int m = 0; m < 2; ++m) {
                     lo[m] = *reinterpret_cast<const uint4*>(w + (16 * m + gq) * 128 + (((4 * i + q) ^ gq) << 4));
                     hi[m] = *reinterpret_cast<const uint4*>(w + (16 * m + 8 + gq) * 128 + (((4 * i + q) ^ gq) << 4));
+                    used ^= lo[m].x ^ hi[m].x;
                 }
                 uint32_t l[2][4], h[2][4];
                 if (F == FMT_I8) {
@@ -212,6 +216,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
                             a = at < pitch && ra < pb.n_out ? __ldg(reinterpret_cast<const unsigned short*>(s + (size_t)ra * pitch + at)) : 0u;
                             b = at < pitch && rb < pb.n_out ? __ldg(reinterpret_cast<const unsigned short*>(s + (size_t)rb * pitch + at)) : 0u;
                         }
+                        used ^= a ^ b;
                         sl[m] = e4m3x2_to_half2(a);
                         sh[m] = e4m3x2_to_half2(b);
                     }
@@ -231,6 +236,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
                     }
                 }
             }
+            return used;
         };
         // A lane finishes one weight row for some of the batch rows: 64 consecutive bytes a warp and batch row.
         auto scale_of = [&](int row) {
@@ -251,8 +257,9 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
             const int tile = t0 + slot + round * tpr, row = tile * SG_ROWS + lane;
             const float scale = scale_of(row);   // (used at the end of the tile)
             for (int c = 0; c < nc; ++c, ++i) {
-                                if (!failed && !mbar_wait_bounded(&w_full[warp][stage], parity, 1u << 16)) failed = true;
-                piece(ring + stage * SG_PIECE, F == FMT_FP4 && pb.sc_map ? ring_sc + stage * SG_PIECE_SC : nullptr, c0 + c, tile * SG_ROWS);
+                if (!failed && !mbar_wait_bounded(&w_full[warp][stage], parity, 1u << 16)) failed = true;
+                const uint32_t used = piece(ring + stage * SG_PIECE, F == FMT_FP4 && pb.sc_map ? ring_sc + stage * SG_PIECE_SC : nullptr, c0 + c, tile * SG_ROWS);
+                loads_returned(used, &s_nobody);
                 __syncwarp();   // every lane has read the stage
                 if (lane == 0 && !failed) request();
                 if (++stage == g.stages) { stage = 0; parity ^= 1u; }

@@ -471,3 +471,17 @@ def test_sampler_at_the_edges_of_its_batches(rows, V):
     assert torch.equal(sampler_simple_batch(dev, noise=0.0).flatten().cpu(), logits.float().argmax(1))
     a = sampler_simple_batch(dev, noise=0.5, seed=3).flatten().cpu()     # noise below the winner's margin of 1
     assert torch.equal(a, logits.float().argmax(1))
+
+
+@pytest.mark.parametrize("fmt,rows,n,k", [("int8", 8, 65536, 2048), ("none", 8, 4096, 4096), ("nvfp4", 8, 65536, 2048), ("none", 16, 2560, 2560), ("nvfp4", 5, 8192, 4288)])
+def test_products_of_few_rows_read_a_piece_before_it_is_asked_for_again(fmt, rows, n, k):
+    """A warp's stages of weights are refilled as soon as it has read them: call after call the same bits, and those within one
+    rounding of the product (fp16: 2**-11 of a value) plus fp32 sums (k / 16 additions, each off by 2**-23 of a sum below 8)."""
+    from albatross_b200 import quant
+    torch.manual_seed(n + rows)
+    pm = quant.quantize((torch.randn(n, k, device="cuda") * 0.02), None if fmt == "none" else fmt)
+    x = torch.randn(rows, k, device="cuda").half()
+    first = _gemm(pm, x, 0, None)
+    want = x.double() @ pm.dequantize().double().t()
+    assert ((first.double() - want).abs() <= 2 ** -11 * 1.02 * want.abs() + k / 16 * 8 * 2 ** -23).all()
+    assert all(torch.equal(_gemm(pm, x, 0, None), first) for _ in range(100))
