@@ -74,7 +74,7 @@ __device__ __forceinline__ void stage_phase(DecodePhase* dst, const DecodePhase*
 // The per-head phase of one network block. Its own function (not inlined) so that the register allocation of the
 // matrix-vector phases, which run at the kernel's register cap, does not have to make room for it.
 __device__ __noinline__ void head_phase(const HeadParams& hp, int my_head, int bid, int nb, int tid, unsigned char* smem, unsigned char* pref,
-                                        const __half* xn, HeadShared& hsh, uint32_t epoch, unsigned long long* htl) {
+                                        HeadShared& hsh, uint32_t epoch, unsigned long long* htl) {
     // adapter up-projections inside the phase: block h needs only the 64 channels of head h, so the
     // matrix-vector phase (and the grid barrier) that would produce them for everybody is not needed
     const bool ups = hp.w2 != nullptr;
@@ -96,12 +96,9 @@ __device__ __noinline__ void head_phase(const HeadParams& hp, int my_head, int b
             head_step(hp, 0, h, tid, st, hsh, ups, SyncNamed256(), tg, (pair && ups) ? head_par_area(hp, dsm) : nullptr);
             if (htl) htl[3] = global_ns();
             store_state(st, sbase, tid >> 2, tid & 3);
-            // token-shift state hand-over. Pair mode: the normalised input of the phase before is still in this
-            // block's shared memory (every block prepared it), so no other block's global write is read here.
+            // token-shift state hand-over (pair mode: not before the phase that has seen every head's output)
             if (hp.copy_dst && tid < 32)
-                reinterpret_cast<__half2*>(hp.copy_dst + h * 64)[tid] =
-                    pair ? reinterpret_cast<const __half2*>(xn + h * 64)[tid]
-                         : __ldcg(reinterpret_cast<const __half2*>(hp.copy_src + h * 64) + tid);
+                reinterpret_cast<__half2*>(hp.copy_dst + h * 64)[tid] = __ldcg(reinterpret_cast<const __half2*>(hp.copy_src + h * 64) + tid);
             SyncNamed256()();
         }
     }
@@ -188,7 +185,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
             // sit in front of the loads that wait for the inputs).
             if (tid == 32 && j >= 0 && prog->l2_prefetch_bytes > 0) prefetch_share(phs[j & 3].g, plans[j & 3], 0, prog->l2_prefetch_bytes);
         } else {
-            head_phase(ph.h, plans[i & 3].head, bid, nb, tid, smem, m.pref, m.xn, hsh, epoch,
+            head_phase(ph.h, plans[i & 3].head, bid, nb, tid, smem, m.pref, hsh, epoch,
                        (tid == 0 && tl_base()) ? tl_base() + 2 * n_phases + 4 * i : nullptr);
         }
         if (tid == 0 && tl_base()) tl_base()[2 * i + 1] = global_ns();

@@ -363,8 +363,10 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
             h.w0 = (const __half*)Ly.w0; h.a0 = (const __half*)Ly.a0; h.v0 = (const __half*)Ly.v0;
             h.k_k = (const __half*)Ly.k_k; h.k_a = (const __half*)Ly.k_a; h.r_k = (const __half*)Ly.r_k;
             h.lnx_w = (const __half*)Ly.lnx_w; h.lnx_b = (const __half*)Ly.lnx_b;
-            h.out = ws.att; h.copy_src = ws.xn; h.copy_dst = att_prev;
-            if (fused) {
+            h.out = ws.att;
+            if (!fused) {
+                h.copy_src = ws.xn; h.copy_dst = att_prev;
+            } else {
                 h.pair_mode = -prog->phases[n - 2].rows_per_block; h.tag_in = n - 1; h.tag_out = n;   // n - 1: the phase before (1-based), n: this one
                 ph.no_barrier = 2;
             }
@@ -378,7 +380,10 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
             GemvParams p = {};
             p.K = D; p.x = ws.att; p.nseg = 1;
             p.seg[0] = seg_of(Ly.output, nullptr, EPI_RESID, ws.x, ws.x);
-            if (fused) { p.tag_in = n; p.seg[0].tag_resid = x_tag; p.seg[0].tag_out = n + 1; }   // n: the head phase before
+            if (fused) {
+                p.tag_in = n; p.seg[0].tag_resid = x_tag; p.seg[0].tag_out = n + 1;   // n: the head phase before
+                p.copy_src = ws.xn; p.copy_dst = att_prev; p.copy_n = D;   // every head has run: all blocks have read the old one
+            }
             AB_TRY(gemv_phase(p));
             if (fused) { prog->phases[n - 1].no_barrier = 2; x_tag = n; }
         }
@@ -431,6 +436,28 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
                 }
                 else compute_plan(prog->phases[i].g, b, m->n_sm, bp);
             }
+    return OK;
+}
+
+// What orders the untagged writes of a program in dataflow mode. A phase that hands the token-shift state over overwrites what every
+// block has read in an earlier phase; it may do so because its inputs, all of which it has waited for, were made from the
+// results of every block with a share of that phase: either they are that phase's outputs, or those of the heads behind it.
+int check_decode_program(const DecodeProgram& prog) {
+    for (int i = 0; i < prog.n_phases; ++i) {
+        const DecodePhase& ph = prog.phases[i];
+        if (ph.type == PHASE_HEAD) {
+            AB_CHECK_ARG(!ph.h.pair_mode || !ph.h.copy_dst, "decode program: head phase %d writes a state that other blocks may be reading", i);
+            continue;
+        }
+        if (!ph.g.copy_dst) continue;
+        int reader = i;
+        while (reader >= 0 && !(prog.phases[reader].type == PHASE_GEMV && prog.phases[reader].g.x_prev == ph.g.copy_dst)) --reader;
+        AB_CHECK_ARG(reader >= 0 && reader < i, "decode program: nobody reads the state that phase %d writes", i);
+        if (!prog.phases[reader].no_barrier) continue;   // a barrier among all blocks
+        const int from = (ph.g.tag_in ? ph.g.tag_in : ph.g.seg[0].tag_x) - 1;   // the phase its inputs come from
+        AB_CHECK_ARG(from == reader || (from > reader && from < i && prog.phases[from].type == PHASE_HEAD && prog.phases[from].h.tag_in == reader + 1),
+                     "decode program: phase %d writes a state without waiting for the blocks that read it in phase %d", i, reader);
+    }
     return OK;
 }
 
@@ -691,6 +718,26 @@ int ab_decode_program_build(ab_model* m, const int32_t* token, void* const* stat
     AB_CUDA(cudaMemcpyAsync(program, buf.data(), buf.size(), cudaMemcpyHostToDevice, (cudaStream_t)stream));
     AB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     return OK;
+}
+
+int ab_decode_plan_selftest(ab_model* m, int n_blocks) {
+    AB_CHECK_ARG(m && n_blocks >= 1, "ab_decode_plan_selftest: bad argument");
+    for (const ab_layer& l : m->layers)
+        AB_CHECK_ARG(l.w2t.w && l.a2t.w && l.g2t.w, "ab_decode_plan_selftest: transposed adapter up-projections missing");
+    // stand-ins for device addresses (nothing is read through them): distinct and aligned
+    unsigned char* const base = reinterpret_cast<unsigned char*>(uintptr_t(1) << 40);
+    std::vector<void*> state(3 * (size_t)m->d.n_layer);
+    for (size_t i = 0; i < state.size(); ++i) state[i] = base + (i << 24);
+    unsigned char* const wsb = base + (state.size() << 24);
+    const Workspace ws = carve(m, 1, 1, wsb);
+    std::vector<unsigned char> buf;
+    const int n_sm = m->n_sm, xq = m->prog_xq_bytes;
+    m->n_sm = n_blocks;
+    const int st = build_decode_program(m, (const int32_t*)wsb, state.data(), ws, (__half*)wsb, buf, (const DecodeProgram*)wsb);
+    m->n_sm = n_sm;
+    m->prog_xq_bytes = xq;
+    AB_TRY(st);
+    return check_decode_program(*reinterpret_cast<const DecodeProgram*>(buf.data()));
 }
 
 int ab_decode_run(ab_model* m, void* program, void* stream) {

@@ -48,7 +48,7 @@ struct __align__(16) GemvParams {
     const __half* ln_b;
     __half* ln_out;         // optional: block 0 stores the normalised input here
     __half* x_copy;         // optional: block 0 stores the raw input here (embedding row -> residual stream)
-    const __half* copy_src; // optional: block 0 copies copy_n halves to copy_dst (token-shift state hand-over)
+    const __half* copy_src; // optional: block 0 copies copy_n halves to copy_dst at the end (token-shift state hand-over)
     __half* copy_dst;
     int copy_n;
     int use_pdl;            // kernel was launched with programmatic stream serialization

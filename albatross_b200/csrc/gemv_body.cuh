@@ -736,10 +736,6 @@ __device__ __forceinline__ void gemv_consume(const GemvParams& p, const BlockPla
     // dataflow mode: the input is waited for below (tagged words); the first weight slice travels in the meantime
     if (epoch && early == 1) issue_early();
 
-    if (p.copy_src && bid == 0)
-        for (int i = tid; i < p.copy_n / 8; i += NT_CONS)
-            reinterpret_cast<uint4*>(p.copy_dst)[i] = ld_act16(reinterpret_cast<const uint4*>(p.copy_src) + i);
-
     // ---- epilogue operands of this thread's output row: loaded now, used at the end
     int e_seg = -1, e_row = 0;
     float e_scale = 1.f, e_resid = 0.f;
@@ -979,6 +975,19 @@ __device__ __forceinline__ void gemv_consume(const GemvParams& p, const BlockPla
             if (sg.tag_out) st_tagged(sg.out, e_row, o, tag_of(epoch, sg.tag_out));
             else sg.out[e_row] = __float2half_rn(o);
         }
+    }
+
+    // ---- token-shift state hand-over. In dataflow mode nothing but the tagged inputs of this phase says that every block has
+    // read the old state: a block's share of an earlier phase reaches them only after its reads, so the state may be written
+    // once all of them have been seen, and not before. (copy_src is what this block itself stored a phase or two ago.)
+    if (p.copy_src && bid == 0) {
+        if (p.seg[0].tag_x && bp.n_items == 0) {   // small models: no rows for this block, so nobody here has waited yet
+            uint4 a, b;
+            for (int c = tid; c < p.seg[0].K / 16; c += NT_CONS) ld_tagged16(p.seg[0].x, c, tag_of(epoch, p.seg[0].tag_x), a, b);
+            cons_sync();
+        }
+        for (int i = tid; i < p.copy_n / 8; i += NT_CONS)
+            reinterpret_cast<uint4*>(p.copy_dst)[i] = ld_act16(reinterpret_cast<const uint4*>(p.copy_src) + i);
     }
 }
 

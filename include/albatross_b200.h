@@ -188,6 +188,10 @@ size_t ab_decode_timeline_offset(const ab_model* m);
 int ab_decode_program_build(ab_model* m, const int32_t* token, void* const* state, void* workspace, void* logits,
                             void* program, void* stream);
 int ab_decode_run(ab_model* m, void* program, void* stream);
+/* Host-only self-check of the program that ab_decode_program_build would write for a GPU of `n_blocks` SMs (with the model's
+ * options): the token-shift states, which are plain arrays, are written only behind inputs that depend on every reader of the
+ * old ones. Reads none of the model's memory; runs without a GPU. */
+int ab_decode_plan_selftest(ab_model* m, int n_blocks);
 /* Options (set before ab_decode_program_build for those of the persistent kernel):
  *   "pdl" (1)             programmatic dependent launch between the kernels of a step
  *   "debug_sync" (0)      synchronise and check after every launch

@@ -463,3 +463,24 @@ def test_first_norm_reads_the_embedding_rows(B, T):
         outs.append([_run_stage(model, B, T, st, vf, **kw), vf] + list(st))
         assert _lib.device_status() == (8 if "tokens" in kw else 0)
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+def test_persistent_kernel_with_blocks_that_run_late():
+    """Another stream keeps the SMs busy with short kernels, so the blocks of the persistent kernel start and run at different
+    times: the token-shift states, which are plain arrays, must still be read before they are overwritten. Logits and states
+    equal those of the per-phase launches, bit for bit."""
+    from albatross_b200 import _lib
+    pers, args = model_for("0.1b", "int8")
+    eager, _ = model_for("0.1b", "int8", decode_mode="graph")
+    side, noise = torch.cuda.Stream(), torch.zeros(1 << 20, device="cuda")
+    sp, se = pers.new_state(), eager.new_state()
+    for i, t in enumerate(seeded_tokens(args.vocab_size, 120, seed=8)):
+        le, se = eager.forward(t, se)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for j in range(12): noise[: 1 << (12 + j % 8)].add_(1.0)
+        lp, sp = pers.forward(t, sp)
+        torch.cuda.synchronize()
+        assert torch.equal(lp, le), f"token {i}"
+        assert all(torch.equal(a, b) for a, b in zip(sp, se)), f"token {i}"
+    assert _lib.device_status() == 0

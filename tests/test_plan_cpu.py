@@ -157,3 +157,38 @@ def test_state_list_forgets_its_checks_when_changed():
     st = _State(["a", "b"], mark)
     assert st[1] == "b" and len(st) == 2 and st._ab is mark          # reading keeps them
     assert not hasattr(list(st), "_ab") and _State(st)._ab is None   # a copy starts unchecked
+
+
+def _program_check(D, L, ranks, fmt, n_blocks, options=()):
+    """ab_decode_plan_selftest of a model whose pointers are stand-ins (the library only looks at shapes)."""
+    p = 1 << 20
+    mat = lambda n, k, f=F16: _lib.Mat(fmt=f, n_out=n, k=k, w=p, scale=p if f != F16 else None, tscale=1.0)
+    rw, ra, rv, rg = ranks
+    layers = (_lib.Layer * L)()
+    for i, l in enumerate(layers):
+        for name, _ in _lib.Layer._fields_[:19]: setattr(l, name, p)
+        for name in ("receptance", "key", "value", "output"): setattr(l, name, mat(D, D, fmt))
+        l.ffn_key, l.ffn_value = mat(4 * D, D, fmt), mat(D, 4 * D, fmt)
+        l.w1t, l.a1t, l.g1t = mat(rw, D), mat(ra, D), mat(rg, D)
+        l.w2t, l.a2t, l.g2t = mat(D, rw), mat(D, ra), mat(D, rg)
+        l.w2 = l.a2 = l.g2 = p
+        if i > 0: l.v1t, l.v2t, l.v2 = mat(rv, D), mat(D, rv), p
+    desc = _lib.ModelDesc(n_layer=L, n_embd=D, vocab=512, emb=p, lnout_w=p, lnout_b=p, head=mat(512, D, fmt), layers=layers)
+    model = C.c_void_p()
+    assert _lib.lib.ab_model_create(C.byref(desc), C.byref(model)) == 0, _lib.lib.ab_last_error().decode()
+    try:
+        for name, value in options: assert _lib.lib.ab_model_set_option(model, name, value) == 0
+        rc = _lib.lib.ab_decode_plan_selftest(model, n_blocks)
+        assert rc == 0, _lib.lib.ab_last_error().decode()
+    finally:
+        _lib.lib.ab_model_destroy(model)
+
+
+@pytest.mark.parametrize("D,ranks", [(64, (16, 16, 16, 16)), (256, (32, 32, 16, 48)), (768, (64, 64, 32, 128)), (2048, (96, 96, 64, 256)),
+                                     (4096, (128, 128, 96, 480))])
+@pytest.mark.parametrize("fmt", [F16, I8, FP4])
+@pytest.mark.parametrize("options", [(), ((b"fuse_heads", 0),), ((b"merge_ups", 1),)])
+def test_decode_program_orders_the_token_shift_states(D, ranks, fmt, options):
+    """Without a barrier among all blocks a token-shift state may be overwritten only behind inputs that depend on every block that
+    read the old one: not by a head's own phase (its inputs come from a few blocks), and not ahead of the wait for the inputs."""
+    for n_blocks in (148, 132): _program_check(D, 3, ranks, fmt, n_blocks, options)
