@@ -367,7 +367,7 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
             if (!fused) {
                 h.copy_src = ws.xn; h.copy_dst = att_prev;
             } else {
-                h.pair_mode = -prog->phases[n - 2].rows_per_block; h.tag_in = n - 1; h.tag_out = n;   // n - 1: the phase before (1-based), n: this one
+                h.pair_mode = 1; h.tag_in = n - 1; h.tag_out = n;   // n - 1: the phase before (1-based), n: this one
                 ph.no_barrier = 2;
             }
             if (ups_in_head) {   // block h computes the adapter outputs of head h itself (no phase, no barrier for them)
@@ -414,6 +414,17 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
     p.tag_in = x_tag;
     AB_TRY(gemv_phase(p));
     prog->n_phases = n;   // one phase fewer per block when the adapter up-projections run inside the head phase
+    // One number of blocks per head for all layers (the first has fewer adapter rows and could do with more): layer 0's value
+    // vector is a plain array, so every head has to stay with the block that wrote its part of it.
+    int per_head = 0;
+    for (int i = 0; i < n; ++i) {
+        const int P = -prog->phases[i].rows_per_block;
+        if (P > 0 && (per_head == 0 || P < per_head)) per_head = P;
+    }
+    for (int i = 0; i < n; ++i) {
+        if (prog->phases[i].rows_per_block < 0) prog->phases[i].rows_per_block = -per_head;
+        if (prog->phases[i].type == PHASE_HEAD && prog->phases[i].h.pair_mode) prog->phases[i].h.pair_mode = per_head;
+    }
     int nxt = -1;
     for (int i = n - 1; i >= 0; --i) {
         prog->phases[i].next_gemv = nxt;
@@ -442,10 +453,15 @@ int build_decode_program(ab_model* m, const int32_t* token, void* const* state, 
 // What orders the untagged writes of a program in dataflow mode. A phase that hands the token-shift state over overwrites what every
 // block has read in an earlier phase; it may do so because its inputs, all of which it has waited for, were made from the
 // results of every block with a share of that phase: either they are that phase's outputs, or those of the heads behind it.
+// A head's part of layer 0's value vector is another plain array: the block that writes it reads it in every later layer.
 int check_decode_program(const DecodeProgram& prog) {
+    int per_head = -1;
     for (int i = 0; i < prog.n_phases; ++i) {
         const DecodePhase& ph = prog.phases[i];
         if (ph.type == PHASE_HEAD) {
+            AB_CHECK_ARG(per_head < 0 || ph.h.pair_mode == per_head, "decode program: head phase %d runs on other blocks than the one before (%d per head, %d)",
+                         i, ph.h.pair_mode, per_head);
+            per_head = ph.h.pair_mode;
             AB_CHECK_ARG(!ph.h.pair_mode || !ph.h.copy_dst, "decode program: head phase %d writes a state that other blocks may be reading", i);
             continue;
         }

@@ -190,7 +190,7 @@ int ab_decode_program_build(ab_model* m, const int32_t* token, void* const* stat
 int ab_decode_run(ab_model* m, void* program, void* stream);
 /* Host-only self-check of the program that ab_decode_program_build would write for a GPU of `n_blocks` SMs (with the model's
  * options): the token-shift states, which are plain arrays, are written only behind inputs that depend on every reader of the
- * old ones. Reads none of the model's memory; runs without a GPU. */
+ * old ones, and a head stays with its block through all layers. Reads none of the model's memory; runs without a GPU. */
 int ab_decode_plan_selftest(ab_model* m, int n_blocks);
 /* Options (set before ab_decode_program_build for those of the persistent kernel):
  *   "pdl" (1)             programmatic dependent launch between the kernels of a step

@@ -192,3 +192,12 @@ def test_decode_program_orders_the_token_shift_states(D, ranks, fmt, options):
     """Without a barrier among all blocks a token-shift state may be overwritten only behind inputs that depend on every block that
     read the old one: not by a head's own phase (its inputs come from a few blocks), and not ahead of the wait for the inputs."""
     for n_blocks in (148, 132): _program_check(D, 3, ranks, fmt, n_blocks, options)
+
+
+@pytest.mark.parametrize("D,ranks", [(256, (32, 32, 16, 48)), (768, (64, 64, 32, 128)), (768, (128, 64, 256, 128)), (2048, (96, 96, 64, 256)),
+                                     (2560, (96, 96, 64, 320))])
+@pytest.mark.parametrize("fmt", [F16, I8, FP4])
+def test_decode_program_keeps_a_head_on_its_block(D, ranks, fmt):
+    """The first layer has fewer adapter rows than the others, which would leave more blocks to its heads; but a head's part of
+    that layer's value vector is read in all the others, without a tag: the same block has to run the head in every layer."""
+    for n_blocks in (148, 144, 132): _program_check(D, 3, ranks, fmt, n_blocks)
