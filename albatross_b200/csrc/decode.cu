@@ -137,6 +137,10 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
     bool failed = false;
     int pre_phase = -1;
     unsigned n_barriers = 0;
+    // Dataflow mode: every block says that it has read the tag base before the last block advances it. (The barrier word is not
+    // used otherwise there; in barrier mode the barriers say it.)
+    const bool dataflow = phs[0].no_barrier == 2;
+    if (dataflow && tid == 0) red_release_add(prog->barrier, 1u);
     for (int i = 0; i < n_phases; ++i) {
         // Descriptor and plan of phase i + 3 are copied asynchronously (a synchronous copy stalls every warp for a
         // memory round trip at the top of every phase). This thread's copies of the earlier iterations are complete
@@ -164,7 +168,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
                          // the first-slice prefetch uses the area that the phase before a paired head phase stages into
                          (i + 1 < n_phases && phs[(i + 1) & 3].type == PHASE_HEAD && phs[(i + 1) & 3].h.pair_mode) ? 0 : prog->early_slice,
                          [&]() {
-                             const int my_head = plans[(i + 1) & 3].head;   // (0 unless the next phase is a head phase in dataflow mode)
+                             const int my_head = i + 1 < n_phases ? plans[(i + 1) & 3].head : 0;   // (0 unless the next phase is a head phase in dataflow mode)
                              if (tid < HT && my_head > 0) {
                                  // "fused heads": this block runs a head right after the phase. Its slices of the
                                  // four adapter up-projection matrices (weights: no dependency) move into the idle
@@ -210,8 +214,16 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) decode_kernel(const DecodePro
             }
         }
     }
-    // Every block has read the tag base by now (block 0 could not have finished the last phase otherwise).
-    if (bid == 0 && tid == 0) const_cast<DecodeProgram*>(prog)->epoch = epoch + (uint32_t)n_phases;
+    // Blocks that have no rows before the last phase (small models) may start after block 0 has finished it.
+    if (bid == 0 && tid == 0) {
+        if (dataflow)
+            for (uint32_t it = 0; ld_acquire_u32(prog->barrier) < (unsigned)nb; ++it)
+                if (it > (1u << 23)) {
+                    atomicOr(&g_device_status, DEV_WAIT_HEAD);
+                    break;
+                }
+        const_cast<DecodeProgram*>(prog)->epoch = epoch + (uint32_t)n_phases;
+    }
 }
 
 }  // namespace

@@ -754,7 +754,10 @@ __device__ __forceinline__ void gemv_consume(const GemvParams& p, const BlockPla
     }
 
     // ---- shared input vector, optional layer norm, token-shift difference
-    const bool shared_in = p.emb || p.x;
+    // (Dataflow mode: a block without rows here must not wait for the tagged input. Nobody waits for such a block, so the words may
+    // carry the next phase's tag before it has looked at them. Small models and adapters only. Block 0 keeps
+    // copies for others: it has rows, or the first head to run, in every phase whose input is overwritten two phases later.)
+    const bool shared_in = (p.emb || p.x) && !(p.tag_in && bp.n_items == 0 && bid != 0);
     if (shared_in) {
         const int K = p.K;
         const __half* xin = p.x;
