@@ -534,7 +534,7 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
     Workspace ws = ws_in;
     if (io && io->v_first) ws.vfirst = io->v_first;
     if (io && io->x_in) AB_CUDA(cudaMemcpyAsync(ws.x, io->x_in, (size_t)M * D * 2, cudaMemcpyDeviceToDevice, st));
-    // (the embedding rows are read by the first block's norm, or gathered in a pass of their own where that takes the general path)
+    // (the embedding rows are read by the first block's norm, or gathered in a pass of their own where that cannot)
     bool rows_from_ids = !(io && io->x_in);
     const int g0 = m->layer_offset;   // index of this model's first block in the whole network
     for (int li = 0; li < m->d.n_layer; ++li) {
@@ -550,7 +550,7 @@ int forward_rows(ab_model* m, int B, int T, const int32_t* tokens, void* const* 
         const bool first = rows_from_ids;   // nothing of this pass runs yet that the launch could overlap with
         if (rows_from_ids) {
             rows_from_ids = false;
-            if (fused && ((uintptr_t)m->d.emb & 15) == 0) {
+            if (fused && ln_mix_table_ok((const __half*)m->d.emb, mp)) {
                 mp.table = (const __half*)m->d.emb; mp.ids = tokens; mp.vocab = m->d.vocab; mp.x_copy = ws.x;
             } else {
                 AB_TRY(gather_rows((const __half*)m->d.emb, tokens, M, D, m->d.vocab, ws.x, st));

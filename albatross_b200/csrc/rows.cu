@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(RT) mix_rows_kernel(MixParams p) {
 // T == 1: layer norm and token-shift lerps of one row in one pass; the row stays in registers (16-byte loads and
 // stores), the normalised row becomes the new token-shift state. Same rounding points as ln_rows + mix_rows.
 constexpr int LM_MAXV = 4;   // 16-byte chunks per thread: D <= 8 * RT * LM_MAXV
+constexpr int LM_TABLE_MAXV = 2;   // ... for sequences whose rows come from an embedding table
 __global__ void __launch_bounds__(RT) ln_mix_rows_kernel(const __half* __restrict__ x, const __half* __restrict__ w,
                                                          const __half* __restrict__ b, const __grid_constant__ MixParams p,
                                                          int use_pdl) {
@@ -252,12 +253,15 @@ __global__ void __launch_bounds__(RT) ln_mix_rows_kernel(const __half* __restric
 // What bounds it: 2 bytes in and 2 * n_mix out per element (768 rows x 4096, six lerps: 44 MB, about 7 us at the copy
 // bandwidth), then the two block-wide sums per row. Alone on a cold cache 21 us there, 13.5 us with one lerp; the three
 // passes it replaces (norm, lerps with 2-byte accesses, state hand-over) took 62 and 27 us.
+// Rows of an embedding table are read here up to LM_TABLE_MAXV chunks; four per thread leave no registers for it (552 bytes of
+// spills, none without), and rows that long are gathered by a pass of their own.
 template <int V>   // 16-byte chunks per thread: D <= 8 * RT * V
 __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict__ x, const __half* __restrict__ w,
                                                         const __half* __restrict__ b, const __grid_constant__ MixParams p, int R,
                                                         int use_pdl) {
     __shared__ float red[RT / 32];
     const int n_chunks = (p.T + R - 1) / R, seq = blockIdx.x / n_chunks, t0 = (blockIdx.x - seq * n_chunks) * R;
+    constexpr bool TABLE = V <= LM_TABLE_MAXV;
     const int nv = p.D / 8;
     const uint4* xs = reinterpret_cast<const uint4*>(x + (size_t)seq * p.T * p.D);
     uint4* state = reinterpret_cast<uint4*>(p.x_prev + (size_t)seq * p.D);
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
     if (use_pdl) pdl_wait();
     auto load = [&](int t, uint4* raw) {
         const uint4* row = xs + (size_t)t * nv;
-        if (p.table) row = reinterpret_cast<const uint4*>(p.table + token_row(p.ids[(size_t)seq * p.T + t], p.vocab) * p.D);
+        if (TABLE && p.table) row = reinterpret_cast<const uint4*>(p.table + token_row(p.ids[(size_t)seq * p.T + t], p.vocab) * p.D);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             const int i = threadIdx.x + v * RT;
@@ -337,7 +341,7 @@ __global__ void __launch_bounds__(RT) ln_mix_seq_kernel(const __half* __restrict
     for (int t = t0; t < t1; ++t) {
         uint4 xn[V];
         norm(raw, xn);
-        if (p.table) {
+        if (TABLE && p.table) {
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const int i = threadIdx.x + v * RT;
@@ -527,9 +531,12 @@ bool ln_mix_rows_ok(const __half* w, const __half* b, const MixParams& p) {
     for (int j = 0; j < p.n_mix; ++j) any |= (uintptr_t)p.mix[j];
     return p.D % 8 == 0 && p.D <= 8 * RT * LM_MAXV && (any & 15) == 0;
 }
+bool ln_mix_table_ok(const __half* table, const MixParams& p) {
+    return ((uintptr_t)table & 15) == 0 && (p.T == 1 || p.D <= 8 * RT * LM_TABLE_MAXV);
+}
 int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixParams& p, cudaStream_t s, bool pdl) {
     AB_CHECK_ARG(x && w && b && p.x_prev && p.n_mix >= 1 && p.n_mix <= 6 && p.B > 0 && ln_mix_rows_ok(w, b, p), "ln_mix_rows: bad argument");
-    AB_CHECK_ARG(!p.table || (p.ids && p.x_copy && p.vocab > 0 && ((uintptr_t)p.table & 15) == 0), "ln_mix_rows: bad embedding table");
+    AB_CHECK_ARG(!p.table || (p.ids && p.x_copy && p.vocab > 0 && ln_mix_table_ok(p.table, p)), "ln_mix_rows: bad embedding table");
     // rows per block of a sequence: as few as fill the GPU (each block normalises one row more than it owns)
     const int rows = p.B * p.T, R = rows >= 2048 ? 4 : (rows >= 512 ? 2 : 1);
     cudaLaunchConfig_t cfg = {};

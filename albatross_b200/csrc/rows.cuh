@@ -25,6 +25,7 @@ int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t see
 // Layer norm of x (weights w, b) fused with the lerps (p.xn is not used). It works on 16 bytes at a time: for other row lengths
 // and for vectors or states of the caller's that are not 16-byte aligned there are ln_rows and mix_rows, which take any.
 bool ln_mix_rows_ok(const __half* w, const __half* b, const MixParams& p);
+bool ln_mix_table_ok(const __half* table, const MixParams& p);   // ... and whether it takes its rows from that table
 int ln_mix_rows(const __half* x, const __half* w, const __half* b, const MixParams& p, cudaStream_t s, bool pdl = false);
 
 }  // namespace ab

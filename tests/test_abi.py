@@ -60,3 +60,13 @@ def test_streaming_kernels_do_not_spill():
         # streaming loop; measured harmless (the same build is the fastest one), anything beyond that is not
         limit = 32 if "decode_kernel" in name else 0
         assert u["spill_bytes"] <= limit, (name, u)
+
+
+def test_norms_of_sequences_do_not_spill():
+    """The norm and lerps of sequences hold a thread's share of a row in registers, for the widest rows (four chunks per
+    thread) as well."""
+    from albatross_b200 import build
+    build.build()
+    usage = {k: v for k, v in build.resource_usage().items() if "ln_mix_seq_kernel" in k or "ln_mix_rows_kernel" in k}
+    assert len(usage) == 3, sorted(usage)
+    for name, u in usage.items(): assert u["spill_bytes"] == 0, (name, u)

@@ -465,6 +465,23 @@ def test_first_norm_reads_the_embedding_rows(B, T):
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
+@pytest.mark.parametrize("D", [4096, 4160])
+def test_rows_too_long_for_the_first_norm_are_gathered(D):
+    """The widest rows that the norm of sequences takes from the embedding itself, and rows beyond it."""
+    import types
+    from albatross_b200 import RWKV_x070, _lib
+    cfg = (1, D, 256, (16, 16, 16, 16))
+    args = types.SimpleNamespace(MODEL_NAME="", n_layer=1, n_embd=D, head_size=64, vocab_size=256, ranks=cfg[3])
+    model = RWKV_x070(args, quant="int8", state_dict=synth.make_checkpoint(cfg, seed=2))
+    for B, T in ((2, 5), (3, 1)):
+        toks = torch.tensor(seeded_tokens(256, B * T, seed=B), dtype=torch.int32, device="cuda")
+        outs = []
+        for kw in ({"tokens": toks}, {"x_in": model.z["emb.weight"][toks.long()].contiguous()}):
+            st, vf = model.new_state(B), torch.zeros(B * T, D, dtype=torch.float16, device="cuda")
+            outs.append([_run_stage(model, B, T, st, vf, **kw), vf] + list(st))
+        assert _lib.device_status() == 0 and all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 def test_persistent_kernel_with_blocks_that_run_late():
     """Another stream keeps the SMs busy with short kernels, so the blocks of the persistent kernel start and run at different
     times: the token-shift states, which are plain arrays, must still be read before they are overwritten. Logits and states
