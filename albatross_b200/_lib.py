@@ -84,6 +84,7 @@ def _load():
     lib.ab_decode_program_build.argtypes = [vp, vp, C.POINTER(vp), vp, vp, vp, vp]
     lib.ab_decode_run.argtypes = [vp, vp, vp]
     lib.ab_decode_plan_selftest.argtypes = [vp, i32]
+    lib.ab_glue_selftest.argtypes = [i32, C.c_uint64, C.c_uint64, vp, vp]
     return lib
 
 
@@ -91,7 +92,7 @@ lib = _load()
 
 EXPORTS = ["ab_last_error", "ab_version", "ab_device_status", "ab_wkv7_fwd", "ab_gemv", "ab_gemm_scratch_bytes",
            "ab_gemm", "ab_gemm_static", "ab_gemm_static_reset", "ab_gemm_static_debug_counter", "ab_sample_rows", "ab_sample_rows_i64", "ab_gemv_plan_selftest", "ab_gemm_plan_selftest", "ab_dequant", "ab_model_create", "ab_model_destroy", "ab_workspace_bytes", "ab_forward", "ab_forward_stage",
-           "ab_model_set_option", "ab_decode_program_bytes", "ab_decode_timeline_offset", "ab_decode_program_build", "ab_decode_run", "ab_decode_plan_selftest"]
+           "ab_model_set_option", "ab_decode_program_bytes", "ab_decode_timeline_offset", "ab_decode_program_build", "ab_decode_run", "ab_decode_plan_selftest", "ab_glue_selftest"]
 
 
 def check(status: int, what: str = "") -> None:

@@ -240,23 +240,28 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // fp16 rounding points: the reference computes its glue in fp16 tensors, so each torch op rounds.
 __device__ __forceinline__ float rh(float v) { return __half2float(__float2half_rn(v)); }
-// Reciprocal, quotient and square root without branches. The compiler's own end in a test and a call for operands at the ends
-// of the range; nine of them in the per-step glue cut it into pieces that cannot overlap (4000 cycles for two steps whose
-// arithmetic is some 600 instructions; 2000 like this). These take the approximation of the hardware and one Newton step on
-// its residual, computed exactly by a fused multiply-add. The operands they are given stay clear of the range's ends; there
-// the results were the same as the compiler's for every float (reciprocal, root) and for 2^31 pairs of fp16 values
-// (quotient). Infinities and NaNs come out as they should. Two blocks of the network, 4096 wide: 8 sequences one step 250 -> 243 us, a
-// prompt of 768 tokens 1385 -> 1360, 5 of 37 tokens 398 -> 384.
+// Reciprocal, quotient and square root of operands that stay clear of the ends of the range, in straight-line code: several steps of
+// the glue then run side by side. Each is the hardware's approximation, which PTX documents (rcp.approx and rsqrt.approx:
+// relative error below 2^-22), and one Newton step whose residual a fused multiply-add computes with a
+// single rounding (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990):
+//   reciprocal  r' = r + r (1 - d r)          from f(r) = 1/r - d:    1 - d r' = (1 - d r)^2
+//   quotient    q' = q - r (d q - x)          q = x r, with r for 1 / d
+//   root        s' = s + (r / 2) (x - s s)    s = x r, from f(s) = s^2 - x, with r for 1 / s
+// With e the approximation's relative error the corrected value is within e^2 (2^-44) of the true one before the last operation rounds it:
+// half a unit in the last place, but for results that lie within 2^-44 of the middle between two floats. Over all
+// operands that reciprocal and root are given here, and all quotients of fp16 numerators by fp16 norms, the results are those of `1.f / d`,
+// `x / d` and `sqrtf` (ab_glue_selftest goes through every one of them). Two blocks of the network, 4096 wide, with these and with the operators:
+// 8 sequences one step 243 and 250 us, a prompt of 768 tokens 1360 and 1385, 5 of 37 tokens 384 and 398.
 __device__ __forceinline__ float recip_(float d) {   // 1 <= d < 2^126, or NaN
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.f), r);
 }
-__device__ __forceinline__ float quot_(float x, float d) {   // 1e-12 <= d <= 65504, infinite or NaN
+__device__ __forceinline__ float quot_(float x, float d) {   // 1e-12 <= d <= 65504 or infinite; x finite, or infinite with d, or NaN
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     const float q = x * r;
-    return d > 65504.f ? q : fmaf(r, fmaf(-d, q, x), q);
+    return d > 65504.f ? q : fmaf(-r, fmaf(d, q, -x), q);   // (signs like this: a numerator of -0 stays -0)
 }
 __device__ __forceinline__ float root_(float x) {   // 0, 2^-60 <= x < 2^60, infinite or NaN
     float r;

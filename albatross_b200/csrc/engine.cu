@@ -670,6 +670,10 @@ int ab_sample_rows_i64(const void* logits, int rows, int vocab, float noise, uin
     return sample_rows((const __half*)logits, rows, vocab, noise, seed, out, true, (cudaStream_t)stream);
 }
 
+int ab_glue_selftest(int which, uint64_t first, uint64_t n, uint64_t* differ, void* stream) {
+    return glue_check(which, first, n, reinterpret_cast<unsigned long long*>(differ), (cudaStream_t)stream);
+}
+
 int ab_dequant(const ab_mat* m, float* out, void* stream) {
     AB_CHECK_ARG(m, "ab_dequant: null pointer");
     return dequant_launch(*m, out, (cudaStream_t)stream);

@@ -865,4 +865,35 @@ int wkv7_launch(int B, int T, int C, int H, float* state, const __half* r, const
     return OK;
 }
 
+// recip_ (0), root_ (1) and quot_ (2) against the operators, operand by operand (see ab_glue_selftest).
+namespace {
+__global__ void glue_check_kernel(int which, unsigned long long first, unsigned long long n, unsigned long long* differ) {
+    unsigned long long bad = 0;
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n; i += (unsigned long long)gridDim.x * blockDim.x) {
+        const unsigned long long op = first + i;
+        float got, want;
+        if (which == 2) {
+            const float x = __half2float(__ushort_as_half((unsigned short)(op & 0xffffu)));
+            const unsigned short nb = (unsigned short)(op >> 16);
+            const float d = fmaxf(__half2float(__ushort_as_half(nb)), 1e-12f);
+            if (isinf(x) && !isinf(d)) continue;   // (the norm of an infinite value is infinite)
+            got = quot_(x, d);
+            want = x / d;
+        } else {
+            const float x = __uint_as_float((unsigned)op);
+            got = which ? root_(x) : recip_(x);
+            want = which ? sqrtf(x) : 1.f / x;
+        }
+        bad += __float_as_uint(got) != __float_as_uint(want) && !(isnan(got) && isnan(want));
+    }
+    if (bad) atomicAdd(differ, bad);
+}
+}  // namespace
+int glue_check(int which, unsigned long long first, unsigned long long n, unsigned long long* differ, cudaStream_t stream) {
+    AB_CHECK_ARG(which >= 0 && which <= 2 && differ && first + n >= first && first + n <= (1ull << 32), "glue check: bad argument");
+    glue_check_kernel<<<1184, 256, 0, stream>>>(which, first, n, differ);
+    AB_CUDA(cudaGetLastError());
+    return OK;
+}
+
 }  // namespace ab

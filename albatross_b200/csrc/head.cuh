@@ -26,6 +26,7 @@ struct HeadParams {
     int pair_mode, tag_in, tag_out, pad_;
 };
 
+int glue_check(int which, unsigned long long first, unsigned long long n, unsigned long long* differ, cudaStream_t stream);
 int head_launch(const HeadParams& p, cudaStream_t stream);
 int wkv7_launch(int B, int T, int C, int H, float* state, const __half* r, const __half* w, const __half* k,
                 const __half* v, const __half* a, const __half* b, __half* y, cudaStream_t stream);

@@ -154,6 +154,12 @@ int ab_sample_rows_i64(const void* logits, int rows, int vocab, float noise, uin
  * Writes the kernels' in-register de-quantised weights as fp32 [n_out,k] (tensor/row/column scales applied). */
 int ab_dequant(const ab_mat* m, float* out, void* stream);
 
+/* Test hook (no counterpart in the reference): the straight-line reciprocal (which = 0), square root (1) and quotient (2) of the
+ * per-step glue against the compiler's operators. Operands first .. first + n - 1 (below 2^32) are the bits of a float (0, 1), or of a
+ * numerator (low half) and a norm (high half) in fp16 (2; the norm is taken as at least 1e-12, as the glue does, and is infinite for an infinite numerator). Adds to
+ * *differ (device memory) how many results have other bits; two NaNs count as equal. */
+int ab_glue_selftest(int which, uint64_t first, uint64_t n, uint64_t* differ, void* stream);
+
 /* ---- whole-model forward -------------------------------------------------------------------
  * ab_forward replaces RWKV_x070.forward / forward_batch (reference/rwkv7.py:98-126, :128-221):
  * tokens int32 [B,T] on the device; state = HOST array of 3*n_layer device pointers laid out as

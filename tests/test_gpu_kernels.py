@@ -485,3 +485,16 @@ def test_products_of_few_rows_read_a_piece_before_it_is_asked_for_again(fmt, row
     want = x.double() @ pm.dequantize().double().t()
     assert ((first.double() - want).abs() <= 2 ** -11 * 1.02 * want.abs() + k / 16 * 8 * 2 ** -23).all()
     assert all(torch.equal(_gemm(pm, x, 0, None), first) for _ in range(100))
+
+
+@pytest.mark.parametrize("which,first,end", [
+    (0, 0x3f800000, 0x7e800000), (0, 0x7fc00000, 0x80000000),                              # 1 <= d < 2^126, NaN
+    (1, 0x21800000, 0x5d800000), (1, 0, 1), (1, 0x7f800000, 0x7f800001), (1, 0x7fc00000, 0x80000000),   # 2^-60 <= x < 2^60, 0, infinity, NaN
+    (2, 0, 0x7c01 << 16), (2, 0x7e00 << 16, 0x8000 << 16)])                                # norms from 0 (1e-12) to infinity, NaN; every numerator
+def test_glue_arithmetic_equals_the_operators(which, first, end):
+    """Reciprocal, root and quotient of the per-step glue have the bits of `1.f / d`, `sqrtf(x)` and `x / d` for every operand they
+    may be given: all floats of the range, and all pairs of an fp16 numerator and an fp16 norm."""
+    from albatross_b200 import _lib
+    differ = torch.zeros(1, dtype=torch.int64, device="cuda")
+    _lib.check(_lib.lib.ab_glue_selftest(which, first, end - first, differ.data_ptr(), _stream()), "ab_glue_selftest")
+    assert differ.item() == 0
