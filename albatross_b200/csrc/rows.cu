@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(RT) ln_mix_rows_kernel(const __half* __restric
                          : "=r"(raw[v].x), "=r"(raw[v].y), "=r"(raw[v].z), "=r"(raw[v].w)
                          : "l"(xr + i)
                          : "memory");
-            if (p.table) reinterpret_cast<uint4*>(p.x_copy + m * p.D)[i] = raw[v];
+            if (p.table && AB_BC(m < (size_t)p.B && 8 * (i + 1) <= p.D)) reinterpret_cast<uint4*>(p.x_copy + m * p.D)[i] = raw[v];
             prv[v] = reinterpret_cast<const uint4*>(p.x_prev + m * p.D)[i];
             const __half2* h = reinterpret_cast<const __half2*>(&raw[v]);
 #pragma unroll

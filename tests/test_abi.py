@@ -70,3 +70,13 @@ def test_norms_of_sequences_do_not_spill():
     usage = {k: v for k, v in build.resource_usage().items() if "ln_mix_seq_kernel" in k or "ln_mix_rows_kernel" in k}
     assert len(usage) == 3, sorted(usage)
     for name, u in usage.items(): assert u["spill_bytes"] == 0, (name, u)
+
+
+def test_wide_scan_and_few_row_products_do_not_spill():
+    """The wide form of the sequence kernels and the products of few rows are held to what their like are."""
+    from albatross_b200 import build
+    build.build()
+    usage = {k: v for k, v in build.resource_usage().items() if "scan_wide_kernel" in k or
+             ("stream_kernel" in k and "gemv_stream_kernel" not in k)}
+    assert len(usage) == 5, sorted(usage)
+    for name, u in usage.items(): assert u["spill_bytes"] == 0, (name, u)

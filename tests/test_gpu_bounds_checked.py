@@ -29,3 +29,18 @@ def test_ragged_shapes_stay_in_bounds_in_the_checked_build():
     tail = (res.stdout + res.stderr)[-2000:]
     assert res.returncode == 0, tail
     assert "passed" in res.stdout and "AB_BOUNDS_CHECK: a kernel recorded" not in res.stdout, tail
+
+
+def test_newer_kernels_stay_in_bounds_in_the_checked_build():
+    """Products of few rows, the sampler's batches, the norms that read the embedding, both forms of the sequence kernels, the glue
+    at the ends of its range, and small models in the persistent kernel."""
+    from albatross_b200 import build
+    assert os.path.exists(build.LIB_CHECKED), "the range-checking build of the library is missing"
+    cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
+           os.path.join(ROOT, "tests", "test_gpu_kernels.py"),
+           os.path.join(ROOT, "tests", "test_gpu_model.py"),
+           "-k", "products_of_few_rows or sampler_at_the_edges or first_norm or glue_at_the_ends or both_block_forms or more_blocks_than_rows"]
+    res = subprocess.run(cmd, cwd=ROOT, env=dict(os.environ, AB_BOUNDS_CHECK="1"), capture_output=True, text=True, timeout=900)
+    tail = (res.stdout + res.stderr)[-2000:]
+    assert res.returncode == 0, tail
+    assert "passed" in res.stdout and "AB_BOUNDS_CHECK: a kernel recorded" not in res.stdout, tail

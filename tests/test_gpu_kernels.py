@@ -498,3 +498,27 @@ def test_glue_arithmetic_equals_the_operators(which, first, end):
     differ = torch.zeros(1, dtype=torch.int64, device="cuda")
     _lib.check(_lib.lib.ab_glue_selftest(which, first, end - first, differ.data_ptr(), _stream()), "ab_glue_selftest")
     assert differ.item() == 0
+
+
+@pytest.mark.parametrize("B,T,H", [(74, 41, 2), (75, 41, 2), (37, 19, 4), (38, 19, 4), (160, 33, 1)])
+def test_wkv7_sequences_are_the_same_in_both_block_forms(B, T, H):
+    """Up to 148 heads (one per SM) a sequence runs in a wide block, beyond that in a narrow one; over several chunks of eight steps
+    and a cut one, a sequence gives the same bits alone (wide) and in batches on either side of the line."""
+    from albatross_b200 import _lib
+    torch.manual_seed(B + T)
+    C_ = 64 * H
+    kk = torch.nn.functional.normalize(torch.randn(B, T, H, 64), dim=-1).view(B, T, C_)
+    ins = [torch.randn(B, T, C_), -torch.rand(B, T, C_) * 2 - 0.5, torch.randn(B, T, C_), torch.randn(B, T, C_), -kk, kk * torch.rand(B, T, C_)]
+    ins = [t.half().cuda() for t in ins]
+    state = torch.randn(B, H, 64, 64, device="cuda") * 0.3
+
+    def run(sl):
+        st, y = state[sl].clone(), torch.empty_like(ins[0][sl])
+        args = [t[sl].contiguous() for t in ins]
+        _lib.check(_lib.lib.ab_wkv7_fwd(st.shape[0], T, C_, H, st.data_ptr(), *[t.data_ptr() for t in args], y.data_ptr(), _stream()), "ab_wkv7_fwd")
+        return y, st
+    whole = run(slice(0, B))
+    for b in (0, B // 2, B - 1):
+        alone = run(slice(b, b + 1))
+        assert torch.equal(whole[0][b:b + 1], alone[0]) and torch.equal(whole[1][b:b + 1], alone[1])
+    assert torch.isfinite(whole[0].float()).all() and _lib.device_status() == 0

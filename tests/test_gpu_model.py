@@ -526,3 +526,22 @@ def test_persistent_kernel_with_more_blocks_than_rows(D):
         assert torch.equal(lp, le), f"token {i}"
         assert all(torch.equal(a, b) for a, b in zip(sp, se)), f"token {i}"
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("T", [21, 40])
+def test_sequences_are_the_same_in_both_block_forms(T):
+    """The model's recurrence over several chunks of eight steps, with 37 and with 38 sequences of four heads: 148 heads run in wide
+    blocks (one per SM), 152 in narrow ones. Hidden states, the value vector and all states of the shared sequences: the same bits
+    (the products in front of it are too narrow to be split, so their sums do not depend on the rows)."""
+    from albatross_b200 import _lib
+    model, args = model_for("tiny", "int8")
+    toks = torch.tensor(seeded_tokens(args.vocab_size, 38 * T, seed=T), dtype=torch.int32, device="cuda")
+    outs = []
+    for B in (37, 38):
+        st = model.new_state(B)
+        vf, x = (torch.zeros(B * T, args.n_embd, dtype=torch.float16, device="cuda") for _ in range(2))
+        _run_stage(model, B, T, st, vf, tokens=toks[:B * T].contiguous(), x_out=x)
+        assert _lib.device_status() == 0
+        outs.append([t[:37 * T] for t in (x, vf)] + [t[:37] for t in st])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    assert torch.isfinite(outs[0][0]).all()
