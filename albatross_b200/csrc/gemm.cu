@@ -968,17 +968,6 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
         const int s = check_mat(ops[i].w, "gemm");
         if (s != OK) return s;
     }
-    const int n_sm = current_sm_count();
-    GroupShape gs = launch_shape(ops, n, rows, n_sm);
-    AB_CHECK_ARG(gs.n_split_tiles <= G_COUNTERS, "gemm: too many split-K tiles");
-    if (gs.n_split_tiles > 0 && (gs.grid_x * gs.n_tiles_y > n_sm || (size_t)G_COUNTERS * 4 + (size_t)gs.part_floats * 4 > scratch_bytes)) {
-        // the blocks of a split tile wait for one another, so all of them must be resident (one block per SM), and their
-        // partial sums must fit the scratch area; a split grid for which that does not hold is launched without the split
-        GemmOp unsplit[G_MAX_OPS];
-        for (int i = 0; i < n; ++i) unsplit[i] = ops[i];
-        gs = launch_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
-    }
-    AB_CHECK_ARG(gs.part_floats == 0 || (scratch && ((uintptr_t)scratch & 15) == 0), "gemm: split-K needs a 16-byte aligned scratch area");
     int st = OK;
     for (int i = 0; i < n; ++i) {
         const GemmOp& op = ops[i];
@@ -989,9 +978,29 @@ int gemm_group_launch(const GemmOp* ops, int n, int rows, void* scratch, size_t 
         AB_CHECK_ARG(m.k % 16 == 0 && ((uintptr_t)op.x & 15) == 0 && ((uintptr_t)m.w & 15) == 0, "gemm: k %% 16 and 16-byte alignment needed");
         AB_CHECK_ARG(m.fmt != FMT_FP4 || (m.k % 64 == 0 && ((uintptr_t)m.scale & 3) == 0), "gemm: NVFP4 needs k %% 64 == 0");
     }
+    // few rows: before the split of this kernel is planned (a prompt of 2 to 24 tokens plans every launch anew); a call
+    // without a scratch area is refused below where this kernel would need one, whichever kernel would run
+    const bool has_scratch = scratch && ((uintptr_t)scratch & 15) == 0;
     bool taken = false;
-    st = stream_group_launch(ops, n, rows, stream, pdl, &taken);
-    if (st != OK || taken) return st;
+    if (has_scratch) {
+        st = stream_group_launch(ops, n, rows, stream, pdl, &taken);
+        if (st != OK || taken) return st;
+    }
+    const int n_sm = current_sm_count();
+    GroupShape gs = launch_shape(ops, n, rows, n_sm);
+    AB_CHECK_ARG(gs.n_split_tiles <= G_COUNTERS, "gemm: too many split-K tiles");
+    if (gs.n_split_tiles > 0 && (gs.grid_x * gs.n_tiles_y > n_sm || (size_t)G_COUNTERS * 4 + (size_t)gs.part_floats * 4 > scratch_bytes)) {
+        // the blocks of a split tile wait for one another, so all of them must be resident (one block per SM), and their
+        // partial sums must fit the scratch area; a split grid for which that does not hold is launched without the split
+        GemmOp unsplit[G_MAX_OPS];
+        for (int i = 0; i < n; ++i) unsplit[i] = ops[i];
+        gs = launch_shape(unsplit, n, rows, 0);   // no SMs to fill: every product keeps its whole K loop
+    }
+    AB_CHECK_ARG(gs.part_floats == 0 || has_scratch, "gemm: split-K needs a 16-byte aligned scratch area");
+    if (!has_scratch) {
+        st = stream_group_launch(ops, n, rows, stream, pdl, &taken);
+        if (st != OK || taken) return st;
+    }
     EncodeTiledFn encode;
     st = get_encode_fn(&encode);
     if (st != OK) return st;

@@ -362,8 +362,12 @@ bool stream_shape(const GemmOp* ops, int n, int rows, const int* clusters, SgSha
             const int tpr = SG_WARPS / kw, rounds = (tpc + tpr - 1) / tpr;
             return (long long)rounds * (((pieces[i] + kw - 1) / kw) * (PIECE * SG_WARPS) + TILE + 12 * N);
         };
+        int at[7] = {};   // the tiles of a block that `left` and `kw` stand for
+        long long left[7];
         auto most = [&](int i) {
             const int tpc = (tiles[i] + s.n_cl[i] - 1) / s.n_cl[i];
+            if (tpc == at[i]) return left[i];
+            at[i] = tpc;
             long long b = 0;
             for (int kw = SG_WARPS; kw >= SG_WARPS / 8; kw /= 2) {
                 const long long c = share(i, tpc, kw);
@@ -372,9 +376,9 @@ bool stream_shape(const GemmOp* ops, int n, int rows, const int* clusters, SgSha
             return b;
         };
         // the clusters go where the largest share is left
-        long long left[7];
+        if (n == 1) s.n_cl[0] = std::min(tiles[0], total);
         for (int i = 0; i < n; ++i) left[i] = most(i);
-        for (int used = n; used < total; ++used) {
+        for (int used = n; n > 1 && used < total; ++used) {
             int pick = -1;
             for (int i = 0; i < n; ++i)
                 if (s.n_cl[i] < tiles[i] && (pick < 0 || left[i] > left[pick])) pick = i;

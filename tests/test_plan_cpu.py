@@ -201,3 +201,13 @@ def test_decode_program_keeps_a_head_on_its_block(D, ranks, fmt):
     """The first layer has fewer adapter rows than the others, which would leave more blocks to its heads; but a head's part of
     that layer's value vector is read in all the others, without a tag: the same block has to run the head in every layer."""
     for n_blocks in (148, 144, 132): _program_check(D, 3, ranks, fmt, n_blocks)
+
+
+@pytest.mark.parametrize("rows", [2, 8, 24, 100])
+@pytest.mark.parametrize("scratch", [None, (1 << 20) + 8])
+def test_products_that_split_k_are_refused_without_a_scratch_area(rows, scratch):
+    """... whichever kernel would run them: the ones of few rows need no scratch, but what a caller may pass does not depend on that."""
+    p = 1 << 20
+    m = _lib.Mat(fmt=I8, n_out=1024, k=16384, w=p, scale=p, tscale=1.0)
+    assert _lib.lib.ab_gemm(C.byref(m), rows, p, p, 0, None, scratch, None) == -1
+    assert b"scratch" in _lib.lib.ab_last_error()
