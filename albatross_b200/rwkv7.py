@@ -391,7 +391,10 @@ class RWKV_x070:
     def _send_ids(self, ids: torch.Tensor) -> torch.Tensor:
         """A prompt's ids on the device, sent from page-locked memory: a copy from ordinary memory would wait for the stream
         to drain, and the launches of this call would start behind the last one of the call before. (torch's allocator
-        hands a page-locked block out again when the copies that read it have completed.)"""
+        hands a page-locked block out again when the copies that read it have completed.) Under stream capture the recorded copy would
+        read that block again at every replay, long after it was handed out to somebody else: refused, like a copy from ordinary memory."""
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("a prompt's ids come from the host at the time of the call; they cannot be part of a stream capture")
         return ids.pin_memory().to(self.device, non_blocking=True)
 
     def _hand_back(self, state: List[torch.Tensor], batch: Optional[int]):

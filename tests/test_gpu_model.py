@@ -545,3 +545,26 @@ def test_sequences_are_the_same_in_both_block_forms(T):
         outs.append([t[:37 * T] for t in (x, vf)] + [t[:37] for t in st])
     assert all(torch.equal(a, b) for a, b in zip(*outs))
     assert torch.isfinite(outs[0][0]).all()
+
+
+@pytest.mark.parametrize("call", ["forward", "forward_batch"])
+def test_host_ids_are_refused_under_stream_capture(call):
+    """Ids given as Python numbers belong to one call; recording their copy would replay whatever lies in that memory later. The
+    model still works after the refusal, and its state is what it was."""
+    from albatross_b200 import _lib
+    model, args = model_for("tiny", "int8")
+    run = {"forward": lambda st: model.forward([1, 2, 3], st), "forward_batch": lambda st: model.forward_batch([[1, 2], [3, 4]], st)}[call]
+    B = 2 if call == "forward_batch" else None
+    new = (lambda: model.new_state(B)) if B else model.new_state
+    want, _ = run(new())
+    want = want.clone()
+    st = new()
+    before = [t.clone() for t in st]
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="capture"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            run(st)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(st, before))
+    got, _ = run(st)
+    assert torch.equal(got, want) and _lib.device_status() == 0
