@@ -39,7 +39,7 @@ def test_newer_kernels_stay_in_bounds_in_the_checked_build():
     cmd = [sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
            os.path.join(ROOT, "tests", "test_gpu_kernels.py"),
            os.path.join(ROOT, "tests", "test_gpu_model.py"),
-           "-k", "products_of_few_rows or sampler_at_the_edges or first_norm or glue_at_the_ends or both_block_forms or more_blocks_than_rows"]
+           "-k", "products_of_few_rows or wide_steps or sampler_at_the_edges or first_norm or glue_at_the_ends or both_block_forms or more_blocks_than_rows"]
     res = subprocess.run(cmd, cwd=ROOT, env=dict(os.environ, AB_BOUNDS_CHECK="1"), capture_output=True, text=True, timeout=900)
     tail = (res.stdout + res.stderr)[-2000:]
     assert res.returncode == 0, tail

@@ -522,3 +522,22 @@ def test_wkv7_sequences_are_the_same_in_both_block_forms(B, T, H):
         alone = run(slice(b, b + 1))
         assert torch.equal(whole[0][b:b + 1], alone[0]) and torch.equal(whole[1][b:b + 1], alone[1])
     assert torch.isfinite(whole[0].float()).all() and _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("fmt,rows,n,k", [("int8", 8, 65536, 2048), ("nvfp4", 2, 65536, 2048), ("int8", 2, 65536, 4096), ("nvfp4", 8, 65536, 4096), ("int8", 8, 37901, 1024),
+                                          ("nvfp4", 3, 37901, 1024), ("int8", 8, 16384, 4096), ("nvfp4", 8, 16384, 4096), ("int8", 8, 4096, 16384)])
+def test_products_of_few_rows_over_several_rounds_of_tiles(fmt, rows, n, k):
+    """A block's warps work through more tiles than they hold at a time (the vocabulary head, wide feed-forwards): the request cursor
+    moves on to the next tile, stage and phase bit are carried across tiles, and partial sums are read before the next tile's
+    are written. 37901 rows: one more than eight tiles of 32 rows for every warp of 148 SMs, and a ragged end. Every epilogue; bounds as above."""
+    from albatross_b200 import quant
+    torch.manual_seed(n + k + rows)
+    pm = quant.quantize((torch.randn(n, k, device="cuda") * 0.02), fmt)
+    x, r = torch.randn(rows, k).half().cuda(), torch.randn(rows, n).half().cuda()
+    want = x.double() @ pm.dequantize().double().t()
+    for epi, fn in ((0, lambda t: t), (3, lambda t: torch.relu(t) ** 2), (4, lambda t: t + r.double())):
+        got = _gemm(pm, x, epi, r if epi == 4 else None)
+        ref = fn(want)
+        assert rel_err(got.double().cpu(), ref.cpu()) < 2e-3, epi
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -10.5, epi
+        assert torch.equal(_gemm(pm, x, epi, r if epi == 4 else None), got)

@@ -568,3 +568,25 @@ def test_host_ids_are_refused_under_stream_capture(call):
     assert all(torch.equal(a, b) for a, b in zip(st, before))
     got, _ = run(st)
     assert torch.equal(got, want) and _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("fmt", ["int8", "nvfp4"])
+def test_wide_steps_of_few_sequences(fmt):
+    """Blocks 4096 wide: r, k, v and the adapters of a step of 2 and of 8 sequences are one launch of products of several formats with
+    shares of their own. The same sequences among 32 (the general kernel, other sums) are the reference: logits and states within the
+    tolerance between kernel families."""
+    import types
+    from albatross_b200 import RWKV_x070, _lib
+    cfg = (2, 4096, 1024, (128, 128, 96, 480))
+    args = types.SimpleNamespace(MODEL_NAME="", n_layer=2, n_embd=4096, head_size=64, vocab_size=1024, ranks=cfg[3])
+    model = RWKV_x070(args, quant=fmt, state_dict=synth.make_checkpoint(cfg, seed=4))
+    toks = torch.tensor(seeded_tokens(1024, 2 * 32, seed=5), dtype=torch.int64).view(2, 32, 1)
+    runs = {}
+    for B in (32, 8, 2):
+        st = None
+        for part in toks: logits, st = model.forward_batch(part[:B].tolist(), st)
+        runs[B] = [logits.clone()] + [t.clone() for t in st]
+    assert _lib.device_status() == 0
+    for B in (8, 2):
+        for a, b in zip(runs[B], runs[32]):
+            assert torch.isfinite(a).all() and rel_err(a.float().cpu().numpy(), b[:B].float().cpu().numpy()) <= LOGIT_REL_TOL
