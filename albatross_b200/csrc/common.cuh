@@ -70,6 +70,8 @@ struct PerDeviceOnce {
     }
 };
 
+int current_sm_count();   // SMs of the current device
+
 // Device-side status word: kernels OR a bit in when a bounded wait gives up.
 // The host reads it with ab_device_status().
 static __device__ unsigned int g_device_status = 0;

@@ -407,8 +407,8 @@ __device__ __forceinline__ float sample_noise(uint32_t seed, uint32_t row, uint3
 // (With the maximum over a warp instead of the block, eight chunks per warp and batch still took the long way: 18.1 us, then 13.3.)
 // NT threads per row: 1024 for up to 16 rows, whose rows are a batch of eight chunks per thread (8 rows of 65536: 4.5 us); more
 // threads than that do not share an SM, so further rows take 512 threads as long as every row has an SM to itself and 256
-// beyond, in batches of four chunks of which the next travels while one is looked at (100 rows of 65536 8.9 -> 6.1 us, 200 of
-// 50277 9.5 -> 8.0, 320 of 65536 11.0 -> 10.5, in a graph).
+// beyond, in batches of four chunks of which the next travels while one is looked at (in a graph 100 rows of 65536 8.6 -> 5.8 us,
+// 200 of 50277 9.4 -> 7.8, 320 of 65536 11.0 -> 10.1; in calls one after the other, whose launches outweigh it, 12.4 -> 12.1).
 template <class OutT, int NT>
 __global__ void __launch_bounds__(NT) sample_rows_kernel(const __half* __restrict__ logits, int V, float noise, uint32_t seed,
                                                          OutT* __restrict__ out) {
@@ -558,7 +558,7 @@ int sample_rows(const __half* logits, int rows, int V, float noise, uint32_t see
     if (rows <= 16) {
         if (out_i64) sample_rows_kernel<long long, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (long long*)out);
         else sample_rows_kernel<int, 1024><<<rows, 1024, 0, s>>>(logits, V, noise, seed, (int*)out);
-    } else if (rows <= 148) {
+    } else if (rows <= current_sm_count()) {
         if (out_i64) sample_rows_kernel<long long, 512><<<rows, 512, 0, s>>>(logits, V, noise, seed, (long long*)out);
         else sample_rows_kernel<int, 512><<<rows, 512, 0, s>>>(logits, V, noise, seed, (int*)out);
     } else {
