@@ -32,8 +32,8 @@
 // that the memory and the hand-over between the warps, about 390 cycles a k-step whatever the batch (int8 rows at the
 // copy bandwidth: 350). Around the main loop a block spends 1 us before it (tensor memory, barriers, first rows on their
 // way) and 1 - 3 us behind it; the exchange of a split K costs 5 us.
-// 16384 x 4096, back to back: 320 rows nvfp4 41.2 -> 35.4 us (1214 TFLOP/s), 64 rows nvfp4 32.0 -> 17.9, 8 rows int8 32.6 ->
-// 19.7, against the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below). Launches of
+// 16384 x 4096, back to back: 320 rows nvfp4 41.2 -> 35.4 us (1214 TFLOP/s), 64 rows nvfp4 32.0 -> 17.9 (24 rows int8 now 19.4),
+// against the same kernel with cp.async rows and single-lane issue of MMAs and TMA copies (see *_one below). Launches of
 // few rows, which none of this hides, go to stream.cu.
 #include <cuda.h>
 

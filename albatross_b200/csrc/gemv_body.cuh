@@ -188,8 +188,8 @@ struct SegPlan {
     unsigned npc_inv;        // 2^31 / npc, rounded up: an item's row group without a division
 };
 // (A division of integers is a long chain of dependent instructions, and every item of every warp begins with it. A test for
-// npc == 1 around it helped the 0.1B model and cost the 7.2B shapes; this helps both: 0.1B int8 366.7 -> 362.7 us a token, four
-// blocks of the 7.2B shapes 313.1 -> 308.1.)
+// npc == 1 around it helped the 0.1B model and cost the 7.2B shapes; this helps the first (0.1B int8
+// 366.7 -> 362.7 us a token) and leaves four blocks of the 7.2B shapes where they were (309.3 without, 306.6 with: two runs differ by more).)
 __host__ __device__ inline unsigned npc_inverse(int npc) { return npc == 1 ? 0x80000000u : (0x80000000u + (unsigned)npc - 1u) / (unsigned)npc; }
 // it / npc, exact while it * npc < 2^31
 __host__ __device__ __forceinline__ int group_of_item(int it, unsigned npc_inv) {
@@ -388,13 +388,13 @@ __device__ __forceinline__ void prefetch_share(const GemvParams& q, const BlockP
 }
 
 // ---- work items ------------------------------------------------------------------------------------
-// In bytes every format looks the same: an item is GEMV_ROWS rows x 1024 bytes of each row starting at byte
-// `sb`; lane l reads bytes [sb + u*512 + l*16, +16) of each row for u = 0, 1.
+// In bytes every format looks the same: an item is GEMV_ROWS rows x n_slices slices of 2048 bytes of each row starting
+// at byte `sb`; in slice s lane l reads bytes [sb + s*2048 + u*512 + l*16, +16) of each row for sweeps u = 0 .. 3.
 struct Item {
     const unsigned char* w0;   // first row of the group
     const unsigned char* s0;   // its NVFP4 block scales (else null)
     int row_bytes, rows, sb;   // sb: first byte of the item in each row
-    int n_slices;              // consecutive 1 KB slices in this item
+    int n_slices;              // consecutive slices (GEMV_SLICE_BYTES) in this item
     int seg, pidx;             // segment; index of the item's first partial sum (+ lane * npc per row)
 };
 struct ItemBuf {

@@ -1,4 +1,4 @@
-// Batched products of few rows (up to 32): weights from memory straight into registers, mma.sync.
+// Batched products of few rows (up to 24): weights streamed past resident activations, mma.sync.
 //
 //   Y[rows, n_out] = X[rows, k] W^T       (the products of gemm.cu, same formats, roundings and epilogues)
 //
@@ -36,7 +36,6 @@ constexpr int SG_MAX_ROWS = 24;
 constexpr int SG_SMEM = 225 * 1024;
 
 struct SgProb {
-    const unsigned char* w;
     const void* scale;
     const __half* resid;
     __half* y;
@@ -315,13 +314,18 @@ __global__ void __launch_bounds__(SG_THREADS, 1) stream_kernel(const __grid_cons
 struct SgShape {
     int ks, n_cl[7], kw[7], x_bytes, ring_bytes, red_bytes, stages, smem;
 };
-// Where this kernel is the faster one. Measured, graph of launches, rotating matrices, this kernel and gemm.cu's (us):
-// up to 8 rows everywhere (int8 4096 x 4096 9.0 and 13.2, 16384 x 4096 18.1 and 19.0, 4096 x 16384 19.1 and 23.2; nvfp4 7.4 and
-// 12.7, 17.5 and 18.0, 18.4 and 22.2), but for large fp16 matrices, whose k-steps are long enough to hide the hand-over there (10240
-// x 2560 15.6 and 12.8); up to 16 rows, where reading the activations takes as long as the weights, for what the launch and the
-// split K of the other kernel dominate (int8 2560 x 2560 8.2 and 11.1, 4096 x 4096 12.9 and 13.2, 16384 x 4096 28 and 19);
-// up to 24 for small matrices (768 x 3072 7.9 and 10.3, 2560 x 2560 12.0 and 11.3). Many tiles with little K (adapters) cost
-// a round of sums each: 8.6 and 6 in the step of a batch.
+// Where this kernel is the faster one, measured in graphs of launches over rotating matrices (this kernel and gemm.cu's, us):
+//   up to 8 rows everywhere (int8 4096 x 4096 8.8 and 13.2, 16384 x 4096 17.9 and 19.3, 4096 x 16384 18.8 and 23.3, 65536 x 1024 20.7
+//     and 28.8; nvfp4 6.8 and 11.8, 17.3 and 18.0, 18.4 and 22.6, 20.0 and 28.0; fp16 9.9 and 14.2), but for large fp16 matrices, whose
+//     k-steps are long enough to hide the hand-over there (10240 x 2560 15.6 and 12.8);
+//   up to 16 rows for matrices of 17 M weights (int8 2560 x 2560 6.9 and 10.1, 1024 x 16384 15.8 and 16.6, 4096 x 4096 12.4 and 13.2,
+//     16384 x 4096 28 and 19; nvfp4 7.2 and 10.1, 12.5 and 15.5, 9.8 and 11.8; fp16 9.0 and 11.0);
+//   up to 24 for small ones (2048 x 2048 int8 7.2 and 10.0, nvfp4 6.8 and 10.0, fp16 8.5 and 9.8; 1024 x 4096 7.7 and 10.8, 9.0 and 10.9, 8.3
+//     and 10.8; 2560 x 2560 int8 12.0 and 11.3).
+// In 16 shapes of 768 x 768 to 65536 x 1024, three formats, 2 to 24 rows, it is nowhere the slower one by more than 1 %. From 9 rows on
+// the K split that the plan takes costs more than the planner's constants say (int8 4096 x 4096, 16 rows: 9.5 us in blocks that keep the
+// whole of K, 12.2 and 16.7 in clusters of four and eight). Many tiles with little K (adapters) cost a round of sums each: 8.6 and 6
+// in the step of a batch.
 bool stream_pays(const GemmOp* ops, int n, int rows, int n_sm) {
     long long elems = 0, f16 = 0, tiles = 0, pieces = 0;
     for (int i = 0; i < n; ++i) {
@@ -458,7 +462,7 @@ int stream_group_launch(const GemmOp* ops, int n, int rows, cudaStream_t stream,
     for (int i = 0; i < n; ++i) {
         const ab_mat& m = ops[i].w;
         SgProb& pb = g.pr[i];
-        pb.w = reinterpret_cast<const unsigned char*>(m.w); pb.scale = m.scale; pb.tscale = m.tscale;
+        pb.scale = m.scale; pb.tscale = m.tscale;
         pb.resid = ops[i].resid; pb.y = ops[i].y; pb.epi = ops[i].epi;
         pb.fmt = m.fmt; pb.n_out = m.n_out; pb.k = m.k; pb.n_tiles = (m.n_out + SG_ROWS - 1) / SG_ROWS; pb.kw = sh.kw[i];
         g.cl_base[i] = cl;
